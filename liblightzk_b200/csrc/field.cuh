@@ -13,6 +13,7 @@
 // carry chains (red_row).
 #pragma once
 #include <cstdint>
+#include "inverse.cuh"
 
 namespace lzk {
 
@@ -33,6 +34,11 @@ struct FqP {
         return i == 0 ? 0x538afa89u : i == 1 ? 0xf32cfc5bu : i == 2 ? 0xd44501fbu : i == 3 ? 0xb5e71911u
              : i == 4 ? 0x0a417ff6u : i == 5 ? 0x47ab1effu : i == 6 ? 0xcab8351fu : 0x06d89f71u;
     }
+    // R^3 mod p
+    __host__ __device__ static constexpr uint32_t r3(int i) {
+        return i == 0 ? 0xda1530dfu : i == 1 ? 0xb1cd6dafu : i == 2 ? 0xa7283db6u : i == 3 ? 0x62f210e6u
+             : i == 4 ? 0x0ada0afbu : i == 5 ? 0xef7f0b0cu : i == 6 ? 0x2d592544u : 0x20fd6e90u;
+    }
 };
 
 // Fr: r = 0x30644e72e131a029b85045b68181585d2833e84879b9709143e1f593f0000001
@@ -49,6 +55,11 @@ struct FrP {
     __host__ __device__ static constexpr uint32_t r2(int i) {
         return i == 0 ? 0xae216da7u : i == 1 ? 0x1bb8e645u : i == 2 ? 0xe35c59e3u : i == 3 ? 0x53fe3ab1u
              : i == 4 ? 0x53bb8085u : i == 5 ? 0x8c49833du : i == 6 ? 0x7f4e44a5u : 0x0216d0b1u;
+    }
+    // R^3 mod p
+    __host__ __device__ static constexpr uint32_t r3(int i) {
+        return i == 0 ? 0xb4bf0040u : i == 1 ? 0x5e94d8e1u : i == 2 ? 0x1cfbb6b8u : i == 3 ? 0x2a489cbeu
+             : i == 4 ? 0xa19fcfedu : i == 5 ? 0x893cc664u : i == 6 ? 0x7fcc657cu : 0x0cf8594bu;
     }
 };
 
@@ -339,21 +350,15 @@ __device__ __forceinline__ Fp<P> to_mont(const Fp<P>& a)
     return mul(a, r2);
 }
 
-// a^(p-2) by left-to-right square-and-multiply (Fermat inverse; 0 -> 0)
+// Inverse of a Montgomery element (0 -> 0), canonical: the integer inverse of
+// aR times R^3, one Montgomery product, is a^-1 R.
 template <class P>
 __device__ __noinline__ Fp<P> inverse(const Fp<P>& a)
 {
-    Fp<P> r = Fp<P>::one();
-    #pragma unroll 1
-    for (int i = 7; i >= 0; i--) {
-        uint32_t e = P::p(i) - (i == 0 ? 2u : 0u);
-        #pragma unroll 1
-        for (int b = 31; b >= 0; b--) {
-            r = sqr(r);
-            if ((e >> b) & 1) r = mul(r, a);
-        }
-    }
-    return r;
+    Fp<P> x, r3;
+    inverse_int<P>(x.v, a.v);
+    _Pragma("unroll") for (int i = 0; i < 8; i++) r3.v[i] = P::r3(i);
+    return mul(x, r3);
 }
 
 using Fq = Fp<FqP>;

@@ -516,13 +516,14 @@ __device__ void point_from_wire(const Aff<F>& w, Jac<F>* J, uint32_t* bad)
     *J = Jac<F>{wire_in(w.x), wire_in(w.y), F::one()};
 }
 
-// one thread per proof point: 0 = A, 1 = B, 2 = C
+// one warp per proof point (its lane 0): 0 = A, 1 = B, 2 = C, so the three
+// points' inversions run side by side instead of one after the other
 __global__ void k_proof_to_wire(const Jac<Fq>* A, const Jac<Fq2>* B, const Jac<Fq>* C, uint32_t* wire)
 {
     Aff<Fq>* w1 = reinterpret_cast<Aff<Fq>*>(wire);
     if (threadIdx.x == 0) point_to_wire(*A, w1);
-    if (threadIdx.x == 1) point_to_wire(*B, reinterpret_cast<Aff<Fq2>*>(wire + 16));
-    if (threadIdx.x == 2) point_to_wire(*C, reinterpret_cast<Aff<Fq>*>(wire + 48));
+    if (threadIdx.x == 32) point_to_wire(*B, reinterpret_cast<Aff<Fq2>*>(wire + 16));
+    if (threadIdx.x == 64) point_to_wire(*C, reinterpret_cast<Aff<Fq>*>(wire + 48));
 }
 
 __global__ void k_proof_from_wire(const uint32_t* wire, Jac<Fq>* A, Jac<Fq2>* B, Jac<Fq>* C, uint32_t* bad)
@@ -542,7 +543,7 @@ int lzk_groth16_proof_to_wire(const lzk_groth16_proof* proof, void* wire, void* 
 {
     if (!proof || !wire) return LZK_EINVAL;
     if (reinterpret_cast<uintptr_t>(proof) % 4 || reinterpret_cast<uintptr_t>(wire) % 4) return LZK_EINVAL;
-    k_proof_to_wire<<<1, 32, 0, as_stream(stream)>>>(reinterpret_cast<const Jac<Fq>*>(&proof->A),
+    k_proof_to_wire<<<1, 96, 0, as_stream(stream)>>>(reinterpret_cast<const Jac<Fq>*>(&proof->A),
                                                      reinterpret_cast<const Jac<Fq2>*>(&proof->B),
                                                      reinterpret_cast<const Jac<Fq>*>(&proof->C),
                                                      static_cast<uint32_t*>(wire)); note_launch();

@@ -134,7 +134,9 @@ int lzk_msm_g1(const lzk_fr_t* scalars, const void* bases, size_t n,
                lzk_g1_t* out, const lzk_msm_cfg* cfg, void* stream);
 int lzk_msm_g2(const lzk_fr_t* scalars, const void* bases, size_t n,
                lzk_g2_t* out, const lzk_msm_cfg* cfg, void* stream);
-/* Scratch bytes lzk_msm_g1/_g2 need for this n and cfg (group 1 or 2). */
+/* Scratch bytes lzk_msm_g1/_g2 use for this n and cfg (group 1 or 2).  A
+ * workspace too small for the batched affine rounds (about 56 bytes a sorted
+ * entry for G1, 112 for G2) still runs, with XYZZ additions alone. */
 size_t lzk_msm_workspace_bytes(int group, size_t n, const lzk_msm_cfg* cfg);
 /* Window width the autotuner picks for an MSM of n points (group 1 or 2,
  * precomputed or not). */

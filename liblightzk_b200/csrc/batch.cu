@@ -49,6 +49,10 @@ struct lzk_batch_plan {
     struct NGroup { uint32_t k; int dir; uint32_t count; lzk::Fr** ptrs; };
     std::vector<NGroup> ngroups;
     uint64_t total_pts = 0, total_buckets = 0, total_windows = 0, max_entries = 0, chunks = 0, lvl = 0;
+    uint32_t rounds = 0;               // affine rounds before the accumulation
+    uint64_t max_slots = 0, slice = 0;
+    char* aff = nullptr;               // their scratch, and the points they leave
+    void* fin = nullptr;
     uint32_t chunk = 0, run = 0;       // accumulation chunk, reduction run (tuning table, at creation; the
                                        // width groups take their own runs)
     char* ws = nullptr;
@@ -218,12 +222,12 @@ k_bpersist(const __grid_constant__ PersistArgs<F> a, const __grid_constant__ Red
 {
     __shared__ uint4 fx_raw[128 * sizeof(XYZZ<F>) / 16];
     for (uint64_t t = gtid(); t < a.chunks; t += gstride())
-        accumulate_chunk<F, LZK_BASES_AFFINE>(t, a.bases, a.ent, a.off, a.B, a.chunks, a.chunk, a.nbases, a.bsum,
+        accumulate_chunk<F, LZK_BASES_AFFINE>(t, a.bases, a.ent, a.off, a.B, a.chunks, a.chunk, 0, a.nbases, a.bsum,
                                              a.head, a.tail);
     if (!persist_barrier(a.bar, 1, a.extra, a.polls)) return;
-    fixup_items<F>(a.off, a.B, a.chunk, a.chunks, a.bsum, a.head, a.tail, a.large);
+    fixup_items<F>(a.off, a.B, a.chunk, 0, a.chunks, a.bsum, a.head, a.tail, a.large);
     if (!persist_barrier(a.bar, 2, a.extra, a.polls)) return;
-    fixup_large_items<F>(a.off, a.chunk, a.bsum, a.head, a.tail, a.large, reinterpret_cast<XYZZ<F>*>(fx_raw));
+    fixup_large_items<F>(a.off, a.chunk, 0, a.bsum, a.head, a.tail, a.large, reinterpret_cast<XYZZ<F>*>(fx_raw));
     if (!persist_barrier(a.bar, 3, a.extra, a.polls)) return;
     red_tile_items<F>(jobs, a.tiles);
     if (!persist_barrier(a.bar, 4, a.extra, a.polls)) return;
@@ -311,7 +315,9 @@ static int run_plan(lzk_batch_plan* p, cudaStream_t st)
         }
         LZK_CUDA(cudaMemsetAsync(p->cnt, 0, sizeof(uint32_t) * p->total_buckets, st));
         k_bdigits<false><<<g, 256, 0, st>>>(p->d_desc, p->d_ptsoff, count, p->total_pts, p->fixed, p->off, p->cnt, p->ent); note_launch();
-        LZK_TRY(scan_offsets(p->cnt, (uint32_t)p->total_buckets, p->off, p->bsums, st));
+        LZK_TRY(scan_offsets(p->cnt, (uint32_t)p->total_buckets, p->off, p->bsums, st, p->rounds));
+        // the gaps that pad buckets keep kNoEntry
+        if (p->rounds) LZK_CUDA(cudaMemsetAsync(p->ent, 0xff, sizeof(uint32_t) * p->max_slots, st));
         k_bdigits<true><<<g, 256, 0, st>>>(p->d_desc, p->d_ptsoff, count, p->total_pts, p->fixed, p->off, p->cnt, p->ent); note_launch();
         trace_end(tr, st);
         if (p->persistent) {
@@ -322,17 +328,27 @@ static int run_plan(lzk_batch_plan* p, cudaStream_t st)
         }
         X* bsum = static_cast<X*>(p->bsum);
         tr = trace_begin("batch_msm_accumulate", st);
-        k_accumulate<F, LZK_BASES_AFFINE><<<grid_for(p->chunks, 128), 128, 0, st>>>(
-            p->fixed ? p->table : p->bases, p->ent, p->off, (uint32_t)p->total_buckets, p->chunks, p->chunk,
-            p->fixed ? p->table_pts : p->total_pts, bsum, static_cast<X*>(p->head), static_cast<X*>(p->tail)); note_launch();
+        const void* pts = p->fixed ? p->table : p->bases;
+        const uint64_t npts = p->fixed ? p->table_pts : p->total_pts;
+        if (p->rounds) {
+            Aff<F>* fin = static_cast<Aff<F>*>(p->fin);
+            LZK_TRY(affine_sum<F>(pts, p->ent, p->off + p->total_buckets, p->max_slots, p->slice, p->rounds, npts, p->aff, fin, st));
+            k_accumulate<F, kLayoutPoints><<<grid_for(p->chunks, 128), 128, 0, st>>>(
+                fin, p->ent, p->off, (uint32_t)p->total_buckets, p->chunks, p->chunk, p->rounds, p->max_slots >> p->rounds,
+                bsum, static_cast<X*>(p->head), static_cast<X*>(p->tail)); note_launch();
+        } else {
+            k_accumulate<F, LZK_BASES_AFFINE><<<grid_for(p->chunks, 128), 128, 0, st>>>(
+                pts, p->ent, p->off, (uint32_t)p->total_buckets, p->chunks, p->chunk, 0, npts, bsum,
+                static_cast<X*>(p->head), static_cast<X*>(p->tail)); note_launch();
+        }
         trace_end(tr, st);
         tr = trace_begin("batch_msm_fixup", st);
         LZK_CUDA(cudaMemsetAsync(p->large, 0, sizeof(uint32_t), st));
-        k_fixup<F><<<grid_for(p->total_buckets, 256, sm_count() * 8), 256, 0, st>>>(p->off, (uint32_t)p->total_buckets, p->chunk, p->chunks, bsum,
+        k_fixup<F><<<grid_for(p->total_buckets, 256, sm_count() * 8), 256, 0, st>>>(p->off, (uint32_t)p->total_buckets, p->chunk, p->rounds, p->chunks, bsum,
                                                                             static_cast<X*>(p->head),
                                                                             static_cast<X*>(p->tail), p->large); note_launch();
         constexpr unsigned fx_threads = 32768 / sizeof(X);
-        k_fixup_large<F><<<sm_count() * 2, fx_threads, fx_threads * sizeof(X), st>>>(p->off, p->chunk, bsum, static_cast<X*>(p->head),
+        k_fixup_large<F><<<sm_count() * 2, fx_threads, fx_threads * sizeof(X), st>>>(p->off, p->chunk, p->rounds, bsum, static_cast<X*>(p->head),
                                                                              static_cast<X*>(p->tail), p->large); note_launch();
         trace_end(tr, st);
         // the bucket reductions of all window widths, in the same four launches
@@ -389,7 +405,7 @@ static void destroy_plan(lzk_batch_plan* p)
 
 template <class F>
 static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_desc* ntts, size_t n_ntt,
-                       lzk_batch_plan* p)
+                       lzk_batch_plan* p, bool with_rounds)
 {
     using X = XYZZ<F>;
     // MSMs: widths, ordering, global layout
@@ -441,7 +457,11 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
     p->run = tune_run(p->group, largest, p->fixed);
     // each width group reduces with the run of its own largest MSM's size class
     for (auto& g : p->wgroups) g.run = tune_run(p->group, g.largest, p->fixed);
-    p->chunks = (p->max_entries + p->chunk - 1) / p->chunk;
+    if (!p->persistent && with_rounds) p->rounds = affine_rounds(p->max_entries, std::max<uint64_t>(p->total_buckets, 1));
+    p->max_slots = p->max_entries + p->total_buckets * ((1u << p->rounds) - 1);
+    p->slice = p->max_slots < kAffSlice ? align_up(p->max_slots, size_t(1) << p->rounds) : kAffSlice;
+    p->chunk = acc_chunk(p->chunk, p->rounds);
+    p->chunks = ((p->max_slots >> p->rounds) + p->chunk - 1) / p->chunk;
     // the persistent launch takes every width group's reduction job at once
     if (p->persistent && p->wgroups.size() > kMaxRedJobs) return LZK_EUNSUPPORTED;
     // every width group reduces in the same launches, each in its own slice
@@ -458,13 +478,15 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
     size_t o_bsums = cv.take<uint32_t>((B + 4095) / 4096 + 1);
     size_t o_large = cv.take<uint32_t>(p->chunks / kFixSmall + 2);
     size_t o_bar = cv.take<uint32_t>(2);
-    size_t o_ent = cv.take<uint32_t>(std::max<uint64_t>(p->max_entries, 1));
+    size_t o_ent = cv.take<uint32_t>(std::max<uint64_t>(p->max_slots, 1));
     size_t o_bases = cv.take<Aff<F>>(p->fixed ? 1 : std::max<uint64_t>(p->total_pts, 1));
     size_t o_bsum = cv.take<X>(B);
     size_t o_head = cv.take<X>(std::max<uint64_t>(p->chunks, 1)), o_tail = cv.take<X>(std::max<uint64_t>(p->chunks, 1));
     size_t o_lr0 = cv.take<X>(std::max<uint64_t>(p->lvl, 1)), o_lr1 = cv.take<X>(std::max<uint64_t>(p->lvl, 1));
     size_t o_la0 = cv.take<X>(std::max<uint64_t>(p->lvl, 1)), o_la1 = cv.take<X>(std::max<uint64_t>(p->lvl, 1));
     size_t o_wres = cv.take<X>(std::max<uint64_t>(p->total_windows, 1));
+    size_t o_fin = cv.take<Aff<F>>(p->rounds ? p->max_slots >> p->rounds : 0);
+    size_t o_aff = cv.take<char>(AffineScratch<F>(p->slice, p->rounds).bytes());
     p->ws_bytes = cv.off;
     LZK_TRY(dev_malloc(reinterpret_cast<void**>(&p->ws), p->ws_bytes));
     char* b = p->ws;
@@ -482,6 +504,8 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
     p->tail = b + o_tail;
     p->lr[0] = b + o_lr0; p->lr[1] = b + o_lr1; p->la[0] = b + o_la0; p->la[1] = b + o_la1;
     p->wres = b + o_wres;
+    p->fin = b + o_fin;
+    p->aff = b + o_aff;
     if (n_msm) {
         LZK_CUDA(cudaMemcpy(p->d_desc, p->msm.data(), sizeof(BDesc) * n_msm, cudaMemcpyHostToDevice));
         LZK_CUDA(cudaMemcpy(p->d_ptsoff, ptsoff.data(), sizeof(uint64_t) * n_msm, cudaMemcpyHostToDevice));
@@ -540,14 +564,23 @@ int lzk_batch_plan_create_ex(int group, const lzk_msm_desc* msms, size_t n_msm, 
     if (!out || (group != 1 && group != 2) || (n_msm && !msms) || (n_ntt && !ntts)) return LZK_EINVAL;
     if (flags & ~(LZK_BATCH_FIXED_BASES | LZK_BATCH_PERSISTENT)) return LZK_EINVAL;
     *out = nullptr;
-    lzk_batch_plan* p = new (std::nothrow) lzk_batch_plan();
-    if (!p) return LZK_ENOMEM;
-    p->group = group;
-    p->flags = flags;
-    p->fixed = (flags & LZK_BATCH_FIXED_BASES) != 0;
-    p->persistent = (flags & LZK_BATCH_PERSISTENT) != 0;
-    int rc = group == 2 ? create_plan<Fq2>(msms, n_msm, ntts, n_ntt, p) : create_plan<Fq>(msms, n_msm, ntts, n_ntt, p);
-    if (rc != LZK_OK) { destroy_plan(p); return rc; }
+    lzk_batch_plan* p = nullptr;
+    int rc = LZK_ENOMEM;
+    // a device without room for the affine rounds' scratch still takes the plan
+    for (bool rounds : {true, false}) {
+        p = new (std::nothrow) lzk_batch_plan();
+        if (!p) return LZK_ENOMEM;
+        p->group = group;
+        p->flags = flags;
+        p->fixed = (flags & LZK_BATCH_FIXED_BASES) != 0;
+        p->persistent = (flags & LZK_BATCH_PERSISTENT) != 0;
+        rc = group == 2 ? create_plan<Fq2>(msms, n_msm, ntts, n_ntt, p, rounds)
+                        : create_plan<Fq>(msms, n_msm, ntts, n_ntt, p, rounds);
+        if (rc == LZK_OK) break;
+        const bool again = rc == LZK_ENOMEM && p->rounds;
+        destroy_plan(p);
+        if (!again) return rc;
+    }
     *out = p;
     return LZK_OK;
 }

@@ -99,7 +99,8 @@ const char* lzk_status_string(int status)
 uint32_t lzk_debug_check_word(int clear)
 {
     bool c = clear != 0;
-    return lzk::debug_word_sort(c) | lzk::debug_word_g1(c) | lzk::debug_word_g2(c) | lzk::debug_word_batch(c);
+    return lzk::debug_word_sort(c) | lzk::debug_word_g1(c) | lzk::debug_word_g2(c) | lzk::debug_word_batch(c) |
+           lzk::debug_word_affine_g1(c) | lzk::debug_word_affine_g2(c);
 }
 
 int lzk_debug_checks_enabled(void)

@@ -125,11 +125,13 @@ static inline uint32_t debug_word_here(bool clear)
 static inline uint32_t debug_word_here(bool) { return 0; }
 #endif
 // the error words of the files whose kernels check (msm_sort.cu, msm_g1.cu,
-// msm_g2.cu, batch.cu)
+// msm_g2.cu, batch.cu, affine_g1.cu, affine_g2.cu)
 uint32_t debug_word_sort(bool clear);
 uint32_t debug_word_g1(bool clear);
 uint32_t debug_word_g2(bool clear);
 uint32_t debug_word_batch(bool clear);
+uint32_t debug_word_affine_g1(bool clear);
+uint32_t debug_word_affine_g2(bool clear);
 
 __device__ __forceinline__ uint64_t gtid() { return (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; }
 __device__ __forceinline__ uint64_t gstride() { return (uint64_t)gridDim.x * blockDim.x; }

@@ -202,13 +202,53 @@ void ctx_destroy(ProveCtx* x)
     delete x;
 }
 
+// The affine rounds of a context's MSMs, and the bytes of its buffers: 0
+// x, 1..3 the workspaces, 4..7 the shared sort.
+struct CtxShape {
+    uint32_t lh_rounds = 0, z_rounds = 0;
+    SortWords sort;
+    size_t wsb[3];
+};
+static CtxShape ctx_shape(const lzk_prover* p, bool lean)
+{
+    CtxShape s;
+    if (!lean) {
+        s.lh_rounds = table_rounds(p->tn[2], p->c);
+        s.z_rounds = table_rounds(p->n_vars, p->c);
+    }
+    // the A, B1 and B2 tables all have level stride n_vars
+    s.sort = msm_sort_words(p->n_vars, p->c, p->n_vars, s.z_rounds);
+    for (int i = 0; i < 3; i++) {
+        // ws[0]: the concatenated L and H MSM, which sorts in its workspace;
+        // ws[1]: A and B1; ws[2]: B2
+        const size_t n = i == 0 ? p->tn[2] : p->n_vars;
+        const lzk_msm_cfg cfg = prover_msm_cfg(p, i, n);
+        if (i) s.wsb[i] = msm_presorted_bytes(i == 2 ? 2 : 1, n, &cfg, s.z_rounds);
+        else s.wsb[i] = msm_concat_bytes(n, &cfg, s.lh_rounds);
+    }
+    return s;
+}
+
+// what ctx_create allocates
+size_t ctx_bytes(const lzk_prover* p, bool serving, bool lean)
+{
+    const CtxShape s = ctx_shape(p, lean);
+    size_t b = 3 * p->L * sizeof(Fr) + 4 * sizeof(Jac<Fq>) + sizeof(Jac<Fq2>) + 6 * sizeof(XYZZ<Fq>) + sizeof(XYZZ<Fq2>);
+    b += s.wsb[0] + s.wsb[1] + s.wsb[2] + 4 * (s.sort.cnt + s.sort.off + s.sort.ent + s.sort.bsums);
+    return serving ? b + p->n_vars * sizeof(Fr) + sizeof(lzk_groth16_proof) : b;
+}
+
 // Scratch for one proof of prover p; serving contexts also get their own
 // main stream and witness and proof buffers.
-int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out)
+int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out, bool lean)
 {
     *out = nullptr;
     ProveCtx* x = new (std::nothrow) ProveCtx();
     if (!x) return LZK_ENOMEM;
+    x->lean = lean;
+    const CtxShape s = ctx_shape(p, lean);
+    x->lh_rounds = s.lh_rounds;
+    x->z_rounds = s.z_rounds;
     int rc = LZK_OK;
     do {
         if ((rc = dalloc(&x->bytes, &x->x, 3 * p->L))) break;
@@ -217,21 +257,14 @@ int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out)
         if ((rc = dalloc(&x->bytes, &x->sm1, 6))) break;
         if ((rc = dalloc(&x->bytes, &x->sm2, 1))) break;
         for (int i = 0; i < 3 && rc == LZK_OK; i++) {
-            // ws[0]: the concatenated L and H MSM; ws[1]: A and B1; ws[2]: B2
-            size_t n = i == 0 ? p->tn[2] : p->n_vars;
-            lzk_msm_cfg cfg = prover_msm_cfg(p, i, n);
-            x->wsb[i] = lzk_msm_workspace_bytes(i == 2 ? 2 : 1, n, &cfg);
+            x->wsb[i] = s.wsb[i];
             rc = dalloc(&x->bytes, reinterpret_cast<char**>(&x->ws[i]), x->wsb[i]);
         }
         if (rc) break;
-        {
-            // the A, B1 and B2 tables all have level stride n_vars
-            SortWords w = msm_sort_words(p->n_vars, p->c, p->n_vars);
-            if ((rc = dalloc(&x->bytes, &x->zs_cnt, w.cnt))) break;
-            if ((rc = dalloc(&x->bytes, &x->zs_off, w.off))) break;
-            if ((rc = dalloc(&x->bytes, &x->zs_ent, w.ent))) break;
-            if ((rc = dalloc(&x->bytes, &x->zs_bsums, w.bsums))) break;
-        }
+        if ((rc = dalloc(&x->bytes, &x->zs_cnt, s.sort.cnt))) break;
+        if ((rc = dalloc(&x->bytes, &x->zs_off, s.sort.off))) break;
+        if ((rc = dalloc(&x->bytes, &x->zs_ent, s.sort.ent))) break;
+        if ((rc = dalloc(&x->bytes, &x->zs_bsums, s.sort.bsums))) break;
         if (serving) {
             if ((rc = dalloc(&x->bytes, &x->z, p->n_vars))) break;
             if ((rc = dalloc(&x->bytes, &x->proof, 1))) break;
@@ -260,7 +293,8 @@ static void destroy(lzk_prover* p)
     delete p;
 }
 
-static int create(const lzk_groth16_circuit* c, const lzk_groth16_pk* pk, int mode, uint32_t window_bits, lzk_prover* p)
+static int create(const lzk_groth16_circuit* c, const lzk_groth16_pk* pk, int mode, uint32_t window_bits, bool lean,
+                  lzk_prover* p)
 {
     if (!c || !pk || (mode != LZK_PROVE_STANDARD && mode != LZK_PROVE_REFERENCE)) return LZK_EINVAL;
     if (c->log_domain < 1 || c->log_domain > 24 || c->n_vars < c->n_public + 1) return LZK_EINVAL;
@@ -291,7 +325,7 @@ static int create(const lzk_groth16_circuit* c, const lzk_groth16_pk* pk, int mo
         p->run[i] = tune_run(group, n, true);
     }
 
-    LZK_TRY(ctx_create(p, false, &p->ctx0));
+    LZK_TRY(ctx_create(p, false, &p->ctx0, lean));
     cudaStream_t st = p->ctx0->s1;
 
     // tables: a and b1 (level stride n_vars); l and h concatenated in one
@@ -363,7 +397,7 @@ static int msm_tab1(const lzk_prover* p, ProveCtx* x, int q, const Fr* scal, siz
     lzk_msm_cfg cfg = prover_msm_cfg(p, wsi, p->tn[q]);
     cfg.workspace = x->ws[wsi];
     cfg.workspace_bytes = x->wsb[wsi];
-    if (presorted) return msm_g1_presorted(scal, p->tab[q], n, out, &cfg, st, x->zs_off, x->zs_ent);
+    if (presorted) return msm_g1_presorted(scal, p->tab[q], n, out, &cfg, st, x->zs_off, x->zs_ent, x->z_rounds);
     return lzk_msm_g1(reinterpret_cast<const lzk_fr_t*>(scal), reinterpret_cast<const lzk_g1_affine_t*>(p->tab[q]), n,
                       reinterpret_cast<lzk_g1_t*>(out), &cfg, st);
 }
@@ -386,7 +420,7 @@ int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, 
 
     // s1: one digit sort of z for the A, B1 and B2 MSMs (same scalars, same
     // window width, tables of the same level stride n_vars)
-    LZK_TRY(msm_sort_scalars(z, p->n_vars, p->c, p->n_vars, x->zs_cnt, x->zs_off, x->zs_ent, x->zs_bsums, x->s1));
+    LZK_TRY(msm_sort_scalars(z, p->n_vars, p->c, p->n_vars, x->zs_cnt, x->zs_off, x->zs_ent, x->zs_bsums, x->s1, x->z_rounds));
 
     // s1: A and B1 MSMs; s3 picks up A and B1 for s*A and r*B1
     LZK_TRY(msm_tab1(p, x, 0, z, p->n_vars, x->g1res + 0, 1, x->s1, true));
@@ -401,7 +435,7 @@ int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, 
         lzk_msm_cfg cfg = prover_msm_cfg(p, 2, p->tn2);
         cfg.workspace = x->ws[2];
         cfg.workspace_bytes = x->wsb[2];
-        LZK_TRY(msm_g2_presorted(z, p->tab2, p->n_vars, x->g2res, &cfg, x->s2, x->zs_off, x->zs_ent));
+        LZK_TRY(msm_g2_presorted(z, p->tab2, p->n_vars, x->g2res, &cfg, x->s2, x->zs_off, x->zs_ent, x->z_rounds));
     }
     LZK_CUDA(cudaEventRecord(x->ev_s2, x->s2));
 
@@ -464,7 +498,7 @@ int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, 
         lzk_msm_cfg cfg = prover_msm_cfg(p, 0, p->tn[2]);
         cfg.workspace = x->ws[0];
         cfg.workspace_bytes = x->wsb[0];
-        LZK_TRY(msm_g1_concat(z + p->n_public + 1, p->nl, hs, p->M - 1, p->tab[2], x->g1res + 2, &cfg, st));
+        LZK_TRY(msm_g1_concat(z + p->n_public + 1, p->nl, hs, p->M - 1, p->tab[2], x->g1res + 2, &cfg, st, x->lh_rounds));
     }
 
     // join and assemble
@@ -476,6 +510,18 @@ int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, 
     trace_end(tr_as, st);
     trace_end(tr, st);
     return launch_status();
+}
+
+int prover_make_lean(lzk_prover* p)
+{
+    std::lock_guard<std::mutex> g(p->mu);
+    if (p->ctx0->lean) return LZK_OK;
+    LZK_CUDA(cudaDeviceSynchronize());   // proofs in flight use the context
+    ProveCtx* x = nullptr;
+    LZK_TRY(ctx_create(p, false, &x, true));
+    ctx_destroy(p->ctx0);
+    p->ctx0 = x;
+    return LZK_OK;
 }
 
 // ---------------- proof wire format ----------------
@@ -567,10 +613,17 @@ int lzk_prover_create(const lzk_groth16_circuit* c, const lzk_groth16_pk* pk, in
 {
     if (!out) return LZK_EINVAL;
     *out = nullptr;
-    lzk_prover* p = new (std::nothrow) lzk_prover();
-    if (!p) return LZK_ENOMEM;
-    int rc = create(c, pk, mode, window_bits, p);
-    if (rc != LZK_OK) { destroy(p); return rc; }
+    // a device without room for the affine rounds' scratch still proves
+    lzk_prover* p = nullptr;
+    for (bool lean : {false, true}) {
+        p = new (std::nothrow) lzk_prover();
+        if (!p) return LZK_ENOMEM;
+        int rc = create(c, pk, mode, window_bits, lean, p);
+        if (rc == LZK_OK) break;
+        const bool again = rc == LZK_ENOMEM && !lean && (table_rounds(p->tn[2], p->c) || table_rounds(p->n_vars, p->c));
+        destroy(p);
+        if (!again) return rc;
+    }
     *out = p;
     return LZK_OK;
 }
@@ -598,6 +651,7 @@ int lzk_groth16_prove(lzk_prover* p, const lzk_fr_t* z, const lzk_fr_t* r, const
                       lzk_groth16_proof* proof, void* stream)
 {
     if (!p) return LZK_EINVAL;
+    std::lock_guard<std::mutex> g(p->mu);
     return prove_ctx(p, p->ctx0, reinterpret_cast<const Fr*>(z), r, s, proof, as_stream(stream));
 }
 

@@ -10,15 +10,13 @@
 //
 // 30 steps at a time depend only on the low 30 bits of f and g, so they run
 // on single registers and leave a 2 x 2 matrix of signed 31-bit entries that
-// is then applied to the full numbers (nine signed 30-bit limbs).  Inside the
-// 30 steps, runs of zero bits are taken at once, and while delta < 0 (f stays)
-// up to six bits of g are cleared by one multiple of f.
+// is then applied to the full numbers (nine signed 30-bit limbs).
 //
 // Bound by the latency of its dependent steps where one point is converted:
-// 20 rounds of about 350 instructions here, against the 254 dependent
+// 20 rounds of about 700 instructions here, against the 254 dependent
 // squarings and about 130 products of a Fermat power.  Measured on one point:
-// the affine conversion 228 -> 46 us (G1); the three points of a proof's wire
-// form, one warp each, 686 -> 80 us.
+// an MSM with its affine conversion 1063 -> 881 us (1000 points); a proof with
+// its wire form (one warp a point) 2963 -> 2358 us (2^12 constraints).
 #pragma once
 #include <cstdint>
 
@@ -39,40 +37,26 @@ struct Divsteps30 {
     int32_t u, v, q, r;   // 2^30 f' = u f + v g, 2^30 g' = q f + r g
 };
 
-// 30 divsteps on the low words f0 (odd), g0; d holds delta - 1/2
+// 30 divsteps on the low words f (odd), g; d holds delta - 1/2.  Every step
+// is the same branch-free code, so the lanes of a warp stay together: a
+// version that skips runs of zero bits took more instructions per warp, since
+// the slowest lane sets its length.
 __host__ __device__ __forceinline__ void divsteps30(int32_t& d, uint32_t f, uint32_t g, Divsteps30& t)
 {
-    int32_t u = 1, v = 0, q = 0, r = 1;
-    int rem = 30;
-    for (;;) {
-        const uint32_t stop = g | (0xffffffffu << rem);
-#ifdef __CUDA_ARCH__
-        const int z = __ffs((int)stop) - 1;
-#else
-        const int z = __builtin_ctz(stop);
-#endif
-        g >>= z;
-        u = (int32_t)((uint32_t)u << z);
-        v = (int32_t)((uint32_t)v << z);
-        d += z;
-        rem -= z;
-        if (rem == 0) break;
-        if (d >= 0) {
-            uint32_t x = f; f = g; g = 0u - x;
-            int32_t y = u; u = q; q = -y;
-            y = v; v = r; r = -y;
-            d = -d - 1;
-        }
-        // f stays for the next -d steps: w = -g / f mod 2^lim clears their
-        // low bits (f (f^2 - 2) is -1/f modulo 64 for odd f)
-        int lim = rem < -d ? rem : -d;
-        if (lim > 6) lim = 6;
-        const uint32_t w = (g * f * (f * f - 2u)) & ((1u << lim) - 1u);
-        g += f * w;
-        q = (int32_t)((uint32_t)q + (uint32_t)u * w);
-        r = (int32_t)((uint32_t)r + (uint32_t)v * w);
+    uint32_t u = 1, v = 0, q = 0, r = 1;
+    _Pragma("unroll 6") for (int i = 0; i < 30; i++) {
+        const uint32_t bit = g & 1u, swap = (0u - bit) & ~(uint32_t)(d >> 31);   // all ones: swap f and g
+        const uint32_t s = bit | swap;                                           // 0, 1 or -1
+        const uint32_t ng = g + s * f, nq = q + s * u, nr = r + s * v;
+        f = (g & swap) | (f & ~swap);
+        u = ((q & swap) | (u & ~swap)) << 1;
+        v = ((r & swap) | (v & ~swap)) << 1;
+        g = ng >> 1;
+        q = nq;
+        r = nr;
+        d = (int32_t)(((uint32_t)d ^ swap) + 1u);   // -d or d + 1
     }
-    t.u = u; t.v = v; t.q = q; t.r = r;
+    t.u = (int32_t)u; t.v = (int32_t)v; t.q = (int32_t)q; t.r = (int32_t)r;
 }
 
 // a^-1 mod p of an integer a < p given as 8 limbs (0 for a = 0)

@@ -13,6 +13,35 @@ struct G2 { using F = Fq2; };
 constexpr uint32_t kLevelL = 32;     // smallest warp tile of the bucket reduction (scratch bound)
 constexpr uint32_t kFixSmall = 64;   // partials a single fix-up thread folds
 
+// Batched affine rounds before the XYZZ accumulation (affine.cuh).
+constexpr uint32_t kNoEntry = 0xffffffffu;   // a gap in the padded entry list
+constexpr int kLayoutPoints = 16;            // accumulation operands: the points the rounds leave
+constexpr uint32_t kAffMaxRounds = 5;
+// threads a block and blocks an SM holds (128 and 254 registers; 3 or 5
+// blocks for G1, 3 or 4 for G2 measured slower)
+constexpr uint32_t kAffThreads = 128, kAffBlocksG1 = 4, kAffBlocksG2 = 2;
+constexpr unsigned kAffMinPairs = 4;   // pairs a thread takes at least
+constexpr int kInvGroup = 4;           // products an inverting thread takes
+// Slots whose rounds run together, a bound on the scratch (48 bytes a slot for
+// G1, 96 for G2).  Each slice pays its rounds' inversions (29 us) again: the
+// proof at 2^20 takes 21.0 ms with 2^24, 22.2 with 2^23 (G1) and 2^22 (G2).
+constexpr size_t kAffSlice = size_t(1) << 24;
+// Rounds R for `entries` sorted entries over B buckets: as long as a bucket
+// still holds kAffFill 2^R entries on average, so that the gaps that pad
+// buckets to multiples of 2^R stay below a tenth of the slots.  At 2^20 over a
+// table (240 entries a bucket) R = 1 .. 4 measured 3480, 3279, 3204, 3207 us,
+// against 3641 us without rounds.  Short lists run at the latency of the
+// rounds' launches, which is more than the additions they save.
+constexpr size_t kAffMinEntries = 1u << 16, kAffFill = 8;
+inline uint32_t affine_rounds(size_t entries, size_t B)
+{
+    uint32_t R = 0;
+    if (entries < kAffMinEntries) return 0;
+    while (R < kAffMaxRounds && entries >= (B << (R + 1)) * kAffFill) R++;
+    // slot numbers are 32 bits
+    return entries + (B << R) < (1ull << 32) ? R : 0;
+}
+
 struct MsmPlan {
     size_t n = 0;
     uint32_t c = 0;        // window bits
@@ -26,9 +55,59 @@ struct MsmPlan {
     uint32_t chunk = 0;    // sorted entries per accumulation thread
     uint32_t run = 0;      // buckets per lane run of the reduction tiles
     size_t chunks = 0;
+    uint32_t rounds = 0;      // batched affine rounds before the accumulation
+    size_t max_slots = 0;     // entries with the gaps that pad buckets to 2^rounds
+    size_t slice = 0;         // slots a slice
     // workspace offsets
-    size_t o_cnt, o_off, o_ent, o_bsum, o_head, o_tail, o_lr0, o_la0, o_lr1, o_la1, o_scan, o_large, bytes;
+    size_t o_cnt, o_off, o_ent, o_bsum, o_head, o_tail, o_lr0, o_la0, o_lr1, o_la1, o_scan, o_large, o_aff, o_fin,
+        bytes;
 };
+
+// One affine round (affine.cuh) of slots [s0, s0 + slots) of a padded entry
+// list of *total slots: src are the bases (r = 1) or the slice's points of the
+// round before, out its results, r the rounds done after this one, acc a
+// product per thread.
+struct L5;
+template <class F>
+struct AffineRound {
+    const Aff<F>* src;
+    const uint32_t* ent;   // the slice's first entry
+    const uint32_t* total;
+    uint64_t s0, slots, nbases;
+    uint32_t r;
+    Aff<F>* out;
+    L5* acc;
+};
+int affine_round(const AffineRound<Fq>& a, unsigned blocks, cudaStream_t st);
+int affine_round(const AffineRound<Fq2>& a, unsigned blocks, cudaStream_t st);
+// A thread takes at least kAffMinPairs pairs, and a launch at most the blocks
+// the device holds at once, so that the inversions are shared by as many
+// pairs as the size allows.
+template <class F>
+inline size_t affine_blocks(size_t pairs)
+{
+    return grid_for(pairs / kAffMinPairs, kAffThreads, sm_count() * (sizeof(F) == 32 ? kAffBlocksG1 : kAffBlocksG2));
+}
+// scratch of a slice: a half and a quarter of its slots as points (the odd
+// and the even rounds' results, but the last's), and the products
+template <class F>
+struct AffineScratch {
+    size_t odd, even, acc;   // bytes
+    AffineScratch(size_t slots, uint32_t rounds)
+    {
+        odd = align_up(rounds > 1 ? slots / 2 * sizeof(Aff<F>) : 0);
+        even = align_up(rounds > 2 ? slots / 4 * sizeof(Aff<F>) : 0);
+        acc = align_up(rounds ? affine_blocks<F>(slots / 2) * kAffThreads * 40 : 0);
+    }
+    size_t bytes() const { return odd + even + acc; }
+};
+
+// points an accumulation thread adds after the rounds: its chunk in entries
+// before them, at least kMinChunk
+inline uint32_t acc_chunk(uint32_t chunk, uint32_t rounds)
+{
+    return rounds && chunk >> rounds < kMinChunk ? kMinChunk : chunk >> rounds;
+}
 
 inline uint32_t windows_for(uint32_t c) { return (255 + c - 1) / c; }
 
@@ -47,24 +126,28 @@ inline uint32_t msm_run(const lzk_msm_cfg* cfg, int group, size_t n)
 
 template <class Gp>
 inline void plan_msm(MsmPlan& p, size_t n, uint32_t c, bool shared, size_t stride, uint32_t chunk = kDefaultChunk,
-                     uint32_t run = kDefaultRun)
+                     uint32_t run = kDefaultRun, uint32_t rounds = 0, bool presorted = false)
 {
     using X = XYZZ<typename Gp::F>;
+    using A = Aff<typename Gp::F>;
     p.n = n; p.c = c; p.W = windows_for(c); p.nb = 1u << (c - 1);
     p.shared = shared; p.stride = stride;
     p.wb = shared ? 1 : p.W;
     p.B = p.wb * p.nb;
     p.max_entries = n * (size_t)p.W;
-    p.chunk = chunk;
     p.run = run;
-    p.chunks = (p.max_entries + chunk - 1) / chunk;
+    p.rounds = rounds;
+    p.max_slots = p.max_entries + (size_t)p.B * ((1u << rounds) - 1);
+    p.chunk = acc_chunk(chunk, rounds);
+    p.chunks = ((p.max_slots >> rounds) + p.chunk - 1) / p.chunk;
+    p.slice = p.max_slots < kAffSlice ? align_up(p.max_slots, size_t(1) << rounds) : kAffSlice;
     // bucket reduction scratch: wb * max(1, nb / kLevelL) points per buffer
     // (reduce_buckets)
     size_t lvl = (size_t)p.wb * (p.nb > kLevelL ? p.nb / kLevelL : 1);
     Carver cv;
     p.o_cnt = cv.take<uint32_t>(p.B);
     p.o_off = cv.take<uint32_t>(p.B + 1);
-    p.o_ent = cv.take<uint32_t>(p.max_entries ? p.max_entries : 1);
+    p.o_ent = cv.take<uint32_t>(p.max_slots && !presorted ? p.max_slots : 1);
     p.o_bsum = cv.take<X>(p.B);
     p.o_head = cv.take<X>(p.chunks ? p.chunks : 1);
     p.o_tail = cv.take<X>(p.chunks ? p.chunks : 1);
@@ -74,6 +157,8 @@ inline void plan_msm(MsmPlan& p, size_t n, uint32_t c, bool shared, size_t strid
     p.o_la1 = cv.take<X>(lvl);
     p.o_scan = cv.take<uint32_t>((p.B + 4095) / 4096 + 1);
     p.o_large = cv.take<uint32_t>(p.chunks / kFixSmall + 2);   // count, then bucket ids
+    p.o_fin = cv.take<A>(rounds ? p.max_slots >> rounds : 0);
+    p.o_aff = cv.take<char>(AffineScratch<typename Gp::F>(p.slice, rounds).bytes());
     p.bytes = cv.off;
 }
 
@@ -83,37 +168,70 @@ inline void plan_msm(MsmPlan& p, size_t n, uint32_t c, bool shared, size_t strid
 int msm_sort(const MsmPlan& p, const Fr* scalars, uint32_t* cnt, uint32_t* off, uint32_t* ent, uint32_t* bsums,
              cudaStream_t st, const Fr* hi = nullptr, size_t split = 0);
 uint32_t msm_autotune(int group, size_t n, bool shared);
+// the least workspace a plain G1 MSM runs in (without the affine rounds)
+size_t msm_lean_bytes(size_t n, const lzk_msm_cfg* cfg);
 
 // One digit sort shared by several shifted-table MSMs over the same scalars
 // (the Groth16 A, B1 and B2 queries all take the witness): sizes of its
 // buffers in 32-bit words, the sort itself, and the G1 / G2 MSMs that consume
 // it (msm_sort.cu, msm_g1.cu, msm_g2.cu).  The consumers must use the same
 // n, window width and table level stride as the sort.
+// Rounds: those of a table MSM of n points (or 0), the same for the sort and
+// its consumers, since the sort pads the buckets.
+inline uint32_t table_rounds(size_t n, uint32_t c) { return affine_rounds(n * (size_t)windows_for(c), size_t(1) << (c - 1)); }
 struct SortWords { size_t cnt, off, ent, bsums; };
-SortWords msm_sort_words(size_t n, uint32_t c, size_t stride);
+SortWords msm_sort_words(size_t n, uint32_t c, size_t stride, uint32_t rounds);
+// scratch of a table MSM over a shared sort
+size_t msm_presorted_bytes(int group, size_t n, const lzk_msm_cfg* cfg, uint32_t rounds);
 int msm_sort_scalars(const Fr* scalars, size_t n, uint32_t c, size_t stride, uint32_t* cnt, uint32_t* off,
-                     uint32_t* ent, uint32_t* bsums, cudaStream_t st);
+                     uint32_t* ent, uint32_t* bsums, cudaStream_t st, uint32_t rounds);
 int msm_g1_presorted(const Fr* scalars, const void* table, size_t n, Jac<Fq>* out, const lzk_msm_cfg* cfg,
-                     cudaStream_t st, const uint32_t* off, const uint32_t* ent);
+                     cudaStream_t st, const uint32_t* off, const uint32_t* ent, uint32_t rounds);
 int msm_g2_presorted(const Fr* scalars, const void* table, size_t n, Jac<Fq2>* out, const lzk_msm_cfg* cfg,
-                     cudaStream_t st, const uint32_t* off, const uint32_t* ent);
+                     cudaStream_t st, const uint32_t* off, const uint32_t* ent, uint32_t rounds);
 // A shifted-table G1 MSM whose scalars are two arrays, lo[0..n_lo) then
 // hi[0..n_hi), over one table of n_lo + n_hi points per level (msm_g1.cu):
 // two MSMs whose results are only ever added, done as one (one sort, one
 // bucket set, one reduction).  cfg must carry a workspace.
 int msm_g1_concat(const Fr* lo, size_t n_lo, const Fr* hi, size_t n_hi, const void* table, Jac<Fq>* out,
-                  const lzk_msm_cfg* cfg, cudaStream_t st);
-// exclusive scan of cnt[0..B) into off[0..B], off[B] = total; bsums holds
-// (B + 4095) / 4096 + 1 words (msm_sort.cu)
-int scan_offsets(const uint32_t* cnt, uint32_t B, uint32_t* off, uint32_t* bsums, cudaStream_t st);
+                  const lzk_msm_cfg* cfg, cudaStream_t st, uint32_t rounds);
+size_t msm_concat_bytes(size_t n, const lzk_msm_cfg* cfg, uint32_t rounds);
+// exclusive scan of cnt[0..B), each rounded up to a multiple of 2^rounds,
+// into off[0..B], off[B] = total; bsums holds (B + 4095) / 4096 + 1 words
+// (msm_sort.cu)
+int scan_offsets(const uint32_t* cnt, uint32_t B, uint32_t* off, uint32_t* bsums, cudaStream_t st, uint32_t rounds = 0);
+// All rounds of a padded list of at most max_slots slots into fin (point i is
+// what slots [i 2^rounds, (i + 1) 2^rounds) sum to), a slice at a time.
+template <class F>
+int affine_sum(const void* bases, const uint32_t* ent, const uint32_t* total, size_t max_slots, size_t slice,
+               uint32_t rounds, uint64_t nbases, char* scratch, Aff<F>* fin, cudaStream_t st)
+{
+    const AffineScratch<F> sz(slice, rounds);
+    AffineRound<F> a{};
+    a.total = total;
+    a.nbases = nbases;
+    a.acc = reinterpret_cast<L5*>(scratch + sz.odd + sz.even);
+    for (size_t s0 = 0; s0 < max_slots; s0 += slice) {
+        a.ent = ent + s0;
+        a.s0 = s0;
+        a.slots = max_slots - s0 < slice ? max_slots - s0 : slice;
+        a.src = static_cast<const Aff<F>*>(bases);
+        for (a.r = 1; a.r <= rounds; a.r++) {
+            a.out = a.r == rounds ? fin + (s0 >> rounds) : reinterpret_cast<Aff<F>*>(scratch + (a.r & 1 ? 0 : sz.odd));
+            LZK_TRY(affine_round(a, (unsigned)affine_blocks<F>(a.slots >> a.r), st));
+            a.src = a.out;
+        }
+    }
+    return LZK_OK;
+}
 
-// largest b in [lo, B) with off[b] <= e
-__device__ __forceinline__ uint32_t bucket_of(const uint32_t* off, uint32_t lo, uint32_t B, uint32_t e)
+// largest b in [lo, B) with off[b] >> shift <= e
+__device__ __forceinline__ uint32_t bucket_of(const uint32_t* off, uint32_t lo, uint32_t B, uint32_t e, uint32_t shift)
 {
     uint32_t hi = B;  // invariant: off[lo] <= e, answer in [lo, hi)
     while (hi - lo > 1) {
         uint32_t mid = (lo + hi) >> 1;
-        if (off[mid] <= e) lo = mid; else hi = mid;
+        if (off[mid] >> shift <= e) lo = mid; else hi = mid;
     }
     return lo;
 }
@@ -155,6 +273,26 @@ __device__ __forceinline__ Aff<Fq2> load_raw<Fq2, LZK_BASES_REF_G2_LANES>(const 
     return Aff<Fq2>{Fq2{h0.X, h1.X}, Fq2{h0.Y, h1.Y}};
 }
 
+// An infinite intermediate point is marked by a top word no canonical
+// coordinate has, so that loading x alone shows it.
+__device__ __forceinline__ bool is_marker(const Fq& x) { return x.v[7] == 0xffffffffu; }
+__device__ __forceinline__ bool is_marker(const Fq2& x) { return is_marker(x.c0); }
+template <class F> __device__ __forceinline__ F marker();
+template <> __device__ __forceinline__ Fq marker<Fq>() { Fq m = Fq::zero(); m.v[7] = 0xffffffffu; return m; }
+template <> __device__ __forceinline__ Fq2 marker<Fq2>() { return {marker<Fq>(), Fq::zero()}; }
+template <>
+__device__ __forceinline__ Aff<Fq> load_raw<Fq, kLayoutPoints>(const void* bases, uint32_t idx)
+{
+    Aff<Fq> a = ldg_elem(reinterpret_cast<const Aff<Fq>*>(bases) + idx);
+    return is_marker(a.x) ? Aff<Fq>{Fq::zero(), Fq::zero()} : a;
+}
+template <>
+__device__ __forceinline__ Aff<Fq2> load_raw<Fq2, kLayoutPoints>(const void* bases, uint32_t idx)
+{
+    Aff<Fq2> a = ldg_elem(reinterpret_cast<const Aff<Fq2>*>(bases) + idx);
+    return is_marker(a.x) ? Aff<Fq2>{Fq2::zero(), Fq2::zero()} : a;
+}
+
 template <class F, int LAYOUT>
 __device__ __forceinline__ Aff<F> load_base(const void* bases, uint32_t v)
 {
@@ -164,22 +302,23 @@ __device__ __forceinline__ Aff<F> load_base(const void* bases, uint32_t v)
 }
 
 // The work of one accumulation thread, chunk t (k_accumulate below; the
-// persistent batch kernel runs it too).
+// persistent batch kernel runs it too).  The list is the sorted entries, or
+// (kLayoutPoints) the points that `shift` affine rounds left of them.
 template <class F, int LAYOUT>
 __device__ __forceinline__ void accumulate_chunk(uint64_t t, const void* __restrict__ bases,
                                                  const uint32_t* __restrict__ ent, const uint32_t* __restrict__ off,
-                                                 uint32_t B, size_t chunks, uint32_t chunk, uint64_t nbases,
-                                                 XYZZ<F>* __restrict__ bsum, XYZZ<F>* __restrict__ head,
-                                                 XYZZ<F>* __restrict__ tail)
+                                                 uint32_t B, size_t chunks, uint32_t chunk, uint32_t shift,
+                                                 uint64_t nbases, XYZZ<F>* __restrict__ bsum,
+                                                 XYZZ<F>* __restrict__ head, XYZZ<F>* __restrict__ tail)
 {
     (void)nbases;   // the base records behind the entries (debug checks)
     if (t >= chunks) return;
-    uint32_t T = off[B];
+    uint32_t T = off[B] >> shift;
     uint64_t cs64 = t * chunk;
     if (cs64 >= T) return;
     uint32_t cs = (uint32_t)cs64, ce = (uint32_t)min((uint64_t)cs + chunk, (uint64_t)T);
-    uint32_t b = bucket_of(off, 0, B, cs);
-    uint32_t bbeg = off[b], bend = off[b + 1];
+    uint32_t b = bucket_of(off, 0, B, cs, shift);
+    uint32_t bbeg = off[b] >> shift, bend = off[b + 1] >> shift;
     XYZZ<F> acc = xyzz_inf<F>();
     for (uint32_t e = cs; e < ce; e++) {
         if (e == bend) {
@@ -192,15 +331,15 @@ __device__ __forceinline__ void accumulate_chunk(uint64_t t, const void* __restr
             // e < off[B], b + 1 < B and off[b + 2] exists.
             if (!LZK_CHECK(b + 2 <= B, 3)) return;
             bbeg = bend;
-            bend = off[b + 2];
+            bend = off[b + 2] >> shift;
             b = b + 1;
             if (bend <= e) {
-                b = bucket_of(off, b + 1, B, e);
-                bbeg = off[b]; bend = off[b + 1];
+                b = bucket_of(off, b + 1, B, e, shift);
+                bbeg = off[b] >> shift; bend = off[b + 1] >> shift;
             }
             acc = xyzz_inf<F>();
         }
-        const uint32_t v = ent[e];
+        const uint32_t v = LAYOUT == kLayoutPoints ? e : ent[e];
         if (!LZK_CHECK((v & 0x7fffffffu) < nbases, 2)) continue;
         acc = xyzz_madd(acc, load_base<F, LAYOUT>(bases, v));
     }
@@ -217,20 +356,21 @@ __device__ __forceinline__ void accumulate_chunk(uint64_t t, const void* __restr
 template <class F, int LAYOUT>
 __global__ void __launch_bounds__(128, sizeof(F) == 32 ? 3 : 2) k_accumulate(const void* __restrict__ bases, const uint32_t* __restrict__ ent,
                                                     const uint32_t* __restrict__ off, uint32_t B, size_t chunks,
-                                                    uint32_t chunk, uint64_t nbases, XYZZ<F>* __restrict__ bsum,
-                                                    XYZZ<F>* __restrict__ head, XYZZ<F>* __restrict__ tail)
+                                                    uint32_t chunk, uint32_t shift, uint64_t nbases,
+                                                    XYZZ<F>* __restrict__ bsum, XYZZ<F>* __restrict__ head,
+                                                    XYZZ<F>* __restrict__ tail)
 {
-    accumulate_chunk<F, LAYOUT>(gtid(), bases, ent, off, B, chunks, chunk, nbases, bsum, head, tail);
+    accumulate_chunk<F, LAYOUT>(gtid(), bases, ent, off, B, chunks, chunk, shift, nbases, bsum, head, tail);
 }
 
 template <class F>
-__device__ __forceinline__ void fixup_items(const uint32_t* __restrict__ off, uint32_t B, uint32_t chunk, uint64_t chunks,
-                        XYZZ<F>* __restrict__ bsum, const XYZZ<F>* __restrict__ head, const XYZZ<F>* __restrict__ tail,
+__device__ __forceinline__ void fixup_items(const uint32_t* __restrict__ off, uint32_t B, uint32_t chunk, uint32_t shift,
+                        uint64_t chunks, XYZZ<F>* __restrict__ bsum, const XYZZ<F>* __restrict__ head, const XYZZ<F>* __restrict__ tail,
                         uint32_t* __restrict__ large)
 {
     (void)chunks;
     for (uint64_t b = gtid(); b < B; b += gstride()) {
-        uint32_t s = off[b], e = off[b + 1];
+        uint32_t s = off[b] >> shift, e = off[b + 1] >> shift;
         if (s == e) continue;
         uint32_t c0 = s / chunk, c1 = (e - 1) / chunk;
         if (!LZK_CHECK(c1 < chunks, 4)) continue;
@@ -245,11 +385,11 @@ __device__ __forceinline__ void fixup_items(const uint32_t* __restrict__ off, ui
     }
 }
 template <class F>
-__global__ void k_fixup(const uint32_t* __restrict__ off, uint32_t B, uint32_t chunk, uint64_t chunks,
+__global__ void k_fixup(const uint32_t* __restrict__ off, uint32_t B, uint32_t chunk, uint32_t shift, uint64_t chunks,
                         XYZZ<F>* __restrict__ bsum, const XYZZ<F>* __restrict__ head, const XYZZ<F>* __restrict__ tail,
                         uint32_t* __restrict__ large)
 {
-    fixup_items<F>(off, B, chunk, chunks, bsum, head, tail, large);
+    fixup_items<F>(off, B, chunk, shift, chunks, bsum, head, tail, large);
 }
 
 // One block per listed bucket: strided partial sums, then a tree in shared
@@ -257,7 +397,7 @@ __global__ void k_fixup(const uint32_t* __restrict__ off, uint32_t B, uint32_t c
 // (blockDim.x points of shared memory at sm; the persistent batch kernel
 // runs it too)
 template <class F>
-__device__ __forceinline__ void fixup_large_items(const uint32_t* __restrict__ off, uint32_t chunk,
+__device__ __forceinline__ void fixup_large_items(const uint32_t* __restrict__ off, uint32_t chunk, uint32_t shift,
                                                   XYZZ<F>* __restrict__ bsum, const XYZZ<F>* __restrict__ head,
                                                   const XYZZ<F>* __restrict__ tail, const uint32_t* __restrict__ large,
                                                   XYZZ<F>* sm)
@@ -265,7 +405,7 @@ __device__ __forceinline__ void fixup_large_items(const uint32_t* __restrict__ o
     uint32_t nl = large[0];
     for (uint32_t idx = blockIdx.x; idx < nl; idx += gridDim.x) {
         uint32_t b = large[1 + idx];
-        uint32_t c0 = off[b] / chunk, c1 = (off[b + 1] - 1) / chunk;
+        uint32_t c0 = (off[b] >> shift) / chunk, c1 = ((off[b + 1] >> shift) - 1) / chunk;
         uint32_t np = c1 - c0 + 1;
         XYZZ<F> acc = xyzz_inf<F>();
         for (uint32_t q = threadIdx.x; q < np; q += blockDim.x)
@@ -281,12 +421,12 @@ __device__ __forceinline__ void fixup_large_items(const uint32_t* __restrict__ o
     }
 }
 template <class F>
-__global__ void k_fixup_large(const uint32_t* __restrict__ off, uint32_t chunk, XYZZ<F>* __restrict__ bsum,
+__global__ void k_fixup_large(const uint32_t* __restrict__ off, uint32_t chunk, uint32_t shift, XYZZ<F>* __restrict__ bsum,
                               const XYZZ<F>* __restrict__ head, const XYZZ<F>* __restrict__ tail,
                               const uint32_t* __restrict__ large)
 {
     extern __shared__ uint4 fx_raw[];
-    fixup_large_items<F>(off, chunk, bsum, head, tail, large, reinterpret_cast<XYZZ<F>*>(fx_raw));
+    fixup_large_items<F>(off, chunk, shift, bsum, head, tail, large, reinterpret_cast<XYZZ<F>*>(fx_raw));
 }
 
 // Warp shuffles of whole points
@@ -599,16 +739,26 @@ __global__ void k_write_inf(Jac<F>* out)
     if (gtid() == 0) st_elem(out, Jac<F>{F::zero(), F::one(), F::zero()});
 }
 
+// affine rounds of an MSM over bases in this layout
+inline uint32_t msm_rounds(size_t n, uint32_t c, bool shared, uint32_t layout)
+{
+    const size_t W = windows_for(c);
+    return layout == LZK_BASES_AFFINE ? affine_rounds(n * W, (shared ? 1 : W) << (c - 1)) : 0;
+}
+
 // pre_off / pre_ent: bucket offsets and sorted entries of these scalars made
 // earlier by msm_sort for the same n, window width and table stride (MSMs
-// over the same scalars share one sort); null = sort here.
+// over the same scalars share one sort, padded for pre_rounds affine rounds);
+// null = sort here.
 template <class Gp>
 int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>* out,
                    const lzk_msm_cfg* cfg, cudaStream_t st, uint32_t c_auto,
-                   const uint32_t* pre_off = nullptr, const uint32_t* pre_ent = nullptr)
+                   const uint32_t* pre_off = nullptr, const uint32_t* pre_ent = nullptr, uint32_t pre_rounds = 0,
+                   bool pre_in_ws = false)
 {
     using F = typename Gp::F;
     using X = XYZZ<F>;
+    using A = Aff<F>;
     if (!out || (n && (!scalars || !bases))) return LZK_EINVAL;
     if (n >= (1ull << 31)) return LZK_EINVAL;
     uint32_t flags = cfg ? cfg->flags : 0u;
@@ -632,10 +782,17 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
     uint32_t chunk = msm_chunk(cfg, group, n), run = msm_run(cfg, group, n);
     if (!tune_valid(LZK_TUNE_MSM_CHUNK, chunk) || !tune_valid(LZK_TUNE_MSM_REDUCE_RUN, run)) return LZK_EINVAL;
     MsmPlan p;
-    plan_msm<Gp>(p, n, c, shared, stride, chunk, run);
+    plan_msm<Gp>(p, n, c, shared, stride, chunk, run, pre_off ? pre_rounds : msm_rounds(n, c, shared, layout),
+                 pre_off && !pre_in_ws);
     void* tr_all = trace_begin(sizeof(F) == 32 ? "msm_g1" : "msm_g2", st);
     Scratch ws;
-    LZK_TRY(ws.acquire(p.bytes, cfg ? cfg->workspace : nullptr, cfg ? cfg->workspace_bytes : 0, st));
+    int got = ws.acquire(p.bytes, cfg ? cfg->workspace : nullptr, cfg ? cfg->workspace_bytes : 0, st);
+    if (got != LZK_OK && p.rounds && !pre_off) {
+        // too little scratch for the affine rounds: XYZZ additions alone
+        plan_msm<Gp>(p, n, c, shared, stride, chunk, run);
+        got = ws.acquire(p.bytes, cfg ? cfg->workspace : nullptr, cfg ? cfg->workspace_bytes : 0, st);
+    }
+    LZK_TRY(got);
     char* base = ws.base;
     uint32_t* cnt = reinterpret_cast<uint32_t*>(base + p.o_cnt);
     uint32_t* off_ws = reinterpret_cast<uint32_t*>(base + p.o_off);
@@ -661,19 +818,24 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
         // base records the entries may name: the whole table, or the n bases
         const uint64_t nbases = shared ? (uint64_t)cfg->precomp_windows * stride : (uint64_t)n;
         constexpr int REF = sizeof(F) == 32 ? (int)LZK_BASES_REF_G1_JAC : (int)LZK_BASES_REF_G2_LANES;
-        if (layout == LZK_BASES_AFFINE) {
-            k_accumulate<F, LZK_BASES_AFFINE><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, nbases, bsum, head, tail); note_launch();
+        if (p.rounds) {
+            A* fin = reinterpret_cast<A*>(base + p.o_fin);
+            LZK_TRY(affine_sum<F>(bases, ent, off + p.B, p.max_slots, p.slice, p.rounds, nbases,
+                                  base + p.o_aff, fin, st));
+            k_accumulate<F, kLayoutPoints><<<g, 128, 0, st>>>(fin, ent, off, p.B, p.chunks, p.chunk, p.rounds, p.max_slots >> p.rounds, bsum, head, tail); note_launch();
+        } else if (layout == LZK_BASES_AFFINE) {
+            k_accumulate<F, LZK_BASES_AFFINE><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, 0, nbases, bsum, head, tail); note_launch();
         } else {
-            k_accumulate<F, REF><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, nbases, bsum, head, tail); note_launch();
+            k_accumulate<F, REF><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, 0, nbases, bsum, head, tail); note_launch();
         }
     }
     trace_end(tr, st);
     void* tr_fix = trace_begin(sizeof(F) == 32 ? "msm_g1_fixup" : "msm_g2_fixup", st);
     LZK_CUDA(cudaMemsetAsync(large, 0, sizeof(uint32_t), st));
-    k_fixup<F><<<grid_for(p.B, 256, sm_count() * 8), 256, 0, st>>>(off, p.B, p.chunk, p.chunks, bsum, head, tail, large); note_launch();
+    k_fixup<F><<<grid_for(p.B, 256, sm_count() * 8), 256, 0, st>>>(off, p.B, p.chunk, p.rounds, p.chunks, bsum, head, tail, large); note_launch();
     {
         constexpr unsigned fx_threads = 32768 / sizeof(X);   // 32 KB of shared memory
-        k_fixup_large<F><<<sm_count() * 2, fx_threads, fx_threads * sizeof(X), st>>>(off, p.chunk, bsum, head, tail, large); note_launch();
+        k_fixup_large<F><<<sm_count() * 2, fx_threads, fx_threads * sizeof(X), st>>>(off, p.chunk, p.rounds, bsum, head, tail, large); note_launch();
     }
     trace_end(tr_fix, st);
     LZK_TRY(launch_status());

@@ -8,14 +8,14 @@ namespace lzk {
 uint32_t debug_word_g1(bool clear) { return debug_word_here(clear); }
 
 int msm_g1_presorted(const Fr* scalars, const void* table, size_t n, Jac<Fq>* out, const lzk_msm_cfg* cfg,
-                     cudaStream_t st, const uint32_t* off, const uint32_t* ent)
+                     cudaStream_t st, const uint32_t* off, const uint32_t* ent, uint32_t rounds)
 {
     if (!cfg || !(cfg->flags & LZK_MSM_PRECOMPUTED) || !off || !ent) return LZK_EINVAL;
-    return run_msm<G1>(scalars, table, n, out, cfg, st, cfg->window_bits, off, ent);
+    return run_msm<G1>(scalars, table, n, out, cfg, st, cfg->window_bits, off, ent, rounds);
 }
 
 int msm_g1_concat(const Fr* lo, size_t n_lo, const Fr* hi, size_t n_hi, const void* table, Jac<Fq>* out,
-                  const lzk_msm_cfg* cfg, cudaStream_t st)
+                  const lzk_msm_cfg* cfg, cudaStream_t st, uint32_t rounds)
 {
     size_t n = n_lo + n_hi;
     if (!cfg || !(cfg->flags & LZK_MSM_PRECOMPUTED) || !cfg->workspace || !out || !table) return LZK_EINVAL;
@@ -24,7 +24,7 @@ int msm_g1_concat(const Fr* lo, size_t n_lo, const Fr* hi, size_t n_hi, const vo
     if (c < 2 || c > 24 || cfg->precomp_windows < windows_for(c) || cfg->level_stride < n) return LZK_EINVAL;
     if ((size_t)windows_for(c) * cfg->level_stride >= (1ull << 31)) return LZK_EINVAL;
     MsmPlan p;
-    plan_msm<G1>(p, n, c, true, cfg->level_stride, msm_chunk(cfg, 1, n), msm_run(cfg, 1, n));
+    plan_msm<G1>(p, n, c, true, cfg->level_stride, msm_chunk(cfg, 1, n), msm_run(cfg, 1, n), rounds);
     if (cfg->workspace_bytes < p.bytes) return LZK_EINVAL;
     // sort into the workspace at the offsets run_msm carves from it
     char* base = static_cast<char*>(cfg->workspace);
@@ -34,7 +34,7 @@ int msm_g1_concat(const Fr* lo, size_t n_lo, const Fr* hi, size_t n_hi, const vo
     LZK_TRY(msm_sort(p, n_lo ? lo : hi, reinterpret_cast<uint32_t*>(base + p.o_cnt), off, ent,
                      reinterpret_cast<uint32_t*>(base + p.o_scan), st, hi, n_lo));
     trace_end(tr, st);
-    return run_msm<G1>(n_lo ? lo : hi, table, n, out, cfg, st, c, off, ent);
+    return run_msm<G1>(n_lo ? lo : hi, table, n, out, cfg, st, c, off, ent, rounds, true);
 }
 }  // namespace lzk
 

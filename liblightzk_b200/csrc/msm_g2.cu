@@ -8,10 +8,10 @@ namespace lzk {
 uint32_t debug_word_g2(bool clear) { return debug_word_here(clear); }
 
 int msm_g2_presorted(const Fr* scalars, const void* table, size_t n, Jac<Fq2>* out, const lzk_msm_cfg* cfg,
-                     cudaStream_t st, const uint32_t* off, const uint32_t* ent)
+                     cudaStream_t st, const uint32_t* off, const uint32_t* ent, uint32_t rounds)
 {
     if (!cfg || !(cfg->flags & LZK_MSM_PRECOMPUTED) || !off || !ent) return LZK_EINVAL;
-    return run_msm<G2>(scalars, table, n, out, cfg, st, cfg->window_bits, off, ent);
+    return run_msm<G2>(scalars, table, n, out, cfg, st, cfg->window_bits, off, ent, rounds);
 }
 }  // namespace lzk
 

@@ -36,7 +36,7 @@
 // every call (the array's name in host code is only a stand-in and must
 // never be handed to a kernel); once the module is loaded the lookup is a
 // table read.
-#include "common.cuh"
+#include "msm.cuh"
 #include <mutex>
 
 namespace lzk {
@@ -98,14 +98,16 @@ int lzk_msm_g1_noalloc(const lzk_fr_t* scalars, const lzk_g1_affine_t* bases, si
     if (n > LZK_MSM_NOALLOC_MAX_POINTS) return LZK_EINVAL;
     lzk_msm_cfg cfg = {};
     cfg.window_bits = window_bits;
-    size_t need = lzk_msm_workspace_bytes(1, n, &cfg);
+    // without the affine rounds: their scratch does not fit the array at every
+    // size it takes, and the set-up loads only the kernels of this form
+    size_t need = msm_lean_bytes(n, &cfg);
     if (need > LZK_MSM_NOALLOC_SCRATCH_BYTES) return LZK_EINVAL;
     void* scratch = nullptr;
     int dev = 0;
     LZK_TRY(noalloc_scratch(&scratch, &dev));
     LZK_TRY(noalloc_setup(static_cast<char*>(scratch), dev, as_stream(stream)));
     cfg.workspace = scratch;
-    cfg.workspace_bytes = LZK_MSM_NOALLOC_SCRATCH_BYTES;
+    cfg.workspace_bytes = need;
     return lzk_msm_g1(scalars, bases, n, out, &cfg, stream);
 }
 

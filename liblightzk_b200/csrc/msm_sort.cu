@@ -7,9 +7,12 @@
 //                  (window, |digit|) buckets (global atomics).
 //   2. k_scan_*    exclusive prefix sum -> bucket offsets; off[B] = entries.
 //   3. k_scatter   counting-sort scatter of (point index, sign) entries.
-//   4. k_accumulate each thread adds exactly K consecutive sorted entries
-//                  (XYZZ mixed adds of affine bases), so the work is even
-//                  whatever the bucket sizes; segments that cross a chunk
+//      (long lists) the affine rounds: pairs of a bucket's entries added in
+//                  affine form with batched inversions, halving the list each
+//                  round (affine.cuh).
+//   4. k_accumulate each thread adds exactly K consecutive sorted entries, or
+//                  points the rounds left (XYZZ mixed adds), so the work is
+//                  even whatever the bucket sizes; segments that cross a chunk
 //                  boundary leave partial sums.
 //   5. k_fixup     folds those partial sums into their buckets: one thread
 //                  per bucket with at most kFixSmall partials, one block and
@@ -107,8 +110,8 @@ __global__ void k_scatter(const Fr* __restrict__ scalars, const Fr* __restrict__
     }
 }
 
-// Exclusive scan of cnt[0..B) into off[0..B], off[B] = total, in three
-// passes: per-block scans of 4096 counters (1024 threads x 4), a scan of the
+// Exclusive scan of cnt[0..B), each count rounded up to a multiple of
+// pad + 1 (a power of two), into off[0..B], off[B] = total, in three passes: per-block scans of 4096 counters (1024 threads x 4), a scan of the
 // block totals in one block, and the add-back of each block's offset.
 constexpr uint32_t kScanBlock = 4096;
 
@@ -132,12 +135,13 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t x, uint32_t* w
 }
 
 __global__ void __launch_bounds__(1024) k_scan_local(const uint32_t* __restrict__ cnt, uint32_t B,
-                                                     uint32_t* __restrict__ off, uint32_t* __restrict__ bsums)
+                                                     uint32_t* __restrict__ off, uint32_t* __restrict__ bsums,
+                                                     uint32_t pad)
 {
     __shared__ uint32_t warp_tot[32];
     uint32_t base = blockIdx.x * kScanBlock + threadIdx.x * 4;
     uint32_t v[4];
-    for (int i = 0; i < 4; i++) v[i] = (base + i < B) ? cnt[base + i] : 0u;
+    for (int i = 0; i < 4; i++) v[i] = (base + i < B) ? (cnt[base + i] + pad) & ~pad : 0u;
     uint32_t sum = v[0] + v[1] + v[2] + v[3], total;
     uint32_t run = block_exclusive_scan(sum, warp_tot, total);
     for (int i = 0; i < 4; i++) {
@@ -167,11 +171,11 @@ __global__ void k_scan_add(uint32_t* __restrict__ off, uint32_t B, const uint32_
     for (uint64_t i = gtid(); i < B; i += gstride()) off[i] += bsums[i / kScanBlock];
 }
 
-int scan_offsets(const uint32_t* cnt, uint32_t B, uint32_t* off, uint32_t* bsums, cudaStream_t st)
+int scan_offsets(const uint32_t* cnt, uint32_t B, uint32_t* off, uint32_t* bsums, cudaStream_t st, uint32_t rounds)
 {
     uint32_t nblk = (B + kScanBlock - 1) / kScanBlock;
     if (nblk == 0) nblk = 1;
-    k_scan_local<<<nblk, 1024, 0, st>>>(cnt, B, off, bsums); note_launch();
+    k_scan_local<<<nblk, 1024, 0, st>>>(cnt, B, off, bsums, (1u << rounds) - 1); note_launch();
     k_scan_top<<<1, 1024, 0, st>>>(bsums, nblk, off, B); note_launch();
     k_scan_add<<<grid_for(B, 256, sm_count() * 8), 256, 0, st>>>(off, B, bsums); note_launch();
     return launch_status();
@@ -185,10 +189,9 @@ int msm_sort(const MsmPlan& p, const Fr* scalars, uint32_t* cnt, uint32_t* off, 
     LZK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * p.B, st));
     unsigned g = grid_for(p.n, 256, sm_count() * 16);
     k_count<<<g, 256, 0, st>>>(scalars, hi, split, p.n, p.c, p.W, p.nb, p.shared, cnt); note_launch();
-    uint32_t nblk = (p.B + kScanBlock - 1) / kScanBlock;
-    k_scan_local<<<nblk, 1024, 0, st>>>(cnt, p.B, off, bsums); note_launch();
-    k_scan_top<<<1, 1024, 0, st>>>(bsums, nblk, off, p.B); note_launch();
-    k_scan_add<<<grid_for(p.B, 256, sm_count() * 8), 256, 0, st>>>(off, p.B, bsums); note_launch();
+    LZK_TRY(scan_offsets(cnt, p.B, off, bsums, st, p.rounds));
+    // the gaps that pad buckets keep kNoEntry
+    if (p.rounds) LZK_CUDA(cudaMemsetAsync(ent, 0xff, sizeof(uint32_t) * p.max_slots, st));
     k_scatter<<<g, 256, 0, st>>>(scalars, hi, split, p.n, p.c, p.W, p.nb, p.shared, p.stride, off, cnt, ent); note_launch();
     return launch_status();
 }
@@ -218,23 +221,48 @@ uint32_t msm_autotune(int group, size_t n, bool shared)
     return bc;
 }
 
-SortWords msm_sort_words(size_t n, uint32_t c, size_t stride)
+SortWords msm_sort_words(size_t n, uint32_t c, size_t stride, uint32_t rounds)
 {
     MsmPlan p;
-    plan_msm<G1>(p, n, c, true, stride);
-    return SortWords{p.B, (size_t)p.B + 1, p.max_entries ? p.max_entries : 1, (p.B + 4095) / 4096 + 1};
+    plan_msm<G1>(p, n, c, true, stride, kDefaultChunk, kDefaultRun, rounds);
+    return SortWords{p.B, (size_t)p.B + 1, p.max_slots ? p.max_slots : 1, (p.B + 4095) / 4096 + 1};
 }
 
 int msm_sort_scalars(const Fr* scalars, size_t n, uint32_t c, size_t stride, uint32_t* cnt, uint32_t* off,
-                     uint32_t* ent, uint32_t* bsums, cudaStream_t st)
+                     uint32_t* ent, uint32_t* bsums, cudaStream_t st, uint32_t rounds)
 {
     if (!n || c < 2 || c > 24 || stride < n) return LZK_EINVAL;
     MsmPlan p;
-    plan_msm<G1>(p, n, c, true, stride);
+    plan_msm<G1>(p, n, c, true, stride, kDefaultChunk, kDefaultRun, rounds);
     void* tr = trace_begin("msm_shared_sort", st);
     int rc = msm_sort(p, scalars, cnt, off, ent, bsums, st);
     trace_end(tr, st);
     return rc;
+}
+
+size_t msm_presorted_bytes(int group, size_t n, const lzk_msm_cfg* cfg, uint32_t rounds)
+{
+    MsmPlan p;
+    const uint32_t chunk = msm_chunk(cfg, group, n), run = msm_run(cfg, group, n);
+    if (group == 2) plan_msm<G2>(p, n, cfg->window_bits, true, cfg->level_stride, chunk, run, rounds, true);
+    else plan_msm<G1>(p, n, cfg->window_bits, true, cfg->level_stride, chunk, run, rounds, true);
+    return p.bytes;
+}
+
+size_t msm_concat_bytes(size_t n, const lzk_msm_cfg* cfg, uint32_t rounds)
+{
+    MsmPlan p;
+    plan_msm<G1>(p, n, cfg->window_bits, true, cfg->level_stride, msm_chunk(cfg, 1, n), msm_run(cfg, 1, n), rounds);
+    return p.bytes;
+}
+
+size_t msm_lean_bytes(size_t n, const lzk_msm_cfg* cfg)
+{
+    const uint32_t c = cfg->window_bits ? cfg->window_bits : msm_autotune(1, n, false);
+    if (c < 2 || c > 24 || n == 0) return 0;
+    MsmPlan p;
+    plan_msm<G1>(p, n, c, false, 0, msm_chunk(cfg, 1, n), msm_run(cfg, 1, n));
+    return p.bytes;
 }
 
 uint32_t debug_word_sort(bool clear) { return debug_word_here(clear); }
@@ -260,8 +288,9 @@ size_t lzk_msm_workspace_bytes(int group, size_t n, const lzk_msm_cfg* cfg)
     uint32_t chunk = msm_chunk(cfg, group, n), run = msm_run(cfg, group, n);
     if (!tune_valid(LZK_TUNE_MSM_CHUNK, chunk)) return 0;
     MsmPlan p;
-    if (group == 2) plan_msm<G2>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run);
-    else plan_msm<G1>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run);
+    const uint32_t rounds = msm_rounds(n, c, shared, cfg ? cfg->base_layout : (uint32_t)LZK_BASES_AFFINE);
+    if (group == 2) plan_msm<G2>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run, rounds);
+    else plan_msm<G1>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run, rounds);
     return p.bytes;
 }
 

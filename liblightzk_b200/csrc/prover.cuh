@@ -1,6 +1,7 @@
 // prover.cuh -- the Groth16 prover's resident state and per-proof contexts,
 // shared by the prove chain (groth16.cu) and the serving loop (server.cu).
 #pragma once
+#include <mutex>
 #include "common.cuh"
 #include "curve.cuh"
 #include "r1cs.cuh"
@@ -33,6 +34,8 @@ struct ProveCtx {
     cudaStream_t s0 = nullptr, s1 = nullptr, s2 = nullptr, s3 = nullptr;   // s0: serving contexts only
     cudaEvent_t ev_fork = nullptr, ev_b1 = nullptr, ev_s1 = nullptr, ev_s2 = nullptr, ev_s3 = nullptr,
                 ev_sorted = nullptr;
+    uint32_t lh_rounds = 0, z_rounds = 0;   // affine rounds of the L + H MSM; of A, B1 and B2
+    bool lean = false;                // no affine rounds (affine.cuh): a third of the scratch, slower
     size_t bytes = 0;
 };
 
@@ -64,12 +67,17 @@ struct lzk_prover {
     lzk::Aff<lzk::Fq2>* comb2 = nullptr;  // comb table of d2
     lzk::ProveCtx* ctx0 = nullptr;
     size_t bytes = 0;       // resident bytes (tables, constants)
+    std::mutex mu;          // held while ctx0 is used to enqueue or replaced
 };
 
 namespace lzk {
 
-// scratch (and, for serving, streams and witness/proof buffers) of one proof
-int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out);
+// scratch (and, for serving, streams and witness/proof buffers) of one proof;
+// ctx_bytes: what it will hold
+int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out, bool lean = false);
+size_t ctx_bytes(const lzk_prover* p, bool serving, bool lean);
+// replace the prover's own context by a lean one
+int prover_make_lean(lzk_prover* p);
 void ctx_destroy(ProveCtx* x);
 // enqueue one proof on stream st using context x (x's side streams join st)
 int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, const lzk_fr_t* s,

@@ -48,7 +48,6 @@ struct Request {
 struct Circuit {
     lzk_prover* prover = nullptr;
     std::vector<ProveCtx*> idle;
-    size_t ctx_bytes = 0;   // bytes of one context (0 until the first is made)
     size_t live = 0;        // contexts allocated (idle + running)
 };
 
@@ -109,22 +108,17 @@ ProveCtx* get_ctx(lzk_server* s, uint32_t c, bool* never)
         ci.idle.pop_back();
         return x;
     }
-    size_t need = ci.ctx_bytes;
-    if (need && s->resident_bytes + need > s->cfg.hbm_budget_bytes) { *never = true; return nullptr; }
-    if (need && !make_room(s, c, need)) return nullptr;
+    // a context with the affine rounds' scratch where it fits, else a lean one
     ProveCtx* x = nullptr;
-    if (lzk::ctx_create(ci.prover, true, &x) != LZK_OK) {
+    for (bool lean : {false, true}) {
+        const size_t need = lzk::ctx_bytes(ci.prover, true, lean);
+        if (lean && s->resident_bytes + need > s->cfg.hbm_budget_bytes) { *never = true; return nullptr; }
+        if (s->resident_bytes + need > s->cfg.hbm_budget_bytes || !make_room(s, c, need)) continue;
+        if (lzk::ctx_create(ci.prover, true, &x, lean) == LZK_OK) break;
         cudaGetLastError();
-        if (!ci.live && !s->ctx_bytes) *never = true;
-        return nullptr;
+        if (lean && !ci.live && !s->ctx_bytes) *never = true;
     }
-    if (!ci.ctx_bytes) ci.ctx_bytes = x->bytes;
-    if (used(s) + x->bytes > s->cfg.hbm_budget_bytes && !make_room(s, c, x->bytes)) {
-        bool alone = s->resident_bytes + x->bytes > s->cfg.hbm_budget_bytes;
-        lzk::ctx_destroy(x);
-        *never = alone;
-        return nullptr;
-    }
+    if (!x) return nullptr;
     s->ctx_bytes += x->bytes;
     ci.live++;
     return x;
@@ -233,7 +227,14 @@ int lzk_server_add_circuit(lzk_server* s, lzk_prover* prover, uint32_t* circuit_
     if (!s || !prover || !circuit_id) return LZK_EINVAL;
     std::lock_guard<std::mutex> g(s->mu);
     size_t rb = lzk_prover_device_bytes(prover);
-    if (s->resident_bytes + rb > s->cfg.hbm_budget_bytes) return LZK_EBUSY;
+    if (s->resident_bytes + rb > s->cfg.hbm_budget_bytes) {
+        // a prover too large with its own context's full scratch may fit with
+        // a lean one
+        const size_t lean = rb - prover->ctx0->bytes + lzk::ctx_bytes(prover, false, true);
+        if (s->resident_bytes + lean > s->cfg.hbm_budget_bytes) return LZK_EBUSY;
+        LZK_TRY(lzk::prover_make_lean(prover));
+        rb = lzk_prover_device_bytes(prover);
+    }
     s->resident_bytes += rb;
     Circuit c;
     c.prover = prover;

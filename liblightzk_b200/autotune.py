@@ -8,7 +8,7 @@ seeded random inputs, median of a few runs) and installs the fastest:
   chunk   sorted bucket entries one accumulation thread adds (32, 64, 128)
   run     buckets per lane run in the bucket-reduction tiles (4, 8, 16)
   ntt     elements per block of an NTT pass, i.e. how a transform's stages
-          split into passes (1024, 2048, 4096)
+          split into passes (256, 512, 1024, 2048)
   table_*  window width, chunk and run of MSMs over shifted-copy tables
           (provers, batch plans with fixed bases)
 
@@ -149,7 +149,7 @@ def tune_msm_table(group=1, log_ns=range(10, 21), spread=(4, 2), reps=3, seed=11
     return out
 
 
-def tune_ntt(log_ns=range(12, 23), reps=3, seed=12, blocks=(1024, 2048, 4096), direction=ntt.COSET_FORWARD):
+def tune_ntt(log_ns=range(12, 23), reps=3, seed=12, blocks=(256, 512, 1024, 2048), direction=ntt.COSET_FORWARD):
     """NTT block size per transform size; installs the fastest and returns
     {log_n: (best, {block: ms})}"""
     out = {}

@@ -6,10 +6,11 @@
 // (w_k = w_28^(2^(28-k)), w_28 = 5^((r-1)/2^28)), and the same radix-2
 // decimation-in-frequency butterfly c[j] = lo + hi, c[j^h] = (lo - hi) *
 // w^((j mod h) << s).  Instead of one global-memory launch per stage, each
-// pass loads 2^m-element groups into shared memory and runs m stages there
-// (ceil(k / 11) passes for a size-2^k transform); a final pass applies the
-// bit-reversal permutation in place together with the scale n^-1 and the
-// coset factor.
+// pass runs m stages on 2^m-element groups, two stages at a time in registers
+// and shared memory between them (ceil(k / 10) passes of about equal m for
+// blocks of 1024 elements); the scale n^-1 and the coset factors are applied
+// as the first pass loads or the last one stores, and a final pass permutes
+// in place into natural order.
 //
 // Directions: forward; inverse (w^-1, then * n^-1); coset forward (a_j *
 // g^j first, g = 5 = Fr::multiplicative_generator, alt_bn128_init.cu:50);
@@ -77,6 +78,12 @@ __global__ void k_powers(const Fr* __restrict__ basep, Fr* __restrict__ out, siz
     }
 }
 
+// out[i] = in[i] * *scale
+__global__ void k_scaled(const Fr* __restrict__ in, const Fr* __restrict__ scale, Fr* __restrict__ out, size_t count)
+{
+    for (uint64_t i = gtid(); i < count; i += gstride()) st_elem(out + i, mul(ldg_elem(in + i), ldg_elem(scale)));
+}
+
 // twiddles in radix-2^52 form: twd[kTwdStride e + i] = limb i of tw[e]
 __global__ void k_tw_to_d52(const Fr* __restrict__ tw, double* __restrict__ twd, size_t count)
 {
@@ -106,50 +113,40 @@ int get_tables(uint32_t k, NttTables& out, CosetTables& cos)
     cudaStream_t st;
     LZK_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     int rc = LZK_OK;
+    const size_t nlo = size_t(1) << kPowLoBits, nhi = size_t(1) << (kNttMaxLog - kPowLoBits);
     if (it == g_ntt_tables.end()) {
         NttTables t;
         size_t half = k ? (size_t(1) << (k - 1)) : 1;
-        if (dev_malloc(reinterpret_cast<void**>(&t.consts), 8 * sizeof(Fr)) != LZK_OK ||
-            dev_malloc(reinterpret_cast<void**>(&t.tw[0]), half * sizeof(Fr)) != LZK_OK ||
-            dev_malloc(reinterpret_cast<void**>(&t.tw[1]), half * sizeof(Fr)) != LZK_OK ||
-            dev_malloc(reinterpret_cast<void**>(&t.twd[0]), half * kTwdStride * sizeof(double)) != LZK_OK ||
-            dev_malloc(reinterpret_cast<void**>(&t.twd[1]), half * kTwdStride * sizeof(double)) != LZK_OK) {
-            cudaFree(t.consts);
-            cudaFree(t.tw[0]);
-            cudaFree(t.tw[1]);
-            cudaFree(t.twd[0]);
-            cudaFree(t.twd[1]);
-            rc = LZK_ENOMEM;
-        } else {
-            k_ntt_consts<<<1, 32, 0, st>>>(k, t.consts); note_launch();
-            k_powers<<<grid_for((half + 63) / 64, 128), 128, 0, st>>>(t.consts + 0, t.tw[0], half); note_launch();
-            k_powers<<<grid_for((half + 63) / 64, 128), 128, 0, st>>>(t.consts + 1, t.tw[1], half); note_launch();
-            for (int d = 0; d < 2; d++) {
-                k_tw_to_d52<<<grid_for(half, 128), 128, 0, st>>>(t.tw[d], t.twd[d], half); note_launch();
-            }
-            rc = cuda_status(cudaStreamSynchronize(st));
-            if (rc == LZK_OK) g_ntt_tables[{dev, k}] = t;
-        }
-    }
-    if (rc == LZK_OK && ct == g_coset_tables.end()) {
+        auto get = [](auto** p, size_t count) { return dev_malloc(reinterpret_cast<void**>(p), count * sizeof(**p)) == LZK_OK; };
+        bool ok = get(&t.consts, 8) && get(&t.tw[0], half) && get(&t.tw[1], half) &&
+                  get(&t.twd[0], half * kTwdStride) && get(&t.twd[1], half * kTwdStride) && get(&t.slo[0], nlo) &&
+                  get(&t.slo[1], nlo);
         CosetTables c;
-        size_t nlo = size_t(1) << kPowLoBits, nhi = size_t(1) << (kNttMaxLog - kPowLoBits);
-        Fr* cst = g_ntt_tables[{dev, k}].consts;
-        bool ok = true;
-        for (int d = 0; d < 2 && ok; d++)
-            ok = dev_malloc(reinterpret_cast<void**>(&c.lo[d]), nlo * sizeof(Fr)) == LZK_OK &&
-                 dev_malloc(reinterpret_cast<void**>(&c.hi[d]), nhi * sizeof(Fr)) == LZK_OK;
-        if (!ok) {
-            for (int d = 0; d < 2; d++) { cudaFree(c.lo[d]); cudaFree(c.hi[d]); }
-            rc = LZK_ENOMEM;
-        }
-        else {
+        const bool coset = ct == g_coset_tables.end();
+        if (!coset) c = ct->second;
+        for (int d = 0; d < 2 && coset; d++) ok = ok && get(&c.lo[d], nlo) && get(&c.hi[d], nhi);
+        if (ok) {
+            k_ntt_consts<<<1, 32, 0, st>>>(k, t.consts); note_launch();
             for (int d = 0; d < 2; d++) {
-                k_powers<<<grid_for(nlo / 64, 128), 128, 0, st>>>(cst + 3 + d, c.lo[d], nlo); note_launch();
-                k_powers<<<grid_for(nhi / 64, 128), 128, 0, st>>>(cst + 5 + d, c.hi[d], nhi); note_launch();
+                k_powers<<<grid_for((half + 63) / 64, 128), 128, 0, st>>>(t.consts + d, t.tw[d], half); note_launch();
+                k_tw_to_d52<<<grid_for(half, 128), 128, 0, st>>>(t.tw[d], t.twd[d], half); note_launch();
+                if (coset) {
+                    k_powers<<<grid_for(nlo / 64, 128), 128, 0, st>>>(t.consts + 3 + d, c.lo[d], nlo); note_launch();
+                    k_powers<<<grid_for(nhi / 64, 128), 128, 0, st>>>(t.consts + 5 + d, c.hi[d], nhi); note_launch();
+                }
+                k_scaled<<<grid_for(nlo, 128), 128, 0, st>>>(c.lo[d], t.consts + 2, t.slo[d], nlo); note_launch();
             }
             rc = cuda_status(cudaStreamSynchronize(st));
-            if (rc == LZK_OK) g_coset_tables[dev] = c;
+        } else {
+            rc = LZK_ENOMEM;
+        }
+        if (rc == LZK_OK) {
+            g_ntt_tables[{dev, k}] = t;
+            g_coset_tables[dev] = c;
+        } else {
+            void* mine[] = {t.consts, t.tw[0], t.tw[1], t.twd[0], t.twd[1], t.slo[0], t.slo[1]};
+            for (auto m : mine) cudaFree(m);
+            for (int d = 0; d < 2 && coset; d++) { cudaFree(c.lo[d]); cudaFree(c.hi[d]); }
         }
     }
     cudaStreamDestroy(st);
@@ -161,33 +158,147 @@ int get_tables(uint32_t k, NttTables& out, CosetTables& cos)
 
 struct NttPass {
     uint32_t k, s0, m, lowbits, R;
+    uint32_t canon;     // the last pass: canonical results
+    uint32_t natural;   // a DIF transform of one pass (one block), written in natural order
 };
-
-__device__ __forceinline__ Fr coset_pow(const Fr* lo, const Fr* hi, size_t j)
-{
-    return mul(ldg_elem(lo + (j & ((1u << kPowLoBits) - 1))), ldg_elem(hi + (j >> kPowLoBits)));
-}
 
 __device__ __forceinline__ size_t brev_k(size_t j, uint32_t k)
 {
     return k ? (size_t)(__brevll((unsigned long long)j) >> (64 - k)) : 0;
 }
 
+// ---------------- lazily reduced values ----------------
+// Inside a pass a value stays below 2p (DIF) or 4p (DIT) instead of p: the
+// FP64 product takes operands below 4p (times a table value below 2p) and
+// leaves a result below 2p, so a butterfly needs one conditional subtraction
+// instead of three.
+__host__ __device__ constexpr uint32_t fr_2p(int i) { return (FrP::p(i) << 1) | (i ? FrP::p(i - 1) >> 31 : 0u); }
+
+// a + b, no reduction
+__device__ __forceinline__ Fr add_raw(const Fr& a, const Fr& b)
+{
+    Fr r;
+    add_nored(r.v, a.v, b.v);
+    return r;
+}
+// x < 4p to x mod 2p
+__device__ __forceinline__ Fr red_2p(const Fr& x)
+{
+    uint32_t s[8], br;
+    asm("sub.cc.u32  %0, %9,  %17;\n\t"
+        "subc.cc.u32 %1, %10, %18;\n\t"
+        "subc.cc.u32 %2, %11, %19;\n\t"
+        "subc.cc.u32 %3, %12, %20;\n\t"
+        "subc.cc.u32 %4, %13, %21;\n\t"
+        "subc.cc.u32 %5, %14, %22;\n\t"
+        "subc.cc.u32 %6, %15, %23;\n\t"
+        "subc.cc.u32 %7, %16, %24;\n\t"
+        "subc.u32    %8, 0, 0;"
+        : "=r"(s[0]), "=r"(s[1]), "=r"(s[2]), "=r"(s[3]), "=r"(s[4]), "=r"(s[5]), "=r"(s[6]), "=r"(s[7]), "=r"(br)
+        : "r"(x.v[0]), "r"(x.v[1]), "r"(x.v[2]), "r"(x.v[3]), "r"(x.v[4]), "r"(x.v[5]), "r"(x.v[6]), "r"(x.v[7]),
+          "n"(fr_2p(0)), "n"(fr_2p(1)), "n"(fr_2p(2)), "n"(fr_2p(3)), "n"(fr_2p(4)), "n"(fr_2p(5)), "n"(fr_2p(6)), "n"(fr_2p(7)));
+    Fr r;
+    _Pragma("unroll") for (int i = 0; i < 8; i++) r.v[i] = br ? x.v[i] : s[i];
+    return r;
+}
+// a + 2p - b for a, b < 2p: in (0, 4p)
+__device__ __forceinline__ Fr sub_2p(const Fr& a, const Fr& b)
+{
+    uint32_t t[8];
+    asm("add.cc.u32  %0, %8,  %16;\n\t"
+        "addc.cc.u32 %1, %9,  %17;\n\t"
+        "addc.cc.u32 %2, %10, %18;\n\t"
+        "addc.cc.u32 %3, %11, %19;\n\t"
+        "addc.cc.u32 %4, %12, %20;\n\t"
+        "addc.cc.u32 %5, %13, %21;\n\t"
+        "addc.cc.u32 %6, %14, %22;\n\t"
+        "addc.u32    %7, %15, %23;"
+        : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
+        : "r"(a.v[0]), "r"(a.v[1]), "r"(a.v[2]), "r"(a.v[3]), "r"(a.v[4]), "r"(a.v[5]), "r"(a.v[6]), "r"(a.v[7]),
+          "n"(fr_2p(0)), "n"(fr_2p(1)), "n"(fr_2p(2)), "n"(fr_2p(3)), "n"(fr_2p(4)), "n"(fr_2p(5)), "n"(fr_2p(6)), "n"(fr_2p(7)));
+    Fr r;
+    asm("sub.cc.u32  %0, %8,  %16;\n\t"
+        "subc.cc.u32 %1, %9,  %17;\n\t"
+        "subc.cc.u32 %2, %10, %18;\n\t"
+        "subc.cc.u32 %3, %11, %19;\n\t"
+        "subc.cc.u32 %4, %12, %20;\n\t"
+        "subc.cc.u32 %5, %13, %21;\n\t"
+        "subc.cc.u32 %6, %14, %22;\n\t"
+        "subc.u32    %7, %15, %23;"
+        : "=r"(r.v[0]), "=r"(r.v[1]), "=r"(r.v[2]), "=r"(r.v[3]), "=r"(r.v[4]), "=r"(r.v[5]), "=r"(r.v[6]), "=r"(r.v[7])
+        : "r"(t[0]), "r"(t[1]), "r"(t[2]), "r"(t[3]), "r"(t[4]), "r"(t[5]), "r"(t[6]), "r"(t[7]),
+          "r"(b.v[0]), "r"(b.v[1]), "r"(b.v[2]), "r"(b.v[3]), "r"(b.v[4]), "r"(b.v[5]), "r"(b.v[6]), "r"(b.v[7]));
+    return r;
+}
+
+// A product operand in radix-2^52 form, and x tx, y ty (< 2p) for x, y < 4p.
+// Two products to a call: they interleave, and one body of about 700
+// instructions keeps the pass inside the instruction cache.
+struct Tw {
+    double d[5];
+};
+struct FrPair {
+    Fr a, b;
+};
+static __device__ __noinline__ FrPair fr_mul2(const Fr x, const Fr y, const Tw tx, const Tw ty)
+{
+    double dx[5], dy[5];
+    uint64_t rx[5], ry[5];
+    to_d52<4>(dx, x.v);
+    to_d52<4>(dy, y.v);
+    mont52_core<FrP>(rx, dx, tx.d);
+    mont52_core<FrP>(ry, dy, ty.d);
+    FrPair r;
+    from_limbs52(r.a.v, rx);
+    from_limbs52(r.b.v, ry);
+    return r;
+}
+__device__ __forceinline__ Tw tw_of(const Fr& x)
+{
+    Tw t;
+    to_d52<0>(t.d, x.v);
+    return t;
+}
+// Twiddle e: from the radix-2^52 table (TWD), or converted
+template <bool TWD>
+__device__ __forceinline__ Tw load_tw(const Fr* __restrict__ tw, const double* __restrict__ twd, uint32_t e)
+{
+    if (TWD) {
+        const double2* q = reinterpret_cast<const double2*>(twd + (size_t)e * kTwdStride);
+        const double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
+        return Tw{{a.x, a.y, b.x, b.y, c.x}};
+    }
+    return tw_of(ldg_elem(tw + e));
+}
+
 // Factor a pass applies to each element as it loads it (the first pass) or
 // stores it (the last pass): x * scale * g^e, e = the position j, or, with
 // brev set, the coefficient index brev(j) that a bit-reversed position
-// holds; a null scale or null power tables stand for 1.
-__device__ __forceinline__ Fr edge_apply(const NttEdge& ed, const Fr& sc, Fr x, size_t j, uint32_t k)
+// holds; a null scale or null power tables stand for 1.  x < 4p, result < 2p.
+__device__ __forceinline__ void edge_apply2(const NttEdge& ed, Fr& x, Fr& y, uint32_t jx, uint32_t jy, uint32_t k)
 {
-    if (ed.scale) x = mul(x, sc);
-    if (ed.lo) x = mul(x, coset_pow(ed.lo, ed.hi, ed.brev ? brev_k(j, k) : j));
-    return x;
+    if (ed.lo) {
+        if (ed.brev) { jx = (uint32_t)brev_k(jx, k); jy = (uint32_t)brev_k(jy, k); }
+        const uint32_t m = (1u << kPowLoBits) - 1;
+        FrPair c = fr_mul2(ldg_elem(ed.lo + (jx & m)), ldg_elem(ed.lo + (jy & m)), tw_of(ldg_elem(ed.hi + (jx >> kPowLoBits))),
+                           tw_of(ldg_elem(ed.hi + (jy >> kPowLoBits))));
+        if (ed.scale) {
+            const Tw s = tw_of(ldg_elem(ed.scale));
+            c = fr_mul2(c.a, c.b, s, s);
+        }
+        c = fr_mul2(x, y, tw_of(c.a), tw_of(c.b));
+        x = c.a; y = c.b;
+    } else if (ed.scale) {
+        const Tw s = tw_of(ldg_elem(ed.scale));
+        const FrPair c = fr_mul2(x, y, s, s);
+        x = c.a; y = c.b;
+    }
 }
 
-// m radix-2 stages in shared memory over groups of 2^m elements that differ
-// in index bits [lowbits, lowbits+m); R groups with consecutive (outer, low)
-// index per block.  `batch` transforms of size 2^k lie `bstride` elements
-// apart (or at ptrs[blockIdx.y]).
+// m radix-2 stages over groups of 2^m elements that differ in index bits
+// [lowbits, lowbits+m); R groups with consecutive (outer, low) index per
+// block.  `batch` transforms of size 2^k lie `bstride` elements apart (or at
+// ptrs[blockIdx.y]).
 //   DIF (decimation in frequency): stages s0 .. s0+m-1, natural order in,
 //     bit-reversed out after all passes; c[j] = lo + hi, c[j^h] =
 //     (lo - hi) w^((j mod h) << s) (poly.cuh:38-39).
@@ -195,95 +306,235 @@ __device__ __forceinline__ Fr edge_apply(const NttEdge& ed, const Fr& sc, Fr x, 
 //     order in, natural out; with u = w^((j mod 2^t) << (k-1-t)) hi,
 //     c[j] = lo + u, c[j + 2^t] = lo - u.
 // Both compute X_k = sum_j a_j w^(jk).
-// Twiddle e as the second operand of the product: read from the radix-2^52
-// table (TWD) or converted from the 8x32-bit table.
-template <bool TWD>
-__device__ __forceinline__ Fr tw_mul(const Fr& x, const Fr* __restrict__ tw, const double* __restrict__ twd, size_t e)
-{
-    if (TWD) {
-        const double2* q = reinterpret_cast<const double2*>(twd + e * kTwdStride);
-        double2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
-        const double d[5] = {a.x, a.y, b.x, b.y, c.x};
-        return mul52_pre(x, d);
-    }
-    return mul52(x, ldg_elem(tw + e));
-}
+//
+// A thread takes four elements a quarter of a radix-4 span apart and runs two
+// stages on them in registers (one stage first when m is odd); shared memory
+// holds the block between the steps, the first step reads and the last writes
+// global memory.  Shared memory is two planes of 16-byte halves, swizzled so
+// that the strided reads of the short spans spread over the banks.
+//
+// Bound by the issue of the products (325 instructions of about 460 a
+// butterfly).  Against one stage at a time on canonical values, bit reversal
+// included: 2^12 forward 41.0 -> 32.8 us, 2^20 coset forward 323 -> 296, 2^24
+// coset inverse 6713 -> 5102.  Three blocks a multiprocessor instead of two
+// (80 registers) spilled and was 12 % slower.
+__device__ __forceinline__ uint32_t swz(uint32_t i) { return i ^ ((i >> 2) & 7u); }
 
 template <bool DIT, bool TWD>
-__global__ void __launch_bounds__(kNttThreads) k_ntt_pass(Fr* __restrict__ data, NttPass p, const Fr* __restrict__ tw,
-                                                           const double* __restrict__ twd, NttEdge pre, NttEdge post,
-                                                           size_t bstride, Fr* const* __restrict__ ptrs)
+__global__ void __launch_bounds__(kNttThreads, 2) k_ntt_pass(Fr* __restrict__ data, NttPass p, const Fr* __restrict__ tw,
+                                                             const double* __restrict__ twd, NttEdge pre, NttEdge post,
+                                                             size_t bstride, Fr* const* __restrict__ ptrs)
 {
-    extern __shared__ uint4 smem_raw[];
-    Fr* sm = reinterpret_cast<Fr*>(smem_raw);
+    extern __shared__ uint4 sm[];
     Fr* d = ptrs ? ptrs[blockIdx.y] : data + (size_t)blockIdx.y * bstride;
-    const uint32_t G = 1u << p.m, R = p.R;
-    const uint32_t rbits = __ffs(R) - 1;
-    const size_t lowmask = (size_t(1) << p.lowbits) - 1;
-    const uint32_t tot = G * R;
-    const bool use_pre = pre.scale || pre.lo, use_post = post.scale || post.lo;
-    const Fr psc = pre.scale ? ldg_elem(pre.scale) : Fr::one();
-    const Fr qsc = post.scale ? ldg_elem(post.scale) : Fr::one();
-    for (uint32_t i = threadIdx.x; i < tot; i += blockDim.x) {
-        uint32_t g = i >> rbits, r = i & (R - 1);
-        size_t cidx = (size_t)blockIdx.x * R + r;
-        size_t j = ((cidx >> p.lowbits) << (p.lowbits + p.m)) | ((size_t)g << p.lowbits) | (cidx & lowmask);
-        Fr x = ldg_elem(d + j);
-        if (use_pre) x = edge_apply(pre, psc, x, j, p.k);
-        st_elem(sm + i, x);
-    }
-    __syncthreads();
-    for (uint32_t t = 0; t < p.m; t++) {
-        // DIF: group-index bit hb = m-1-t; DIT: bit hb = t
-        uint32_t hb = DIT ? t : p.m - 1 - t;
-        for (uint32_t b = threadIdx.x; b < tot / 2; b += blockDim.x) {
-            uint32_t r = b & (R - 1), gb = b >> rbits;
-            uint32_t g = ((gb >> hb) << (hb + 1)) | (gb & ((1u << hb) - 1));
-            uint32_t i0 = (g << rbits) | r, i1 = ((g + (1u << hb)) << rbits) | r;
-            size_t low = ((size_t)blockIdx.x * R + r) & lowmask;
-            size_t jm = (((size_t)(g & ((1u << hb) - 1))) << p.lowbits) | low;
-            Fr lo = ld_elem(sm + i0), hi = ld_elem(sm + i1);
-            if (DIT) {
-                Fr u = tw_mul<TWD>(hi, tw, twd, jm << (p.k - 1 - (p.lowbits + t)));
-                st_elem(sm + i0, add(lo, u));
-                st_elem(sm + i1, sub(lo, u));
+    const uint32_t rbits = __ffs(p.R) - 1, tot = p.R << p.m, units = tot >> 2;
+    const uint32_t lowmask = (1u << p.lowbits) - 1;
+    auto sm_ld = [&](uint32_t i) -> Fr {
+        Fr x;
+        uint4* q = reinterpret_cast<uint4*>(&x);
+        q[0] = sm[swz(i)];
+        q[1] = sm[tot + swz(i)];
+        return x;
+    };
+    auto sm_st = [&](uint32_t i, const Fr& x) {
+        const uint4* q = reinterpret_cast<const uint4*>(&x);
+        sm[swz(i)] = q[0];
+        sm[tot + swz(i)] = q[1];
+    };
+    // steps of two stages: quarter spans 2^h; an odd count starts with one stage
+    const uint32_t steps = (p.m + 1) >> 1;
+    for (uint32_t st = 0; st < steps; st++) {
+        const bool first = st == 0, last = st + 1 == steps, odd = (p.m & 1) != 0, one = first && odd;
+        // stages done before this step: 2 st, or 2 st - 1 after an odd start
+        const uint32_t done = 2 * st - (odd && st ? 1u : 0u);
+        const uint32_t h = DIT ? done : one ? p.m - 2 : p.m - 2 - done;
+        for (uint32_t u = threadIdx.x; u < units; u += blockDim.x) {
+            const uint32_t r = u & (p.R - 1), gq = u >> rbits, gl = gq & ((1u << h) - 1);
+            const uint32_t g0 = ((gq >> h) << (h + 2)) | gl;
+            const uint32_t cidx = blockIdx.x * p.R + r, low = cidx & lowmask;
+            const uint32_t j0 = ((cidx >> p.lowbits) << (p.lowbits + p.m)) | (g0 << p.lowbits) | low, js = 1u << (h + p.lowbits);
+            const uint32_t i0 = (g0 << rbits) | r, is = 1u << (h + rbits);
+            const uint32_t jm = (gl << p.lowbits) | low;
+            // twiddle exponent shift of the stage whose two pairs share one
+            // twiddle (1 in the transform's first DIT or last DIF stage);
+            // loading a step's twiddles ahead of its elements spilled: 13 %
+            // slower
+            const uint32_t e = DIT ? p.k - 1 - (p.lowbits + h) : p.s0 + p.m - 1 - h;
+            const bool unit = p.lowbits + h == 0;
+            Fr x0, x1, x2, x3;
+            if (first) {
+                x0 = ld_elem(d + j0);
+                x1 = ld_elem(d + j0 + js);
+                x2 = ld_elem(d + j0 + 2 * js);
+                x3 = ld_elem(d + j0 + 3 * js);
+                if (pre.lo || pre.scale) {
+                    edge_apply2(pre, x0, x1, j0, j0 + js, p.k);
+                    edge_apply2(pre, x2, x3, j0 + 2 * js, j0 + 3 * js, p.k);
+                }
             } else {
-                st_elem(sm + i0, add(lo, hi));
-                // lo + p - hi, unreduced: the product takes it below 2p
-                st_elem(sm + i1, tw_mul<TWD>(sub_plus_p(lo, hi), tw, twd, jm << (p.s0 + t)));
+                x0 = sm_ld(i0);
+                x1 = sm_ld(i0 + is);
+                x2 = sm_ld(i0 + 2 * is);
+                x3 = sm_ld(i0 + 3 * is);
+            }
+            if (DIT) {
+                // stage h on (x0, x1), (x2, x3)
+                if (unit) {
+                    x1 = red_2p(x1);
+                    x3 = red_2p(x3);
+                } else {
+                    const Tw t = load_tw<TWD>(tw, twd, jm << e);
+                    const FrPair v = fr_mul2(x1, x3, t, t);
+                    x1 = v.a; x3 = v.b;
+                }
+                x0 = red_2p(x0);
+                x2 = red_2p(x2);
+                Fr t0 = add_raw(x0, x1), t2 = add_raw(x2, x3);
+                x1 = sub_2p(x0, x1);
+                x3 = sub_2p(x2, x3);
+                x0 = t0;
+                x2 = t2;
+                if (!one) {
+                    // stage h + 1 on (x0, x2), (x1, x3)
+                    const FrPair v = fr_mul2(x2, x3, load_tw<TWD>(tw, twd, jm << (e - 1)),
+                                             load_tw<TWD>(tw, twd, (jm + js) << (e - 1)));
+                    x0 = red_2p(x0);
+                    x1 = red_2p(x1);
+                    x2 = sub_2p(x0, v.a);
+                    x3 = sub_2p(x1, v.b);
+                    x0 = add_raw(x0, v.a);
+                    x1 = add_raw(x1, v.b);
+                }
+            } else {
+                // stage h + 1 on (x0, x2), (x1, x3)
+                Fr t0 = red_2p(add_raw(x0, x2)), t1 = red_2p(add_raw(x1, x3));
+                const FrPair v = fr_mul2(sub_2p(x0, x2), sub_2p(x1, x3), load_tw<TWD>(tw, twd, jm << (e - 1)),
+                                         load_tw<TWD>(tw, twd, (jm + js) << (e - 1)));
+                x0 = t0; x1 = t1; x2 = v.a; x3 = v.b;
+                if (!one) {
+                    // stage h on (x0, x1), (x2, x3)
+                    t0 = red_2p(add_raw(x0, x1));
+                    t1 = red_2p(add_raw(x2, x3));
+                    x1 = sub_2p(x0, x1);
+                    x3 = sub_2p(x2, x3);
+                    if (unit) {
+                        x1 = red_2p(x1);
+                        x3 = red_2p(x3);
+                    } else {
+                        const Tw t = load_tw<TWD>(tw, twd, jm << e);
+                        const FrPair z = fr_mul2(x1, x3, t, t);
+                        x1 = z.a; x3 = z.b;
+                    }
+                    x0 = t0;
+                    x2 = t1;
+                }
+            }
+            if (last) {
+                if (post.lo || post.scale) {
+                    edge_apply2(post, x0, x1, j0, j0 + js, p.k);
+                    edge_apply2(post, x2, x3, j0 + 2 * js, j0 + 3 * js, p.k);
+                } else if (DIT && p.canon) {
+                    x0 = red_2p(x0); x1 = red_2p(x1); x2 = red_2p(x2); x3 = red_2p(x3);
+                }
+                if (p.canon) {
+                    x0 = final_sub<FrP>(x0.v); x1 = final_sub<FrP>(x1.v);
+                    x2 = final_sub<FrP>(x2.v); x3 = final_sub<FrP>(x3.v);
+                }
+                auto at = [&](uint32_t j) { return p.natural ? (uint32_t)brev_k(j, p.k) : j; };
+                st_elem(d + at(j0), x0);
+                st_elem(d + at(j0 + js), x1);
+                st_elem(d + at(j0 + 2 * js), x2);
+                st_elem(d + at(j0 + 3 * js), x3);
+            } else {
+                sm_st(i0, x0);
+                sm_st(i0 + is, x1);
+                sm_st(i0 + 2 * is, x2);
+                sm_st(i0 + 3 * is, x3);
             }
         }
-        __syncthreads();
-    }
-    for (uint32_t i = threadIdx.x; i < tot; i += blockDim.x) {
-        uint32_t g = i >> rbits, r = i & (R - 1);
-        size_t cidx = (size_t)blockIdx.x * R + r;
-        size_t j = ((cidx >> p.lowbits) << (p.lowbits + p.m)) | ((size_t)g << p.lowbits) | (cidx & lowmask);
-        Fr x = ld_elem(sm + i);
-        if (use_post) x = edge_apply(post, qsc, x, j, p.k);
-        st_elem(d + j, x);
+        if (!last) __syncthreads();
     }
 }
 
-// In-place bit reversal; each output position pos is then multiplied by
-// scale (when non-null) and g^-pos (when clo != null).
-__global__ void k_ntt_bitrev(Fr* __restrict__ data, uint32_t k, const Fr* __restrict__ scale,
-                             const Fr* __restrict__ clo, const Fr* __restrict__ chi, size_t bstride,
-                             Fr* const* __restrict__ ptrs)
+// The transform of two elements (k = 1), both factors and directions alike:
+// x0 + x1, x0 - x1 with the edges of the one pass.
+__global__ void k_ntt_two(Fr* __restrict__ data, NttEdge pre, NttEdge post, size_t bstride, Fr* const* __restrict__ ptrs)
+{
+    if (threadIdx.x) return;
+    Fr* d = ptrs ? ptrs[blockIdx.x] : data + (size_t)blockIdx.x * bstride;
+    Fr x = ld_elem(d), y = ld_elem(d + 1);
+    edge_apply2(pre, x, y, 0, 1, 1);
+    x = final_sub<FrP>(x.v);
+    y = final_sub<FrP>(y.v);
+    Fr a = add(x, y), b = sub(x, y);
+    edge_apply2(post, a, b, 0, 1, 1);
+    st_elem(d, final_sub<FrP>(a.v));
+    st_elem(d + 1, final_sub<FrP>(b.v));
+}
+
+// In-place bit reversal, element by element (short transforms).
+__global__ void k_ntt_bitrev(Fr* __restrict__ data, uint32_t k, size_t bstride, Fr* const* __restrict__ ptrs)
 {
     Fr* d = ptrs ? ptrs[blockIdx.y] : data + (size_t)blockIdx.y * bstride;
-    size_t n = size_t(1) << k;
-    Fr sc = scale ? ldg_elem(scale) : Fr::one();
+    const size_t n = size_t(1) << k;
     for (uint64_t j = gtid(); j < n; j += gstride()) {
-        size_t r = brev_k(j, k);
-        if (j > r) continue;
-        Fr a = ld_elem(d + j), b = ld_elem(d + r);
-        // after the swap position j holds b and position r holds a
-        if (scale) { a = mul(a, sc); if (j != r) b = mul(b, sc); }
-        if (clo) { a = mul(a, coset_pow(clo, chi, r)); if (j != r) b = mul(b, coset_pow(clo, chi, j)); }
+        const size_t r = brev_k(j, k);
+        if (j >= r) continue;
+        const Fr a = ld_elem(d + j), b = ld_elem(d + r);
         st_elem(d + r, a);
-        if (j != r) st_elem(d + j, b);
+        st_elem(d + j, b);
     }
+}
+
+// In-place bit reversal by tiles.  With the index split into (H, M, L), H and
+// L of 5 bits, (H, M, L) goes to (brev L, brev M, brev H): the 32 x 32 tile of
+// M, rows of 1 KB, is the tile of brev M transposed with its rows and columns
+// bit-reversed.  A block exchanges tiles M and brev M through shared memory,
+// so every access to global memory is a full row; element by element the
+// writes touch one 32-byte sector at a time.  (In a 2^24 coset inverse the
+// element-wise form took 2080 us, factors included; those are now applied by
+// the last pass.)  A row enters shared memory at its bit-reversed number, so that a column is
+// read at the odd stride of 33 units.
+constexpr uint32_t kTileRow = 33, kTile = 32 * kTileRow;
+__global__ void __launch_bounds__(256) k_ntt_bitrev_tiles(Fr* __restrict__ data, uint32_t k, size_t bstride,
+                                                          Fr* const* __restrict__ ptrs)
+{
+    extern __shared__ uint4 sm[];   // two tiles, two planes each
+    const uint32_t mb = k - 10, M = blockIdx.x, N = mb ? __brev(M) >> (32 - mb) : 0;
+    if (M > N) return;
+    Fr* d = ptrs ? ptrs[blockIdx.y] : data + (size_t)blockIdx.y * bstride;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, tiles = M == N ? 1 : 2;
+    for (uint32_t t = 0; t < tiles; t++) {
+        const Fr* src = d + ((size_t)(t ? N : M) << 5) + lane;
+        uint4* q = sm + t * 2 * kTile + lane;
+        for (uint32_t row = w; row < 32; row += 8) {
+            const Fr x = ld_elem(src + ((size_t)row << (k - 5)));
+            const uint32_t at = (__brev(row) >> 27) * kTileRow;
+            q[at] = reinterpret_cast<const uint4*>(&x)[0];
+            q[kTile + at] = reinterpret_cast<const uint4*>(&x)[1];
+        }
+    }
+    __syncthreads();
+    for (uint32_t t = 0; t < tiles; t++) {
+        // tile t of the source fills the other tile
+        Fr* dst = d + ((size_t)(t ? M : N) << 5) + lane;
+        const uint4* q = sm + t * 2 * kTile + lane * kTileRow;
+        for (uint32_t row = w; row < 32; row += 8) {
+            Fr x;
+            const uint32_t at = __brev(row) >> 27;
+            reinterpret_cast<uint4*>(&x)[0] = q[at];
+            reinterpret_cast<uint4*>(&x)[1] = q[kTile + at];
+            st_elem(dst + ((size_t)row << (k - 5)), x);
+        }
+    }
+}
+
+// the one element of a transform of size 1 times its scale
+__global__ void k_ntt_one(Fr* __restrict__ data, const Fr* __restrict__ scale, size_t bstride, Fr* const* __restrict__ ptrs)
+{
+    if (threadIdx.x) return;
+    Fr* d = ptrs ? ptrs[blockIdx.x] : data + (size_t)blockIdx.x * bstride;
+    st_elem(d, mul(ld_elem(d), ldg_elem(scale)));
 }
 
 int ntt_prepare_launch()
@@ -299,16 +550,26 @@ int ntt_prepare_launch()
         LZK_CUDA(cudaFuncSetAttribute(k_ntt_pass<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxNttBlock * sizeof(Fr)));
         LZK_CUDA(cudaFuncSetAttribute(k_ntt_pass<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxNttBlock * sizeof(Fr)));
         LZK_CUDA(cudaFuncSetAttribute(k_ntt_pass<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxNttBlock * sizeof(Fr)));
+        LZK_CUDA(cudaFuncSetAttribute(k_ntt_bitrev_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * kTile * sizeof(uint4)));
         attr_set[dev] = true;
     }
     return LZK_OK;
 }
 
+// Whether a transform of size 2^k is one pass of several steps, whose only
+// block has read every element when it writes the first one: such a DIF
+// transform writes its results in natural order itself.
+static bool ntt_one_pass(uint32_t k) { return k > 2 && (1u << k) <= tune_ntt_block(k); }
+
 int ntt_passes(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* tw, bool dit, NttEdge pre,
-               NttEdge post, cudaStream_t st, Fr* const* ptrs, const double* twd)
+               NttEdge post, cudaStream_t st, Fr* const* ptrs, const double* twd, bool natural)
 {
     if (k == 0 || k > 30 || count == 0 || count > 65535 || (!data && !ptrs) || !tw) return LZK_EINVAL;
     LZK_TRY(ntt_prepare_launch());
+    if (k == 1) {
+        k_ntt_two<<<count, 32, 0, st>>>(data, pre, post, bstride, ptrs); note_launch();
+        return launch_status();
+    }
     // block size from the tuning table: 2^maxm elements, at most maxm stages a pass
     const uint32_t elems = tune_ntt_block(k);
     uint32_t maxm = 0;
@@ -328,18 +589,21 @@ int ntt_passes(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* t
         if ((size_t)R > (n >> m)) R = (uint32_t)(n >> m);
         if (R == 0) R = 1;
         pp.R = R;
+        pp.canon = q == P - 1;
+        pp.natural = natural && ntt_one_pass(k);
+        const unsigned threads = G * R / 4 < kNttThreads ? G * R / 4 : kNttThreads;
         size_t blocks = (n >> m) / R;
         size_t smem = (size_t)G * R * sizeof(Fr);
         NttEdge a = q == 0 ? pre : NttEdge{}, b = q == P - 1 ? post : NttEdge{};
         const dim3 grid((unsigned)blocks, count);
         if (dit && twd)
-            k_ntt_pass<true, true><<<grid, kNttThreads, smem, st>>>(data, pp, tw, twd, a, b, bstride, ptrs);
+            k_ntt_pass<true, true><<<grid, threads, smem, st>>>(data, pp, tw, twd, a, b, bstride, ptrs);
         else if (dit)
-            k_ntt_pass<true, false><<<grid, kNttThreads, smem, st>>>(data, pp, tw, twd, a, b, bstride, ptrs);
+            k_ntt_pass<true, false><<<grid, threads, smem, st>>>(data, pp, tw, twd, a, b, bstride, ptrs);
         else if (twd)
-            k_ntt_pass<false, true><<<grid, kNttThreads, smem, st>>>(data, pp, tw, twd, a, b, bstride, ptrs);
+            k_ntt_pass<false, true><<<grid, threads, smem, st>>>(data, pp, tw, twd, a, b, bstride, ptrs);
         else
-            k_ntt_pass<false, false><<<grid, kNttThreads, smem, st>>>(data, pp, tw, twd, a, b, bstride, ptrs);
+            k_ntt_pass<false, false><<<grid, threads, smem, st>>>(data, pp, tw, twd, a, b, bstride, ptrs);
         note_launch();
         done += m;
     }
@@ -347,21 +611,25 @@ int ntt_passes(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* t
 }
 
 // Enqueue `count` transforms of size 2^k (natural order in, natural order
-// out) with twiddle table tw (w^e, e < n/2): DIF passes, then the bit
-// reversal with the output factors.
-static int ntt_enqueue(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* tw, const Fr* scale,
-                       const Fr* pre_lo, const Fr* pre_hi, const Fr* post_lo, const Fr* post_hi, cudaStream_t st,
-                       Fr* const* ptrs = nullptr, const double* twd = nullptr)
+// out) with twiddle table tw (w^e, e < n/2): DIF passes with the input and
+// output factors, then the bit reversal.
+static int ntt_enqueue(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* tw, NttEdge pre, NttEdge post,
+                       cudaStream_t st, Fr* const* ptrs = nullptr, const double* twd = nullptr)
 {
     LZK_TRY(ntt_prepare_launch());
-    if (k > 0) {
-        NttEdge pre{pre_lo, pre_hi, nullptr, 0};
-        LZK_TRY(ntt_passes(data, k, count, bstride, tw, false, pre, NttEdge{}, st, ptrs, twd));
-    } else if (!(scale || post_lo || pre_lo)) {
-        return LZK_OK;
+    if (k == 0) {
+        // g^0 = 1: only a scale is left
+        if (!post.scale) return LZK_OK;
+        k_ntt_one<<<count, 32, 0, st>>>(data, post.scale, bstride, ptrs); note_launch();
+        return launch_status();
     }
-    size_t n = size_t(1) << k;
-    k_ntt_bitrev<<<dim3(grid_for(n, 256, sm_count() * 8), count), 256, 0, st>>>(data, k, scale, post_lo, post_hi, bstride, ptrs); note_launch();
+    LZK_TRY(ntt_passes(data, k, count, bstride, tw, false, pre, post, st, ptrs, twd, true));
+    if (k < 2 || ntt_one_pass(k)) return launch_status();
+    if (k < 10) {
+        k_ntt_bitrev<<<dim3(grid_for(size_t(1) << k, 256), count), 256, 0, st>>>(data, k, bstride, ptrs); note_launch();
+    } else {
+        k_ntt_bitrev_tiles<<<dim3(1u << (k - 10), count), 256, 4 * kTile * sizeof(uint4), st>>>(data, k, bstride, ptrs); note_launch();
+    }
     return launch_status();
 }
 
@@ -373,11 +641,15 @@ int ntt_run(Fr* data, uint32_t k, int dir, uint32_t count, size_t bstride, const
     NttTables t; CosetTables c;
     LZK_TRY(get_tables(k, t, c));
     bool inv = dir & 1, coset = dir >= 2;
-    const Fr* scale = scale_override ? scale_override : (inv ? t.consts + 2 : nullptr);
-    return ntt_enqueue(data, k, count, bstride, t.tw[inv ? 1 : 0], scale,
-                       (coset && !inv) ? c.lo[0] : nullptr, (coset && !inv) ? c.hi[0] : nullptr,
-                       (coset && inv) ? c.lo[1] : nullptr, (coset && inv) ? c.hi[1] : nullptr, st, ptrs,
-                       twd_for(t, inv ? 1 : 0, k));
+    NttEdge pre, post;
+    if (coset && !inv) pre = NttEdge{c.lo[0], c.hi[0], nullptr, 0};
+    if (coset && inv) {
+        // h_j = (...) n^-1 g^-j of the coefficient j that position brev(j) holds
+        post = scale_override ? NttEdge{c.lo[1], c.hi[1], scale_override, 1} : NttEdge{t.slo[1], c.hi[1], nullptr, 1};
+    } else {
+        post.scale = scale_override ? scale_override : inv ? t.consts + 2 : nullptr;
+    }
+    return ntt_enqueue(data, k, count, bstride, t.tw[inv ? 1 : 0], pre, post, st, ptrs, twd_for(t, inv ? 1 : 0, k));
 }
 
 }  // namespace lzk
@@ -408,8 +680,8 @@ int lzk_number_theory_transformation(size_t deg, size_t log_deg, lzk_fr_t* coeff
 {
     if (!coeffs || !omega_powers || log_deg > 30 || deg != (size_t(1) << log_deg)) return LZK_EINVAL;
     return ntt_enqueue(reinterpret_cast<Fr*>(coeffs), (uint32_t)log_deg, 1, 0,
-                       reinterpret_cast<const Fr*>(omega_powers), reinterpret_cast<const Fr*>(factor),
-                       nullptr, nullptr, nullptr, nullptr, as_stream(stream));
+                       reinterpret_cast<const Fr*>(omega_powers), NttEdge{},
+                       NttEdge{nullptr, nullptr, reinterpret_cast<const Fr*>(factor), 0}, as_stream(stream));
 }
 
 }  // extern "C"

@@ -11,6 +11,7 @@ struct NttTables {
     // operand form, field52.cuh), kTwdStride doubles per twiddle
     double* twd[2] = {nullptr, nullptr};
     Fr* consts = nullptr;            // see k_ntt_consts
+    Fr* slo[2] = {nullptr, nullptr}; // 2^-k g^j, 2^-k g^-j for j < 4096 (CosetTables::lo with the inverse's scale)
 };
 constexpr uint32_t kTwdStride = 6;   // 5 limbs and a pad: 48-byte records, three 16-byte loads
 // Transforms up to 2^kTwdMaxLog read the radix-2^52 table (its 2^(k-1)
@@ -52,8 +53,9 @@ int ntt_run(Fr* data, uint32_t k, int dir, uint32_t count, size_t bstride, const
 // bit-reversed order, DIT bit-reversed order to natural order.  pre applies
 // to the first pass's loads, post to the last pass's stores.  twd, when
 // given, is the same table in radix-2^52 form (NttTables::twd), which the
-// butterflies then read instead of converting tw.
+// butterflies then read instead of converting tw.  natural: a DIF transform
+// that is one pass writes natural order itself (ntt_run).
 int ntt_passes(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* tw, bool dit, NttEdge pre,
-               NttEdge post, cudaStream_t st, Fr* const* ptrs = nullptr, const double* twd = nullptr);
+               NttEdge post, cudaStream_t st, Fr* const* ptrs = nullptr, const double* twd = nullptr, bool natural = false);
 
 }  // namespace lzk

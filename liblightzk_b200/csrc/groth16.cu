@@ -54,48 +54,88 @@ __device__ __forceinline__ Fr canon(const Scal& s)
     return from_mont(m);
 }
 
-// fixed-base products from comb tables: thread 0 r d1, 1 s a1, 2 r b1,
-// 3 (r s) d1, 4 s d2
+// Fixed-base products from comb tables, a warp each (<<<1, 160>>>): 0 r d1, 1
+// s a1, 2 r b1, 3 (r s) d1, 4 s d2.  Lane j takes the entry of byte j of the
+// scalar and the 32 entries are added in a tree: 5 dependent additions where
+// one thread's 32 took 490 us.
+template <class F>
+__device__ __forceinline__ XYZZ<F> comb_mul_warp(const Aff<F>* __restrict__ T, const Fr& k)
+{
+    const uint32_t j = threadIdx.x & 31;
+    uint32_t word = 0;
+    _Pragma("unroll") for (int i = 0; i < 8; i++) word = (j >> 2) == (uint32_t)i ? k.v[i] : word;
+    const uint32_t d = (word >> (8 * (j & 3))) & 255u;
+    XYZZ<F> x = d ? xyzz_from_aff(ldg_elem(T + j * 256 + d)) : xyzz_inf<F>();
+    for (uint32_t o = 16; o > 0; o >>= 1) x = xyzz_add_cold(x, shfl_xor_pt(x, o));
+    return x;
+}
 __global__ void k_fixed_products(const Aff<Fq>* __restrict__ comb1, const Aff<Fq2>* __restrict__ comb2, Scal r, Scal s,
                                  XYZZ<Fq>* __restrict__ sm1, XYZZ<Fq2>* __restrict__ sm2)
 {
-    uint32_t t = threadIdx.x;
-    if (t > 4) return;
+    const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Fr rm, sm;
     _Pragma("unroll") for (int i = 0; i < 8; i++) { rm.v[i] = r.v[i]; sm.v[i] = s.v[i]; }
-    if (t == 4) { sm2[0] = comb_mul(comb2, from_mont(sm)); return; }
-    const int table[4] = {2, 0, 1, 2};   // d1, a1, b1, d1
-    Fr k = t == 0 ? rm : t == 1 ? sm : t == 2 ? rm : mul(rm, sm);
-    sm1[t] = comb_mul(comb1 + table[t] * 8192, from_mont(k));
+    if (w == 4) {
+        const XYZZ<Fq2> x = comb_mul_warp(comb2, from_mont(sm));
+        if (lane == 0) st_elem(sm2, x);
+    } else if (w < 4) {
+        const int table = w == 1 ? 0 : w == 2 ? 1 : 2;   // d1, a1, b1, d1
+        const Fr k = w == 0 ? rm : w == 1 ? sm : w == 2 ? rm : mul(rm, sm);
+        const XYZZ<Fq> x = comb_mul_warp(comb1 + table * 8192, from_mont(k));
+        if (lane == 0) st_elem(sm1 + w, x);
+    }
 }
 
-// k * P, 4-bit fixed window: 15 precomputed multiples, then per nibble four
-// doublings and one addition (curve_utils.cuh:28-49 computes the same
-// product bit by bit).  Run by a whole warp with warp-uniform point
-// operations: every lane holds P, k and the table, and gets the product.
-template <class F>
-__device__ XYZZ<F> smul_w4_warp(const XYZZ<F>& P, const Fr& k)
+// m P for a magnitude m < 2^126 by signed 4-bit windows: 8 precomputed
+// multiples, then per window four doublings and one addition.  Run by a whole
+// warp with warp-uniform point operations: every lane holds P and m, and gets
+// the product.
+static __device__ XYZZ<Fq> smul_half_warp(const XYZZ<Fq>& P, const uint32_t m[4])
 {
-    XYZZ<F> tab[16];
-    tab[0] = xyzz_inf<F>();
+    XYZZ<Fq> tab[9];
+    tab[0] = xyzz_inf<Fq>();
     tab[1] = P;
-    for (int i = 2; i < 16; i++) tab[i] = (i & 1) ? xyzz_add_warp(tab[i - 1], P) : xyzz_dbl_warp(tab[i >> 1]);
-    XYZZ<F> acc = xyzz_inf<F>();
-    for (int w = 63; w >= 0; w--) {
+    for (int i = 2; i < 9; i++) tab[i] = (i & 1) ? xyzz_add_warp(tab[i - 1], P) : xyzz_dbl_warp(tab[i >> 1]);
+    int8_t dig[32];
+    uint32_t carry = 0;
+    for (int w = 0; w < 32; w++) {
+        const uint32_t raw = ((m[w >> 3] >> (4 * (w & 7))) & 15u) + carry;
+        carry = raw > 8 ? 1u : 0u;
+        dig[w] = (int8_t)(carry ? (int)raw - 16 : (int)raw);
+    }
+    XYZZ<Fq> acc = xyzz_inf<Fq>();
+    for (int w = 31; w >= 0; w--) {
         for (int d = 0; d < 4; d++) acc = xyzz_dbl_warp(acc);
-        uint32_t nib = (k.v[w >> 3] >> (4 * (w & 7))) & 15u;
-        if (nib) acc = xyzz_add_warp(acc, tab[nib]);
+        const int g = dig[w];
+        if (g) acc = xyzz_add_warp(acc, g > 0 ? tab[g] : xyzz_neg(tab[-g]));
     }
     return acc;
 }
 
-// variable-base products: warp 0 s * A, warp 1 r * B1 (<<<1, 64>>>)
+// variable-base products s * A and r * B1 (<<<1, 128>>>): two warps each, one
+// for each half of the scalar over the endomorphism (glv.cuh), which halves
+// the chain of dependent doublings
 __global__ void k_dep_products(const Jac<Fq>* __restrict__ g1res, Scal r, Scal s, XYZZ<Fq>* __restrict__ sm1)
 {
-    const uint32_t w = threadIdx.x >> 5;
-    if (w > 1) return;
-    XYZZ<Fq> x = smul_w4_warp(jac_to_xyzz(g1res[w]), canon(w == 0 ? s : r));
-    if ((threadIdx.x & 31) == 0) sm1[4 + w] = x;
+    __shared__ XYZZ<Fq> half[2];
+    const uint32_t w = threadIdx.x >> 5, q = w >> 1, h = w & 1;
+    if (w < 4) {
+        const Fr k = canon(q == 0 ? s : r);
+        uint32_t k1[4], k2[4];
+        bool n1, n2;
+        glv_split(k.v, k1, n1, k2, n2);
+        XYZZ<Fq> P = jac_to_xyzz(g1res[q]);
+        if (h) P.X = cmul(P.X, glv_beta());
+        if (h ? n2 : n1) P = xyzz_neg(P);
+        _Pragma("unroll") for (int i = 0; i < 4; i++) k1[i] = h ? k2[i] : k1[i];
+        XYZZ<Fq> x = smul_half_warp(P, k1);
+        if (h && (threadIdx.x & 31) == 0) half[q] = x;
+        __syncthreads();
+        if (!h) {
+            x = xyzz_add_warp(x, half[q]);
+            if ((threadIdx.x & 31) == 0) sm1[4 + q] = x;
+        }
+    }
 }
 
 // proof.A = a1 + A + r d1; proof.B = b2 + B2 + s d2;
@@ -415,7 +455,7 @@ int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, 
 
     // s3: fixed-base products
     void* tr_fx = trace_begin("groth16_fixed_products", x->s3);
-    k_fixed_products<<<1, 32, 0, x->s3>>>(p->comb1, p->comb2, rs, ss, x->sm1, x->sm2); note_launch();
+    k_fixed_products<<<1, 160, 0, x->s3>>>(p->comb1, p->comb2, rs, ss, x->sm1, x->sm2); note_launch();
     trace_end(tr_fx, x->s3);
 
     // s1: one digit sort of z for the A, B1 and B2 MSMs (same scalars, same
@@ -443,7 +483,7 @@ int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, 
     LZK_CUDA(cudaEventRecord(x->ev_b1, x->s1));
     LZK_CUDA(cudaStreamWaitEvent(x->s3, x->ev_b1, 0));
     void* tr_dep = trace_begin("groth16_dep_products", x->s3);
-    k_dep_products<<<1, 64, 0, x->s3>>>(x->g1res, rs, ss, x->sm1); note_launch();
+    k_dep_products<<<1, 128, 0, x->s3>>>(x->g1res, rs, ss, x->sm1); note_launch();
     trace_end(tr_dep, x->s3);
     LZK_CUDA(cudaEventRecord(x->ev_s3, x->s3));
     LZK_CUDA(cudaEventRecord(x->ev_s1, x->s1));

@@ -3,6 +3,7 @@
 #pragma once
 #include "common.cuh"
 #include "curve.cuh"
+#include "glv.cuh"
 #include "tune.cuh"
 
 namespace lzk {
@@ -55,11 +56,12 @@ struct MsmPlan {
     uint32_t chunk = 0;    // sorted entries per accumulation thread
     uint32_t run = 0;      // buckets per lane run of the reduction tiles
     size_t chunks = 0;
+    bool glv = false;         // plain G1: every scalar in two halves, over 2 n bases (glv.cuh)
     uint32_t rounds = 0;      // batched affine rounds before the accumulation
     size_t max_slots = 0;     // entries with the gaps that pad buckets to 2^rounds
     size_t slice = 0;         // slots a slice
     // workspace offsets
-    size_t o_cnt, o_off, o_ent, o_bsum, o_head, o_tail, o_lr0, o_la0, o_lr1, o_la1, o_scan, o_large, o_aff, o_fin,
+    size_t o_cnt, o_off, o_ent, o_bsum, o_head, o_tail, o_lr0, o_la0, o_lr1, o_la1, o_scan, o_large, o_aff, o_fin, o_phi,
         bytes;
 };
 
@@ -110,6 +112,8 @@ inline uint32_t acc_chunk(uint32_t chunk, uint32_t rounds)
 }
 
 inline uint32_t windows_for(uint32_t c) { return (255 + c - 1) / c; }
+// windows of a half scalar: its top digit, with the carry, stays <= 2^(c-1)
+inline uint32_t windows_glv(uint32_t c) { return (kGlvBits + 1 + c - 1) / c; }
 
 // accumulation chunk and reduction run of an MSM of n points in group g:
 // cfg's values, else the tuning table's (plain bases, or tables with
@@ -126,15 +130,16 @@ inline uint32_t msm_run(const lzk_msm_cfg* cfg, int group, size_t n)
 
 template <class Gp>
 inline void plan_msm(MsmPlan& p, size_t n, uint32_t c, bool shared, size_t stride, uint32_t chunk = kDefaultChunk,
-                     uint32_t run = kDefaultRun, uint32_t rounds = 0, bool presorted = false)
+                     uint32_t run = kDefaultRun, uint32_t rounds = 0, bool presorted = false, bool glv = false)
 {
     using X = XYZZ<typename Gp::F>;
     using A = Aff<typename Gp::F>;
-    p.n = n; p.c = c; p.W = windows_for(c); p.nb = 1u << (c - 1);
+    p.n = n; p.c = c; p.W = glv ? windows_glv(c) : windows_for(c); p.nb = 1u << (c - 1);
+    p.glv = glv;
     p.shared = shared; p.stride = stride;
     p.wb = shared ? 1 : p.W;
     p.B = p.wb * p.nb;
-    p.max_entries = n * (size_t)p.W;
+    p.max_entries = n * (size_t)p.W * (glv ? 2 : 1);
     p.run = run;
     p.rounds = rounds;
     p.max_slots = p.max_entries + (size_t)p.B * ((1u << rounds) - 1);
@@ -157,6 +162,7 @@ inline void plan_msm(MsmPlan& p, size_t n, uint32_t c, bool shared, size_t strid
     p.o_la1 = cv.take<X>(lvl);
     p.o_scan = cv.take<uint32_t>((p.B + 4095) / 4096 + 1);
     p.o_large = cv.take<uint32_t>(p.chunks / kFixSmall + 2);   // count, then bucket ids
+    p.o_phi = cv.take<A>(glv ? 2 * n : 0);
     p.o_fin = cv.take<A>(rounds ? p.max_slots >> rounds : 0);
     p.o_aff = cv.take<char>(AffineScratch<typename Gp::F>(p.slice, rounds).bytes());
     p.bytes = cv.off;
@@ -168,8 +174,13 @@ inline void plan_msm(MsmPlan& p, size_t n, uint32_t c, bool shared, size_t strid
 int msm_sort(const MsmPlan& p, const Fr* scalars, uint32_t* cnt, uint32_t* off, uint32_t* ent, uint32_t* bsums,
              cudaStream_t st, const Fr* hi = nullptr, size_t split = 0);
 uint32_t msm_autotune(int group, size_t n, bool shared);
-// the least workspace a plain G1 MSM runs in (without the affine rounds)
-size_t msm_lean_bytes(size_t n, const lzk_msm_cfg* cfg);
+// Forms of an MSM: with the affine rounds and the endomorphism where they
+// apply, without the rounds, without either (the least scratch).
+enum MsmForm { kMsmFull, kMsmNoRounds, kMsmLean };
+// A plain G1 MSM in one of the forms without rounds, and the workspace of one.
+size_t msm_form_bytes(size_t n, const lzk_msm_cfg* cfg, MsmForm form);
+int msm_g1_form(const Fr* scalars, const void* bases, size_t n, Jac<Fq>* out, const lzk_msm_cfg* cfg, cudaStream_t st,
+                MsmForm form);
 
 // One digit sort shared by several shifted-table MSMs over the same scalars
 // (the Groth16 A, B1 and B2 queries all take the witness): sizes of its
@@ -739,11 +750,28 @@ __global__ void k_write_inf(Jac<F>* out)
     if (gtid() == 0) st_elem(out, Jac<F>{F::zero(), F::one(), F::zero()});
 }
 
+// Plain G1 bases are doubled by the endomorphism: half the windows, bucket
+// sets and serial doublings for the same additions.  (G2 has none that holds
+// for points outside the prime-order subgroup; a table needs none of these.)
+inline bool msm_glv(int group, size_t n, bool shared) { return group == 1 && !shared && n < (size_t(1) << 30); }
 // affine rounds of an MSM over bases in this layout
-inline uint32_t msm_rounds(size_t n, uint32_t c, bool shared, uint32_t layout)
+inline uint32_t msm_rounds(int group, size_t n, uint32_t c, bool shared, uint32_t layout)
 {
-    const size_t W = windows_for(c);
-    return layout == LZK_BASES_AFFINE ? affine_rounds(n * W, (shared ? 1 : W) << (c - 1)) : 0;
+    const bool glv = msm_glv(group, n, shared);
+    const size_t W = glv ? windows_glv(c) : windows_for(c);
+    return layout == LZK_BASES_AFFINE || glv ? affine_rounds(n * W * (glv ? 2 : 1), (shared ? 1 : W) << (c - 1)) : 0;
+}
+
+// out[i] = base i, out[n + i] = phi(base i)
+template <int LAYOUT>
+__global__ void k_glv_bases(const void* __restrict__ bases, size_t n, Aff<Fq>* __restrict__ out)
+{
+    for (uint64_t i = gtid(); i < n; i += gstride()) {
+        Aff<Fq> p = load_raw<Fq, LAYOUT>(bases, (uint32_t)i);
+        st_elem(out + i, p);
+        p.x = mul52(p.x, glv_beta());
+        st_elem(out + n + i, p);
+    }
 }
 
 // pre_off / pre_ent: bucket offsets and sorted entries of these scalars made
@@ -754,7 +782,7 @@ template <class Gp>
 int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>* out,
                    const lzk_msm_cfg* cfg, cudaStream_t st, uint32_t c_auto,
                    const uint32_t* pre_off = nullptr, const uint32_t* pre_ent = nullptr, uint32_t pre_rounds = 0,
-                   bool pre_in_ws = false)
+                   bool pre_in_ws = false, MsmForm form = kMsmFull)
 {
     using F = typename Gp::F;
     using X = XYZZ<F>;
@@ -782,13 +810,15 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
     uint32_t chunk = msm_chunk(cfg, group, n), run = msm_run(cfg, group, n);
     if (!tune_valid(LZK_TUNE_MSM_CHUNK, chunk) || !tune_valid(LZK_TUNE_MSM_REDUCE_RUN, run)) return LZK_EINVAL;
     MsmPlan p;
-    plan_msm<Gp>(p, n, c, shared, stride, chunk, run, pre_off ? pre_rounds : msm_rounds(n, c, shared, layout),
-                 pre_off && !pre_in_ws);
+    plan_msm<Gp>(p, n, c, shared, stride, chunk, run,
+                 form != kMsmFull ? 0 : pre_off ? pre_rounds : msm_rounds(group, n, c, shared, layout),
+                 pre_off && !pre_in_ws, form != kMsmLean && msm_glv(group, n, shared));
     void* tr_all = trace_begin(sizeof(F) == 32 ? "msm_g1" : "msm_g2", st);
     Scratch ws;
     int got = ws.acquire(p.bytes, cfg ? cfg->workspace : nullptr, cfg ? cfg->workspace_bytes : 0, st);
-    if (got != LZK_OK && p.rounds && !pre_off) {
-        // too little scratch for the affine rounds: XYZZ additions alone
+    if (got != LZK_OK && (p.rounds || p.glv) && !pre_off) {
+        // too little scratch for the affine rounds and the doubled bases: XYZZ
+        // additions alone
         plan_msm<Gp>(p, n, c, shared, stride, chunk, run);
         got = ws.acquire(p.bytes, cfg ? cfg->workspace : nullptr, cfg ? cfg->workspace_bytes : 0, st);
     }
@@ -812,11 +842,22 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
         LZK_TRY(msm_sort(p, scalars, cnt, off_ws, ent_ws, bsums, st));
         trace_end(tr_sort, st);
     }
+    if constexpr (sizeof(F) == 32) {
+        if (p.glv) {
+            A* phi = reinterpret_cast<A*>(base + p.o_phi);
+            const unsigned g = grid_for(n, 128, sm_count() * 16);
+            if (layout == LZK_BASES_AFFINE) k_glv_bases<LZK_BASES_AFFINE><<<g, 128, 0, st>>>(bases, n, phi);
+            else k_glv_bases<LZK_BASES_REF_G1_JAC><<<g, 128, 0, st>>>(bases, n, phi);
+            note_launch();
+            bases = phi;
+            layout = LZK_BASES_AFFINE;
+        }
+    }
     void* tr = trace_begin(sizeof(F) == 32 ? "msm_g1_accumulate" : "msm_g2_accumulate", st);
     {
         unsigned g = grid_for(p.chunks, 128);
         // base records the entries may name: the whole table, or the n bases
-        const uint64_t nbases = shared ? (uint64_t)cfg->precomp_windows * stride : (uint64_t)n;
+        const uint64_t nbases = shared ? (uint64_t)cfg->precomp_windows * stride : (uint64_t)n * (p.glv ? 2 : 1);
         constexpr int REF = sizeof(F) == 32 ? (int)LZK_BASES_REF_G1_JAC : (int)LZK_BASES_REF_G2_LANES;
         if (p.rounds) {
             A* fin = reinterpret_cast<A*>(base + p.o_fin);

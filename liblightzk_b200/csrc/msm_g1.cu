@@ -14,6 +14,12 @@ int msm_g1_presorted(const Fr* scalars, const void* table, size_t n, Jac<Fq>* ou
     return run_msm<G1>(scalars, table, n, out, cfg, st, cfg->window_bits, off, ent, rounds);
 }
 
+int msm_g1_form(const Fr* scalars, const void* bases, size_t n, Jac<Fq>* out, const lzk_msm_cfg* cfg, cudaStream_t st,
+                MsmForm form)
+{
+    return run_msm<G1>(scalars, bases, n, out, cfg, st, msm_autotune(1, n, false), nullptr, nullptr, 0, false, form);
+}
+
 int msm_g1_concat(const Fr* lo, size_t n_lo, const Fr* hi, size_t n_hi, const void* table, Jac<Fq>* out,
                   const lzk_msm_cfg* cfg, cudaStream_t st, uint32_t rounds)
 {

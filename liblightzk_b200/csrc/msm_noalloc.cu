@@ -80,8 +80,9 @@ static int noalloc_setup(char* scratch, int dev, cudaStream_t st)
     cfg.window_bits = 2;
     cfg.workspace = scratch + kIo;
     cfg.workspace_bytes = LZK_MSM_NOALLOC_SCRATCH_BYTES - kIo;
-    LZK_TRY(lzk_msm_g1(s, b, 0, out, &cfg, st));
-    LZK_TRY(lzk_msm_g1(s, b, 1, out, &cfg, st));
+    for (MsmForm form : {kMsmNoRounds, kMsmLean})
+        for (size_t n = 0; n < 2; n++)
+            LZK_TRY(msm_g1_form(reinterpret_cast<const Fr*>(s), b, n, reinterpret_cast<Jac<Fq>*>(out), &cfg, st, form));
     g_noalloc_ready[dev] = true;
     return LZK_OK;
 }
@@ -98,17 +99,19 @@ int lzk_msm_g1_noalloc(const lzk_fr_t* scalars, const lzk_g1_affine_t* bases, si
     if (n > LZK_MSM_NOALLOC_MAX_POINTS) return LZK_EINVAL;
     lzk_msm_cfg cfg = {};
     cfg.window_bits = window_bits;
-    // without the affine rounds: their scratch does not fit the array at every
-    // size it takes, and the set-up loads only the kernels of this form
-    size_t need = msm_lean_bytes(n, &cfg);
-    if (need > LZK_MSM_NOALLOC_SCRATCH_BYTES) return LZK_EINVAL;
+    // never the affine rounds (their scratch is too much for the array at most
+    // sizes), the endomorphism where its doubled bases fit
+    MsmForm form = kMsmNoRounds;
+    if (msm_form_bytes(n, &cfg, form) > LZK_MSM_NOALLOC_SCRATCH_BYTES) form = kMsmLean;
+    if (msm_form_bytes(n, &cfg, form) > LZK_MSM_NOALLOC_SCRATCH_BYTES) return LZK_EINVAL;
     void* scratch = nullptr;
     int dev = 0;
     LZK_TRY(noalloc_scratch(&scratch, &dev));
     LZK_TRY(noalloc_setup(static_cast<char*>(scratch), dev, as_stream(stream)));
     cfg.workspace = scratch;
-    cfg.workspace_bytes = need;
-    return lzk_msm_g1(scalars, bases, n, out, &cfg, stream);
+    cfg.workspace_bytes = LZK_MSM_NOALLOC_SCRATCH_BYTES;
+    return msm_g1_form(reinterpret_cast<const Fr*>(scalars), bases, n, reinterpret_cast<Jac<Fq>*>(out), &cfg,
+                       as_stream(stream), form);
 }
 
 }  // extern "C"

@@ -31,41 +31,47 @@
 
 namespace lzk {
 
-// bits [lo, lo+c) of a canonical 254-bit scalar held as 8 limbs
-__device__ __forceinline__ uint32_t window_bits(const uint32_t s[8], uint32_t lo, uint32_t c)
+// bits [lo, lo+c) of an integer of NW limbs
+template <int NW>
+__device__ __forceinline__ uint32_t window_bits(const uint32_t* s, uint32_t lo, uint32_t c)
 {
-    uint32_t w = lo >> 5, sh = lo & 31;
-    uint64_t v = s[w < 8 ? w : 7] >> sh;
-    if (w < 8 && sh) {
-        uint32_t hi = (w + 1 < 8) ? s[w + 1] : 0u;
-        v = ((uint64_t)s[w] | ((uint64_t)hi << 32)) >> sh;
-    } else if (w >= 8) {
-        v = 0;
-    }
+    const uint32_t w = lo >> 5, sh = lo & 31;
+    if (w >= NW) return 0;
+    const uint64_t v = ((uint64_t)s[w] | ((uint64_t)(w + 1 < NW ? s[w + 1] : 0u) << 32)) >> sh;
     return (uint32_t)v & ((1u << c) - 1u);
 }
 
-// Signed-digit recoding: raw = bits + carry in [0, 2^c]; raw > 2^(c-1) is
-// used as raw - 2^c with a carry into the next window.  |digit| <= 2^(c-1).
-struct DigitIter {
-    uint32_t s[8];
+// Signed-digit recoding of a magnitude: raw = bits + carry in [0, 2^c]; raw >
+// 2^(c-1) is used as raw - 2^c with a carry into the next window, so that
+// |digit| <= 2^(c-1).  f(w, |digit|, negative) for every non-zero digit.
+template <int NW, class Fn>
+__device__ __forceinline__ void for_digits(const uint32_t* s, uint32_t c, uint32_t W, bool neg, Fn f)
+{
     uint32_t carry = 0;
-    __device__ __forceinline__ void load(const Fr* sc)
-    {
-        Fr m = ldg_elem(sc);
-        Fr k = from_mont(m);
-        _Pragma("unroll") for (int i = 0; i < 8; i++) s[i] = k.v[i];
-        carry = 0;
+    const uint32_t half = 1u << (c - 1);
+    for (uint32_t w = 0; w < W; w++) {
+        const uint32_t raw = window_bits<NW>(s, w * c, c) + carry;
+        carry = raw > half ? 1u : 0u;
+        const uint32_t d = carry ? (1u << c) - raw : raw;
+        if (d) f(w, d, neg != (carry != 0));
     }
-    // returns |digit| (0 = skip) and sets neg
-    __device__ __forceinline__ uint32_t next(uint32_t w, uint32_t c, bool& neg)
-    {
-        uint32_t raw = window_bits(s, w * c, c) + carry;
-        uint32_t half = 1u << (c - 1);
-        if (raw > half) { carry = 1; neg = true; return (1u << c) - raw; }
-        carry = 0; neg = false; return raw;
+}
+// The digits of a scalar: of itself (h = 0), or (GLV) of its two halves, f(h,
+// w, |digit|, negative).
+template <bool GLV, class Fn>
+__device__ __forceinline__ void scalar_digits(const Fr* sc, uint32_t c, uint32_t W, Fn f)
+{
+    const Fr k = from_mont(ldg_elem(sc));
+    if (GLV) {
+        uint32_t k1[4], k2[4];
+        bool n1, n2;
+        glv_split(k.v, k1, n1, k2, n2);
+        for_digits<4>(k1, c, W, n1, [&](uint32_t w, uint32_t d, bool neg) { f(0u, w, d, neg); });
+        for_digits<4>(k2, c, W, n2, [&](uint32_t w, uint32_t d, bool neg) { f(1u, w, d, neg); });
+    } else {
+        for_digits<8>(k.v, c, W, false, [&](uint32_t w, uint32_t d, bool neg) { f(0u, w, d, neg); });
     }
-};
+}
 
 // Scalar i of an MSM whose scalars are the concatenation of two arrays:
 // lo[0..split) then hi[0..n - split) (one array: split = n, hi unused).
@@ -74,40 +80,35 @@ __device__ __forceinline__ const Fr* scalar_at(const Fr* lo, const Fr* hi, size_
     return i < split ? lo + i : hi + (i - split);
 }
 
+template <bool GLV>
 __global__ void k_count(const Fr* __restrict__ scalars, const Fr* __restrict__ hi, size_t split, size_t n, uint32_t c,
                         uint32_t W, uint32_t nb, bool shared, uint32_t* __restrict__ cnt)
 {
     const uint32_t B = shared ? nb : W * nb;
     (void)B;
-    for (uint64_t i = gtid(); i < n; i += gstride()) {
-        DigitIter it; it.load(scalar_at(scalars, hi, split, i));
-        for (uint32_t w = 0; w < W; w++) {
-            bool neg; uint32_t d = it.next(w, c, neg);
-            uint32_t b = (shared ? 0u : w * nb) + d - 1;
-            if (d && LZK_CHECK(b < B, 0)) atomicAdd(cnt + b, 1u);
-        }
-    }
+    for (uint64_t i = gtid(); i < n; i += gstride())
+        scalar_digits<GLV>(scalar_at(scalars, hi, split, i), c, W, [&](uint32_t, uint32_t w, uint32_t d, bool) {
+            const uint32_t b = (shared ? 0u : w * nb) + d - 1;
+            if (LZK_CHECK(b < B, 0)) atomicAdd(cnt + b, 1u);
+        });
 }
 
+template <bool GLV>
 __global__ void k_scatter(const Fr* __restrict__ scalars, const Fr* __restrict__ hi, size_t split, size_t n,
                           uint32_t c, uint32_t W, uint32_t nb, bool shared, size_t stride,
                           const uint32_t* __restrict__ off, uint32_t* __restrict__ cnt, uint32_t* __restrict__ ent)
 {
     const uint32_t B = shared ? nb : W * nb;
     (void)B;
-    for (uint64_t i = gtid(); i < n; i += gstride()) {
-        DigitIter it; it.load(scalar_at(scalars, hi, split, i));
-        for (uint32_t w = 0; w < W; w++) {
-            bool neg; uint32_t d = it.next(w, c, neg);
-            if (!d) continue;
-            uint32_t b = (shared ? 0u : w * nb) + d - 1;
-            if (!LZK_CHECK(b < B, 0)) continue;
-            uint32_t slot = off[b] + atomicSub(cnt + b, 1u) - 1u;
-            if (!LZK_CHECK(slot >= off[b] && slot < off[b + 1], 1)) continue;
-            uint32_t idx = (uint32_t)(shared ? (size_t)w * stride + i : i);
+    for (uint64_t i = gtid(); i < n; i += gstride())
+        scalar_digits<GLV>(scalar_at(scalars, hi, split, i), c, W, [&](uint32_t h, uint32_t w, uint32_t d, bool neg) {
+            const uint32_t b = (shared ? 0u : w * nb) + d - 1;
+            if (!LZK_CHECK(b < B, 0)) return;
+            const uint32_t slot = off[b] + atomicSub(cnt + b, 1u) - 1u;
+            if (!LZK_CHECK(slot >= off[b] && slot < off[b + 1], 1)) return;
+            const uint32_t idx = (uint32_t)(shared ? (size_t)w * stride + i : (size_t)h * n + i);
             ent[slot] = idx | (neg ? 0x80000000u : 0u);
-        }
-    }
+        });
 }
 
 // Exclusive scan of cnt[0..B), each count rounded up to a multiple of
@@ -188,11 +189,11 @@ int msm_sort(const MsmPlan& p, const Fr* scalars, uint32_t* cnt, uint32_t* off, 
     if (split > p.n) return LZK_EINVAL;
     LZK_CUDA(cudaMemsetAsync(cnt, 0, sizeof(uint32_t) * p.B, st));
     unsigned g = grid_for(p.n, 256, sm_count() * 16);
-    k_count<<<g, 256, 0, st>>>(scalars, hi, split, p.n, p.c, p.W, p.nb, p.shared, cnt); note_launch();
+    (p.glv ? k_count<true> : k_count<false>)<<<g, 256, 0, st>>>(scalars, hi, split, p.n, p.c, p.W, p.nb, p.shared, cnt); note_launch();
     LZK_TRY(scan_offsets(cnt, p.B, off, bsums, st, p.rounds));
     // the gaps that pad buckets keep kNoEntry
     if (p.rounds) LZK_CUDA(cudaMemsetAsync(ent, 0xff, sizeof(uint32_t) * p.max_slots, st));
-    k_scatter<<<g, 256, 0, st>>>(scalars, hi, split, p.n, p.c, p.W, p.nb, p.shared, p.stride, off, cnt, ent); note_launch();
+    (p.glv ? k_scatter<true> : k_scatter<false>)<<<g, 256, 0, st>>>(scalars, hi, split, p.n, p.c, p.W, p.nb, p.shared, p.stride, off, cnt, ent); note_launch();
     return launch_status();
 }
 
@@ -211,9 +212,10 @@ uint32_t msm_autotune(int group, size_t n, bool shared)
     if (n == 0) return 8;
     double best = 1e300; uint32_t bc = 8;
     for (uint32_t c = 4; c <= 22; c++) {
-        double W = windows_for(c);
+        const bool glv = msm_glv(group, n, shared);
+        double W = glv ? windows_glv(c) : windows_for(c);
         double sets = shared ? 1.0 : W;
-        double cost = (double)n * W * 10.0 + sets * (double)(1u << (c - 1)) * 2.0 * 14.0;
+        double cost = (double)n * (glv ? 2.0 : 1.0) * W * 10.0 + sets * (double)(1u << (c - 1)) * 2.0 * 14.0;
         if (!shared) cost += W * c * 9.0 * 2000.0;  // serial doublings are latency bound
         if (shared && (double)n * W > 1.9e9) continue;
         if (cost < best) { best = cost; bc = c; }
@@ -256,12 +258,12 @@ size_t msm_concat_bytes(size_t n, const lzk_msm_cfg* cfg, uint32_t rounds)
     return p.bytes;
 }
 
-size_t msm_lean_bytes(size_t n, const lzk_msm_cfg* cfg)
+size_t msm_form_bytes(size_t n, const lzk_msm_cfg* cfg, MsmForm form)
 {
     const uint32_t c = cfg->window_bits ? cfg->window_bits : msm_autotune(1, n, false);
     if (c < 2 || c > 24 || n == 0) return 0;
     MsmPlan p;
-    plan_msm<G1>(p, n, c, false, 0, msm_chunk(cfg, 1, n), msm_run(cfg, 1, n));
+    plan_msm<G1>(p, n, c, false, 0, msm_chunk(cfg, 1, n), msm_run(cfg, 1, n), 0, false, form != kMsmLean);
     return p.bytes;
 }
 
@@ -288,9 +290,9 @@ size_t lzk_msm_workspace_bytes(int group, size_t n, const lzk_msm_cfg* cfg)
     uint32_t chunk = msm_chunk(cfg, group, n), run = msm_run(cfg, group, n);
     if (!tune_valid(LZK_TUNE_MSM_CHUNK, chunk)) return 0;
     MsmPlan p;
-    const uint32_t rounds = msm_rounds(n, c, shared, cfg ? cfg->base_layout : (uint32_t)LZK_BASES_AFFINE);
+    const uint32_t rounds = msm_rounds(group, n, c, shared, cfg ? cfg->base_layout : (uint32_t)LZK_BASES_AFFINE);
     if (group == 2) plan_msm<G2>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run, rounds);
-    else plan_msm<G1>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run, rounds);
+    else plan_msm<G1>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run, rounds, false, msm_glv(group, n, shared));
     return p.bytes;
 }
 

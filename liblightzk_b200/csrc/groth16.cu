@@ -6,8 +6,8 @@
 // fixed sequence of launches on three streams with no host round trip:
 //
 //   stream main : SpMV A z, B z, C z -> H polynomial -> L + H MSM -> assembly
-//   stream s1   : A MSM, B1 MSM
-//   stream s2   : B2 MSM (G2), after the A MSM
+//   stream s1   : A MSM, B1 MSM (short ones: B1 beside A, on s4)
+//   stream s2   : B2 MSM (G2), beside the A MSM
 //   stream s3   : fixed-point products r d1, s a1, r b1, (r s) d1, s d2 from
 //                 comb tables; after B1: s*A and r*B1 (variable base)
 //
@@ -235,7 +235,7 @@ void ctx_destroy(ProveCtx* x)
     for (auto m : misc) if (m) cudaFree(m);
     if (x->proof_host) cudaFreeHost(x->proof_host);
     if (x->ev_done) cudaEventDestroy(x->ev_done);
-    cudaStream_t sts[] = {x->s0, x->s1, x->s2, x->s3};
+    cudaStream_t sts[] = {x->s0, x->s1, x->s2, x->s3, x->s4};
     for (auto t : sts) if (t) cudaStreamDestroy(t);
     cudaEvent_t evs[] = {x->ev_fork, x->ev_b1, x->ev_s1, x->ev_s2, x->ev_s3, x->ev_sorted};
     for (auto e : evs) if (e) cudaEventDestroy(e);
@@ -247,8 +247,12 @@ void ctx_destroy(ProveCtx* x)
 struct CtxShape {
     uint32_t lh_rounds = 0, z_rounds = 0;
     SortWords sort;
-    size_t wsb[3];
+    size_t wsb[4] = {0, 0, 0, 0};
 };
+// B1 runs beside A, in a workspace of its own, as long as one of them leaves
+// most of the device idle (2^12 constraints: 1262 -> 988 us); longer MSMs
+// fill it, and B1 follows A in the same workspace.
+constexpr size_t kParallelEntries = size_t(1) << 20;
 static CtxShape ctx_shape(const lzk_prover* p, bool lean)
 {
     CtxShape s;
@@ -266,6 +270,7 @@ static CtxShape ctx_shape(const lzk_prover* p, bool lean)
         if (i) s.wsb[i] = msm_presorted_bytes(i == 2 ? 2 : 1, n, &cfg, s.z_rounds);
         else s.wsb[i] = msm_concat_bytes(n, &cfg, s.lh_rounds);
     }
+    if (!lean && p->n_vars * p->wins <= kParallelEntries) s.wsb[3] = s.wsb[1];
     return s;
 }
 
@@ -274,7 +279,7 @@ size_t ctx_bytes(const lzk_prover* p, bool serving, bool lean)
 {
     const CtxShape s = ctx_shape(p, lean);
     size_t b = 3 * p->L * sizeof(Fr) + 4 * sizeof(Jac<Fq>) + sizeof(Jac<Fq2>) + 6 * sizeof(XYZZ<Fq>) + sizeof(XYZZ<Fq2>);
-    b += s.wsb[0] + s.wsb[1] + s.wsb[2] + 4 * (s.sort.cnt + s.sort.off + s.sort.ent + s.sort.bsums);
+    b += s.wsb[0] + s.wsb[1] + s.wsb[2] + s.wsb[3] + 4 * (s.sort.cnt + s.sort.off + s.sort.ent + s.sort.bsums);
     return serving ? b + p->n_vars * sizeof(Fr) + sizeof(lzk_groth16_proof) : b;
 }
 
@@ -296,8 +301,9 @@ int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out, bool lean)
         if ((rc = dalloc(&x->bytes, &x->g2res, 1))) break;
         if ((rc = dalloc(&x->bytes, &x->sm1, 6))) break;
         if ((rc = dalloc(&x->bytes, &x->sm2, 1))) break;
-        for (int i = 0; i < 3 && rc == LZK_OK; i++) {
+        for (int i = 0; i < 4 && rc == LZK_OK; i++) {
             x->wsb[i] = s.wsb[i];
+            if (!s.wsb[i]) continue;
             rc = dalloc(&x->bytes, reinterpret_cast<char**>(&x->ws[i]), x->wsb[i]);
         }
         if (rc) break;
@@ -312,7 +318,7 @@ int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out, bool lean)
             if (cudaEventCreateWithFlags(&x->ev_done, cudaEventDisableTiming) != cudaSuccess) { rc = LZK_EDEVICE; break; }
             if (cudaMallocHost(&x->proof_host, sizeof(lzk_groth16_proof)) != cudaSuccess) { rc = LZK_ENOMEM; break; }
         }
-        cudaStream_t* sts[] = {&x->s1, &x->s2, &x->s3};
+        cudaStream_t* sts[] = {&x->s1, &x->s2, &x->s3, &x->s4};
         for (auto t : sts) if (cudaStreamCreateWithFlags(t, cudaStreamNonBlocking) != cudaSuccess) rc = LZK_EDEVICE;
         cudaEvent_t* evs[] = {&x->ev_fork, &x->ev_b1, &x->ev_s1, &x->ev_s2, &x->ev_s3, &x->ev_sorted};
         for (auto e : evs) if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) rc = LZK_EDEVICE;
@@ -333,6 +339,18 @@ static void destroy(lzk_prover* p)
     delete p;
 }
 
+// Window width of a prover's tables when the caller leaves it open, by the
+// witness's length n (proofs measured at every width): 13 up to 24 k variables
+// (8194: 994 us, 15: 1048; 17 before: 2201), 15 up to 100 k (36866: 1625, 13: 1706,
+// 16: 2097 before B1 ran beside A), 16 up to 500 k (266242: 6477, 15 and 17: 6663), then 17 (1052674:
+// 20.05 ms, 16: 21.3).  Narrow windows leave fewer buckets to reduce, wide ones
+// fewer additions; widths between them (11, 12, 14) leave a short top window,
+// whose few buckets fill up.
+static uint32_t prover_window(size_t n)
+{
+    return n < 24000 ? 13 : n < 100000 ? 15 : n < 500000 ? 16 : 17;
+}
+
 static int create(const lzk_groth16_circuit* c, const lzk_groth16_pk* pk, int mode, uint32_t window_bits, bool lean,
                   lzk_prover* p)
 {
@@ -351,7 +369,7 @@ static int create(const lzk_groth16_circuit* c, const lzk_groth16_pk* pk, int mo
     p->n_public = c->n_public;
     if (!pk->a_query || !pk->b1_query || !pk->b2_query || !pk->h_query || (!pk->l_query && c->n_vars > c->n_public + 1))
         return LZK_EINVAL;
-    p->c = window_bits ? window_bits : 17;
+    p->c = window_bits ? window_bits : prover_window(c->n_vars);
     if (p->c < 2 || p->c > 24) return LZK_EINVAL;
     p->wins = windows_for(p->c);
     // level strides of the tables (ctx_create sizes the MSM workspaces by them)
@@ -434,7 +452,7 @@ static int create(const lzk_groth16_circuit* c, const lzk_groth16_pk* pk, int mo
 static int msm_tab1(const lzk_prover* p, ProveCtx* x, int q, const Fr* scal, size_t n, Jac<Fq>* out, int wsi,
                     cudaStream_t st, bool presorted = false)
 {
-    lzk_msm_cfg cfg = prover_msm_cfg(p, wsi, p->tn[q]);
+    lzk_msm_cfg cfg = prover_msm_cfg(p, wsi == 3 ? 1 : wsi, p->tn[q]);
     cfg.workspace = x->ws[wsi];
     cfg.workspace_bytes = x->wsb[wsi];
     if (presorted) return msm_g1_presorted(scal, p->tab[q], n, out, &cfg, st, x->zs_off, x->zs_ent, x->z_rounds);
@@ -462,14 +480,13 @@ int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, 
     // window width, tables of the same level stride n_vars)
     LZK_TRY(msm_sort_scalars(z, p->n_vars, p->c, p->n_vars, x->zs_cnt, x->zs_off, x->zs_ent, x->zs_bsums, x->s1, x->z_rounds));
 
+    LZK_CUDA(cudaEventRecord(x->ev_sorted, x->s1));
     // s1: A and B1 MSMs; s3 picks up A and B1 for s*A and r*B1
     LZK_TRY(msm_tab1(p, x, 0, z, p->n_vars, x->g1res + 0, 1, x->s1, true));
 
-    // s2: the G2 MSM, from the same sort, once the A MSM is done: started
-    // beside the A MSM its 2000-block accumulation kept the A MSM's fix-up
-    // and reduction waiting, which delayed B1 and the products that end the
-    // proof (measured 30.00 -> 29.73 ms per proof)
-    LZK_CUDA(cudaEventRecord(x->ev_sorted, x->s1));
+    // s2: the G2 MSM, the longest chain, from the same sort, beside the A MSM
+    // (after it, as was best for the all-XYZZ accumulation, a proof takes 1698
+    // instead of 1334 us at 2^12 constraints, 20.3 instead of 20.0 ms at 2^20)
     LZK_CUDA(cudaStreamWaitEvent(x->s2, x->ev_sorted, 0));
     {
         lzk_msm_cfg cfg = prover_msm_cfg(p, 2, p->tn2);
@@ -479,7 +496,15 @@ int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, 
     }
     LZK_CUDA(cudaEventRecord(x->ev_s2, x->s2));
 
-    LZK_TRY(msm_tab1(p, x, 1, z, p->n_vars, x->g1res + 1, 1, x->s1, true));
+    // B1 after A, or beside it on s4
+    if (x->ws[3]) {
+        LZK_CUDA(cudaStreamWaitEvent(x->s4, x->ev_sorted, 0));
+        LZK_TRY(msm_tab1(p, x, 1, z, p->n_vars, x->g1res + 1, 3, x->s4, true));
+        LZK_CUDA(cudaEventRecord(x->ev_b1, x->s4));
+        LZK_CUDA(cudaStreamWaitEvent(x->s1, x->ev_b1, 0));
+    } else {
+        LZK_TRY(msm_tab1(p, x, 1, z, p->n_vars, x->g1res + 1, 1, x->s1, true));
+    }
     LZK_CUDA(cudaEventRecord(x->ev_b1, x->s1));
     LZK_CUDA(cudaStreamWaitEvent(x->s3, x->ev_b1, 0));
     void* tr_dep = trace_begin("groth16_dep_products", x->s3);

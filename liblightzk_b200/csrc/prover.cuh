@@ -23,15 +23,16 @@ struct ProveCtx {
     Jac<Fq2>* g2res = nullptr;        // B2 MSM result
     XYZZ<Fq>* sm1 = nullptr;          // r d1, s a1, r b1, (r s) d1, s A, r B1
     XYZZ<Fq2>* sm2 = nullptr;         // s d2
-    void* ws[3] = {nullptr, nullptr, nullptr};
-    size_t wsb[3] = {0, 0, 0};
+    void* ws[4] = {nullptr, nullptr, nullptr, nullptr};   // L + H; A (and B1); B2; B1 where it runs beside A
+    size_t wsb[4] = {0, 0, 0, 0};
     // one digit sort of the witness, shared by the A, B1 and B2 MSMs
     uint32_t *zs_cnt = nullptr, *zs_off = nullptr, *zs_ent = nullptr, *zs_bsums = nullptr;
     Fr* z = nullptr;                  // witness buffer (serving contexts only)
     lzk_groth16_proof* proof = nullptr;   // proof buffer (serving contexts only)
     lzk_groth16_proof* proof_host = nullptr;   // pinned copy target (serving contexts only)
     cudaEvent_t ev_done = nullptr;             // end of the proof on s0 (serving contexts only)
-    cudaStream_t s0 = nullptr, s1 = nullptr, s2 = nullptr, s3 = nullptr;   // s0: serving contexts only
+    cudaStream_t s0 = nullptr, s1 = nullptr, s2 = nullptr, s3 = nullptr,   // s0: serving contexts only
+                 s4 = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_b1 = nullptr, ev_s1 = nullptr, ev_s2 = nullptr, ev_s3 = nullptr,
                 ev_sorted = nullptr;
     uint32_t lh_rounds = 0, z_rounds = 0;   // affine rounds of the L + H MSM; of A, B1 and B2

@@ -4,7 +4,7 @@
 // and launches (msm.cuh:210-247, poly.cuh:65-73).  A batch plan lays every
 // MSM of the batch into one global bucket space and runs each MSM phase
 // once for the whole batch:
-//   gather bases -> digit count -> offset scan -> scatter -> accumulate
+//   gather bases (plain G1: twice, glv.cuh) -> digit count -> offset scan -> scatter -> accumulate
 //   -> fix-up -> bucket reduction (one level chain per window width) ->
 //   window combination (one warp per MSM)
 // so 64 MSMs cost about the launches of one; with LZK_BATCH_PERSISTENT
@@ -49,6 +49,7 @@ struct lzk_batch_plan {
     struct NGroup { uint32_t k; int dir; uint32_t count; lzk::Fr** ptrs; };
     std::vector<NGroup> ngroups;
     uint64_t total_pts = 0, total_buckets = 0, total_windows = 0, max_entries = 0, chunks = 0, lvl = 0;
+    bool glv = false;                  // plain G1: scalars in two halves, bases doubled (glv.cuh)
     uint32_t rounds = 0;               // affine rounds before the accumulation
     uint64_t max_slots = 0, slice = 0;
     char* aff = nullptr;               // their scratch, and the points they leave
@@ -82,55 +83,52 @@ __device__ __forceinline__ uint32_t find_msm(const uint64_t* ptsoff, uint32_t co
     return lo;
 }
 
-template <class F>
+// the bases of all MSMs in one array; with GLV each MSM's n bases are followed
+// by their images under the endomorphism
+template <class F, bool GLV>
 __global__ void k_bgather(const BDesc* __restrict__ d, const uint64_t* __restrict__ ptsoff, uint32_t count,
                           uint64_t total, Aff<F>* __restrict__ dst)
 {
     for (uint64_t i = gtid(); i < total; i += gstride()) {
-        uint32_t k = find_msm(ptsoff, count, i);
-        st_elem(dst + i, ldg_elem(reinterpret_cast<const Aff<F>*>(d[k].bases) + (i - d[k].pts_off)));
+        const BDesc& m = d[find_msm(ptsoff, count, i)];
+        const uint64_t at = i - m.pts_off;
+        Aff<F> p = ldg_elem(reinterpret_cast<const Aff<F>*>(m.bases) + at);
+        if constexpr (GLV) {
+            Aff<F>* o = dst + 2 * m.pts_off + at;
+            st_elem(o, p);
+            p.x = mul52(p.x, glv_beta());
+            st_elem(o + m.n, p);
+        } else {
+            st_elem(dst + i, p);
+        }
     }
 }
 
-// signed digits of every scalar of the batch (the recoding of msm_sort.cu)
-__device__ __forceinline__ uint32_t bwindow_bits(const uint32_t s[8], uint32_t lo, uint32_t c)
-{
-    uint32_t w = lo >> 5, sh = lo & 31;
-    if (w >= 8) return 0;
-    uint64_t v = ((uint64_t)s[w] | ((uint64_t)(w + 1 < 8 ? s[w + 1] : 0u) << 32)) >> sh;
-    return (uint32_t)v & ((1u << c) - 1u);
-}
-
-// With tables (shared = true) every window of an MSM lands in its one
-// bucket set and an entry names the table copy of its window:
-// tab_off + w n + i; with plain bases each window has its own set and an
-// entry names the gathered base i.
-template <bool SCATTER>
+// Digits of every scalar of the batch (scalar_digits).  With tables (shared =
+// true) every window of an MSM lands in its one bucket set and an entry names
+// the table copy of its window: tab_off + w n + i; with plain bases each
+// window has its own set and an entry names the gathered base, half h of a
+// scalar (GLV) the second copy of the bases.
+template <bool SCATTER, bool GLV>
 __global__ void k_bdigits(const BDesc* __restrict__ d, const uint64_t* __restrict__ ptsoff, uint32_t count,
                           uint64_t total, bool shared, const uint32_t* __restrict__ off, uint32_t* __restrict__ cnt,
                           uint32_t* __restrict__ ent)
 {
     for (uint64_t i = gtid(); i < total; i += gstride()) {
-        uint32_t k = find_msm(ptsoff, count, i);
+        const uint32_t k = find_msm(ptsoff, count, i);
         const BDesc& m = d[k];
-        Fr sc = from_mont(ldg_elem(m.scalars + (i - m.pts_off)));
-        uint32_t carry = 0, half = m.nb;
-        for (uint32_t w = 0; w < m.W; w++) {
-            uint32_t raw = bwindow_bits(sc.v, w * m.c, m.c) + carry;
-            uint32_t a;
-            bool neg;
-            if (raw > half) { carry = 1; neg = true; a = (1u << m.c) - raw; }
-            else { carry = 0; neg = false; a = raw; }
-            if (!a) continue;
-            uint32_t b = (uint32_t)(m.bucket_base + (shared ? 0 : (uint64_t)w * m.nb) + a - 1);
+        const uint64_t at = i - m.pts_off;
+        scalar_digits<GLV>(m.scalars + at, m.c, m.W, [&](uint32_t h, uint32_t w, uint32_t a, bool neg) {
+            const uint32_t b = (uint32_t)(m.bucket_base + (shared ? 0 : (uint64_t)w * m.nb) + a - 1);
             if (SCATTER) {
-                uint32_t slot = off[b] + atomicSub(cnt + b, 1u) - 1u;
-                uint32_t idx = shared ? (uint32_t)(m.tab_off + (uint64_t)w * m.n + (i - m.pts_off)) : (uint32_t)i;
-                ent[slot] = idx | (neg ? 0x80000000u : 0u);
+                const uint32_t slot = off[b] + atomicSub(cnt + b, 1u) - 1u;
+                const uint64_t idx = shared ? m.tab_off + (uint64_t)w * m.n + at
+                                            : (GLV ? 2 : 1) * m.pts_off + h * m.n + at;
+                ent[slot] = (uint32_t)idx | (neg ? 0x80000000u : 0u);
             } else {
                 atomicAdd(cnt + b, 1u);
             }
-        }
+        });
     }
 }
 
@@ -278,7 +276,7 @@ static int run_persistent(lzk_batch_plan* p, cudaStream_t st)
     a.B = (uint32_t)p->total_buckets;
     a.chunk = p->chunk;
     a.chunks = p->chunks;
-    a.nbases = p->fixed ? p->table_pts : p->total_pts;
+    a.nbases = p->fixed ? p->table_pts : p->total_pts * (p->glv ? 2 : 1);
     a.bsum = static_cast<X*>(p->bsum);
     a.head = static_cast<X*>(p->head);
     a.tail = static_cast<X*>(p->tail);
@@ -306,19 +304,26 @@ template <class F>
 static int run_plan(lzk_batch_plan* p, cudaStream_t st)
 {
     using X = XYZZ<F>;
+    using K = typename LaneOf<F>::T;
+    constexpr uint32_t LP = MemOf<K>::lanes;
     uint32_t count = (uint32_t)p->msm.size();
     if (count && p->total_pts) {
         unsigned g = grid_for(p->total_pts, 256, sm_count() * 16);
         void* tr = trace_begin("batch_msm_sort", st);
         if (!p->fixed) {
-            k_bgather<F><<<g, 256, 0, st>>>(p->d_desc, p->d_ptsoff, count, p->total_pts, static_cast<Aff<F>*>(p->bases)); note_launch();
+            Aff<F>* to = static_cast<Aff<F>*>(p->bases);
+            if constexpr (sizeof(F) == 32) {
+                if (p->glv) k_bgather<F, true><<<g, 256, 0, st>>>(p->d_desc, p->d_ptsoff, count, p->total_pts, to);
+            }
+            if (!p->glv) k_bgather<F, false><<<g, 256, 0, st>>>(p->d_desc, p->d_ptsoff, count, p->total_pts, to);
+            note_launch();
         }
         LZK_CUDA(cudaMemsetAsync(p->cnt, 0, sizeof(uint32_t) * p->total_buckets, st));
-        k_bdigits<false><<<g, 256, 0, st>>>(p->d_desc, p->d_ptsoff, count, p->total_pts, p->fixed, p->off, p->cnt, p->ent); note_launch();
+        (p->glv ? k_bdigits<false, true> : k_bdigits<false, false>)<<<g, 256, 0, st>>>(p->d_desc, p->d_ptsoff, count, p->total_pts, p->fixed, p->off, p->cnt, p->ent); note_launch();
         LZK_TRY(scan_offsets(p->cnt, (uint32_t)p->total_buckets, p->off, p->bsums, st, p->rounds));
         // the gaps that pad buckets keep kNoEntry
         if (p->rounds) LZK_CUDA(cudaMemsetAsync(p->ent, 0xff, sizeof(uint32_t) * p->max_slots, st));
-        k_bdigits<true><<<g, 256, 0, st>>>(p->d_desc, p->d_ptsoff, count, p->total_pts, p->fixed, p->off, p->cnt, p->ent); note_launch();
+        (p->glv ? k_bdigits<true, true> : k_bdigits<true, false>)<<<g, 256, 0, st>>>(p->d_desc, p->d_ptsoff, count, p->total_pts, p->fixed, p->off, p->cnt, p->ent); note_launch();
         trace_end(tr, st);
         if (p->persistent) {
             tr = trace_begin("batch_msm_persistent", st);
@@ -329,41 +334,41 @@ static int run_plan(lzk_batch_plan* p, cudaStream_t st)
         X* bsum = static_cast<X*>(p->bsum);
         tr = trace_begin("batch_msm_accumulate", st);
         const void* pts = p->fixed ? p->table : p->bases;
-        const uint64_t npts = p->fixed ? p->table_pts : p->total_pts;
+        const uint64_t npts = p->fixed ? p->table_pts : p->total_pts * (p->glv ? 2 : 1);
         if (p->rounds) {
             Aff<F>* fin = static_cast<Aff<F>*>(p->fin);
             LZK_TRY(affine_sum<F>(pts, p->ent, p->off + p->total_buckets, p->max_slots, p->slice, p->rounds, npts, p->aff, fin, st));
-            k_accumulate<F, kLayoutPoints><<<grid_for(p->chunks, 128), 128, 0, st>>>(
+            k_accumulate<K, kLayoutPoints><<<grid_for(p->chunks * LP, 128), 128, 0, st>>>(
                 fin, p->ent, p->off, (uint32_t)p->total_buckets, p->chunks, p->chunk, p->rounds, p->max_slots >> p->rounds,
                 bsum, static_cast<X*>(p->head), static_cast<X*>(p->tail)); note_launch();
         } else {
-            k_accumulate<F, LZK_BASES_AFFINE><<<grid_for(p->chunks, 128), 128, 0, st>>>(
+            k_accumulate<K, LZK_BASES_AFFINE><<<grid_for(p->chunks * LP, 128), 128, 0, st>>>(
                 pts, p->ent, p->off, (uint32_t)p->total_buckets, p->chunks, p->chunk, 0, npts, bsum,
                 static_cast<X*>(p->head), static_cast<X*>(p->tail)); note_launch();
         }
         trace_end(tr, st);
         tr = trace_begin("batch_msm_fixup", st);
         LZK_CUDA(cudaMemsetAsync(p->large, 0, sizeof(uint32_t), st));
-        k_fixup<F><<<grid_for(p->total_buckets, 256, sm_count() * 8), 256, 0, st>>>(p->off, (uint32_t)p->total_buckets, p->chunk, p->rounds, p->chunks, bsum,
+        k_fixup<K><<<grid_for(p->total_buckets * LP, 256, sm_count() * 8), 256, 0, st>>>(p->off, (uint32_t)p->total_buckets, p->chunk, p->rounds, p->chunks, bsum,
                                                                             static_cast<X*>(p->head),
                                                                             static_cast<X*>(p->tail), p->large); note_launch();
-        constexpr unsigned fx_threads = 32768 / sizeof(X);
-        k_fixup_large<F><<<sm_count() * 2, fx_threads, fx_threads * sizeof(X), st>>>(p->off, p->chunk, p->rounds, bsum, static_cast<X*>(p->head),
+        constexpr unsigned fx_points = 32768 / sizeof(X);
+        k_fixup_large<K><<<sm_count() * 2, fx_points * LP, fx_points * sizeof(X), st>>>(p->off, p->chunk, p->rounds, bsum, static_cast<X*>(p->head),
                                                                              static_cast<X*>(p->tail), p->large); note_launch();
         trace_end(tr, st);
         // the bucket reductions of all window widths, in the same four launches
         tr = trace_begin("batch_msm_reduce", st);
-        std::vector<RedJob<F>> jobs;
+        std::vector<RedJob<K>> jobs;
         uint64_t wdone = 0;
         for (auto& wg : p->wgroups) {
             const uint64_t o = wg.scratch_off;
-            jobs.push_back(red_job<F>(bsum + wg.bucket_base, p->off + wg.bucket_base, (uint32_t)wg.windows,
+            jobs.push_back(red_job<K>(bsum + wg.bucket_base, p->off + wg.bucket_base, (uint32_t)wg.windows,
                                       1u << (wg.c - 1), wg.run, static_cast<X*>(p->lr[0]) + o,
                                       static_cast<X*>(p->la[0]) + o, static_cast<X*>(p->lr[1]) + o,
                                       static_cast<X*>(p->la[1]) + o, static_cast<X*>(p->wres) + wdone));
             wdone += wg.windows;
         }
-        LZK_TRY(reduce_jobs<F>(jobs.data(), jobs.size(), st));
+        LZK_TRY(reduce_jobs<K>(jobs.data(), jobs.size(), st));
         trace_end(tr, st);
     }
     if (count && !(p->persistent && p->total_pts)) {
@@ -403,6 +408,29 @@ static void destroy_plan(lzk_batch_plan* p)
     delete p;
 }
 
+// Window width of an MSM of n points in a plan that leaves it open: the tuned
+// one of such an MSM alone, but in a plan with points enough to fill the device
+// (kWidePlan) not wider than the cheapest by work, 8 products an addition of an
+// entry and 40 a bucket for its reduction, which in an MSM alone idle lanes do
+// for nothing.  Widths that leave a short top window (its few buckets fill up)
+// are passed over.  A fixed-bases plan of 24 MSMs up to 2^18 and one of 22 up to
+// 2^13 points: 4716 and 720 us, against 5025 and 946 with the tuned widths.
+constexpr size_t kWidePlan = size_t(1) << 15;
+static uint32_t batch_window(int group, size_t n, bool fixed, bool glv, bool wide)
+{
+    const uint32_t tuned = msm_autotune(group, n, fixed), bits = glv ? kGlvBits + 1 : 255;
+    if (!wide) return tuned;
+    uint32_t best = tuned;
+    double least = 1e300;
+    for (uint32_t c = 4; c <= tuned; c++) {
+        const uint32_t W = glv ? windows_glv(c) : windows_for(c);
+        if (c != tuned && W * c > bits + 5) continue;
+        const double cost = (double)n * (glv ? 2 : 1) * W * 8.0 + (fixed ? 1.0 : W) * (double)(1u << (c - 1)) * 40.0;
+        if (cost < least) { least = cost; best = c; }
+    }
+    return best;
+}
+
 template <class F>
 static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_desc* ntts, size_t n_ntt,
                        lzk_batch_plan* p, bool with_rounds)
@@ -411,9 +439,13 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
     // MSMs: widths, ordering, global layout
     std::vector<size_t> order(n_msm);
     std::vector<uint32_t> cw(n_msm);
+    size_t all = 0;
+    for (size_t i = 0; i < n_msm; i++) all += msms[i].n;
+    p->glv = with_rounds && !p->fixed && p->group == 1 && all < (size_t(1) << 30);
+    const bool wide = all >= kWidePlan;
     for (size_t i = 0; i < n_msm; i++) {
         if (!msms[i].out || (msms[i].n && (!msms[i].scalars || !msms[i].bases))) return LZK_EINVAL;
-        cw[i] = msms[i].window_bits ? msms[i].window_bits : msm_autotune(p->group, msms[i].n, p->fixed);
+        cw[i] = msms[i].window_bits ? msms[i].window_bits : batch_window(p->group, msms[i].n, p->fixed, p->glv, wide);
         if (cw[i] < 2 || cw[i] > 24) return LZK_EINVAL;
         order[i] = i;
     }
@@ -427,7 +459,7 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
         d.n = m.n;
         d.out = m.out;
         d.c = cw[o];
-        d.W = windows_for(d.c);
+        d.W = p->glv ? windows_glv(d.c) : windows_for(d.c);
         d.nb = 1u << (d.c - 1);
         d.pts_off = p->total_pts;
         d.bucket_base = p->total_buckets;
@@ -440,7 +472,7 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
         p->total_pts += m.n;
         p->total_buckets += (uint64_t)d.hw * d.nb;
         p->total_windows += d.hw;
-        p->max_entries += m.n * (uint64_t)d.W;
+        p->max_entries += m.n * (uint64_t)d.W * (p->glv ? 2 : 1);
         if (p->wgroups.empty() || p->wgroups.back().c != d.c) p->wgroups.push_back({d.c, d.bucket_base, 0, 0, 0, 0});
         p->wgroups.back().windows += d.hw;
         p->wgroups.back().largest = std::max<size_t>(p->wgroups.back().largest, m.n);
@@ -456,8 +488,9 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
     p->chunk = tune_chunk(p->group, largest, p->fixed);
     p->run = tune_run(p->group, largest, p->fixed);
     // each width group reduces with the run of its own largest MSM's size class
-    for (auto& g : p->wgroups) g.run = tune_run(p->group, g.largest, p->fixed);
-    if (!p->persistent && with_rounds) p->rounds = affine_rounds(p->max_entries, std::max<uint64_t>(p->total_buckets, 1));
+    // (4 buckets a lane at least: shorter runs pay only where lanes are idle)
+    for (auto& g : p->wgroups) g.run = std::max(tune_run(p->group, g.largest, p->fixed), kDefaultRun);
+    if (!p->persistent && with_rounds) p->rounds = affine_rounds(p->max_entries, std::max<uint64_t>(p->total_buckets, 1), kAffFillPlain);
     p->max_slots = p->max_entries + p->total_buckets * ((1u << p->rounds) - 1);
     p->slice = p->max_slots < kAffSlice ? align_up(p->max_slots, size_t(1) << p->rounds) : kAffSlice;
     p->chunk = acc_chunk(p->chunk, p->rounds);
@@ -479,7 +512,7 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
     size_t o_large = cv.take<uint32_t>(p->chunks / kFixSmall + 2);
     size_t o_bar = cv.take<uint32_t>(2);
     size_t o_ent = cv.take<uint32_t>(std::max<uint64_t>(p->max_slots, 1));
-    size_t o_bases = cv.take<Aff<F>>(p->fixed ? 1 : std::max<uint64_t>(p->total_pts, 1));
+    size_t o_bases = cv.take<Aff<F>>(p->fixed ? 1 : std::max<uint64_t>(p->total_pts, 1) * (p->glv ? 2 : 1));
     size_t o_bsum = cv.take<X>(B);
     size_t o_head = cv.take<X>(std::max<uint64_t>(p->chunks, 1)), o_tail = cv.take<X>(std::max<uint64_t>(p->chunks, 1));
     size_t o_lr0 = cv.take<X>(std::max<uint64_t>(p->lvl, 1)), o_lr1 = cv.take<X>(std::max<uint64_t>(p->lvl, 1));
@@ -577,7 +610,7 @@ int lzk_batch_plan_create_ex(int group, const lzk_msm_desc* msms, size_t n_msm, 
         rc = group == 2 ? create_plan<Fq2>(msms, n_msm, ntts, n_ntt, p, rounds)
                         : create_plan<Fq>(msms, n_msm, ntts, n_ntt, p, rounds);
         if (rc == LZK_OK) break;
-        const bool again = rc == LZK_ENOMEM && p->rounds;
+        const bool again = rc == LZK_ENOMEM && (p->rounds || p->glv);
         destroy_plan(p);
         if (!again) return rc;
     }

@@ -16,6 +16,7 @@
 // add-2008-s, dbl-2008-s-1); results are compared with the reference only
 // after normalisation to affine, which is representation independent.
 #pragma once
+#include "common.cuh"
 #include "field52.cuh"
 
 namespace lzk {
@@ -149,10 +150,104 @@ __device__ __forceinline__ void csqr2(Fq2& r0, Fq2& r1, const Fq2& a, const Fq2&
     r1 = cmul(b, b);
 }
 
+// ---------------- Fq2 over two lanes ----------------
+// The coordinate of an Fq2 element that this lane holds: an even lane c0, the
+// odd lane beside it c1.  The two lanes run the same code in step (every
+// branch is on values of both) and exchange operands by shuffles.  A product
+// is one sum of two Fq products a lane, and a point takes half the registers,
+// so the point formulas run without spills at half the latency; all lanes
+// together issue about a quarter more than with whole elements.  For the
+// kernels bound by the length of their chains (fix-up, bucket reduction, and
+// the accumulation).
+struct Fq2P {
+    Fq c;
+    __device__ __forceinline__ static bool odd() { return threadIdx.x & 1; }
+    __device__ __forceinline__ static uint32_t mask() { return 3u << (threadIdx.x & 30); }
+    __device__ __forceinline__ static Fq2P zero() { return {Fq::zero()}; }
+    __device__ __forceinline__ static Fq2P one()
+    {
+        Fq2P r{Fq::one()};
+        if (odd()) r.c = Fq::zero();
+        return r;
+    }
+    __device__ __forceinline__ bool is_zero() const { return __all_sync(mask(), c.is_zero()); }
+    __device__ __forceinline__ bool operator==(const Fq2P& o) const { return __all_sync(mask(), c == o.c); }
+};
+__device__ __forceinline__ Fq pair_swap(const Fq& x)
+{
+    Fq r;
+    _Pragma("unroll") for (int i = 0; i < 8; i++) r.v[i] = __shfl_xor_sync(Fq2P::mask(), x.v[i], 1);
+    return r;
+}
+__device__ __forceinline__ Fq2P add(const Fq2P& a, const Fq2P& b) { return {add(a.c, b.c)}; }
+__device__ __forceinline__ Fq2P sub(const Fq2P& a, const Fq2P& b) { return {sub(a.c, b.c)}; }
+__device__ __forceinline__ Fq2P neg(const Fq2P& a) { return {neg(a.c)}; }
+__device__ __forceinline__ Fq2P dbl(const Fq2P& a) { return {dbl(a.c)}; }
+__device__ __forceinline__ Fq neg_operand(const Fq& x);
+// even: a0 b0 + a1 (-b1); odd (own a1, b1): a1 b0 + a0 b1
+static __device__ __noinline__ Fq2P fq2p_mul_call(const Fq2P a, const Fq2P b)
+{
+    const Fq ao = pair_swap(a.c), bo = pair_swap(b.c), n = neg_operand(bo);
+    Fq x, y;
+    _Pragma("unroll") for (int i = 0; i < 8; i++) {
+        x.v[i] = Fq2P::odd() ? bo.v[i] : b.c.v[i];
+        y.v[i] = Fq2P::odd() ? b.c.v[i] : n.v[i];
+    }
+    return {dot52_call<FqP>(a.c, x, ao, y)};
+}
+// even: (a0 + a1)(a0 - a1); odd: 2 a1 a0
+static __device__ __noinline__ Fq2P fq2p_sqr_call(const Fq2P a)
+{
+    const Fq o = pair_swap(a.c);
+    const Fq s = add(a.c, Fq2P::odd() ? a.c : o), d = sub(a.c, o);
+    Fq y;
+    _Pragma("unroll") for (int i = 0; i < 8; i++) y.v[i] = Fq2P::odd() ? o.v[i] : d.v[i];
+    return {mul52(s, y)};
+}
+__device__ __forceinline__ Fq2P cmul(const Fq2P& a, const Fq2P& b) { return fq2p_mul_call(a, b); }
+__device__ __forceinline__ Fq2P csqr(const Fq2P& a) { return fq2p_sqr_call(a); }
+__device__ __forceinline__ void cmul2(Fq2P& r0, Fq2P& r1, const Fq2P& a0, const Fq2P& b0, const Fq2P& a1, const Fq2P& b1)
+{
+    r0 = cmul(a0, b0);
+    r1 = cmul(a1, b1);
+}
+__device__ __forceinline__ void csqr2(Fq2P& r0, Fq2P& r1, const Fq2P& a, const Fq2P& b)
+{
+    r0 = csqr(a);
+    r1 = csqr(b);
+}
+
 // ---------------- point forms ----------------
 template <class F> struct Aff { F x, y; };
 template <class F> struct XYZZ { F X, Y, ZZ, ZZZ; };
 template <class F> struct Jac { F X, Y, Z; };
+
+// The element type in memory of a coordinate type, the lanes a point takes,
+// and whole points read and written by those lanes.
+template <class F> struct MemOf { using T = F; static constexpr uint32_t lanes = 1; };
+template <> struct MemOf<Fq2P> { using T = Fq2; static constexpr uint32_t lanes = 2; };
+template <class F> using XYZZm = XYZZ<typename MemOf<F>::T>;
+template <class F> __device__ __forceinline__ XYZZ<F> ld_pt(const XYZZm<F>* p)
+{
+    if constexpr (MemOf<F>::lanes == 2) {
+        const Fq* q = reinterpret_cast<const Fq*>(p) + (threadIdx.x & 1);
+        return {{ld_elem(q)}, {ld_elem(q + 2)}, {ld_elem(q + 4)}, {ld_elem(q + 6)}};
+    } else {
+        return ld_elem(p);
+    }
+}
+template <class F> __device__ __forceinline__ void st_pt(XYZZm<F>* p, const XYZZ<F>& v)
+{
+    if constexpr (MemOf<F>::lanes == 2) {
+        Fq* q = reinterpret_cast<Fq*>(p) + (threadIdx.x & 1);
+        st_elem(q, v.X.c);
+        st_elem(q + 2, v.Y.c);
+        st_elem(q + 4, v.ZZ.c);
+        st_elem(q + 6, v.ZZZ.c);
+    } else {
+        st_elem(p, v);
+    }
+}
 
 template <class F> __device__ __forceinline__ bool aff_is_inf(const Aff<F>& p) { return p.x.is_zero() && p.y.is_zero(); }
 
@@ -337,6 +432,36 @@ __device__ __forceinline__ void warp_products(F (&r)[N], const F (&a)[N], const 
     }
     F z = cmul(x, y);
     _Pragma("unroll") for (int k = 0; k < N; k++) r[k] = shfl_elem(z, k);
+}
+
+// p - x for canonical x (p for zero): a negated product operand
+__device__ __forceinline__ Fq neg_operand(const Fq& x)
+{
+    Fq p;
+    _Pragma("unroll") for (int i = 0; i < 8; i++) p.v[i] = FqP::p(i);
+    uint32_t b = 0;
+    _Pragma("unroll") for (int i = 0; i < 8; i++) {
+        const uint64_t d = (uint64_t)p.v[i] - x.v[i] - b;
+        p.v[i] = (uint32_t)d;
+        b = (uint32_t)(d >> 63);
+    }
+    return p;
+}
+// Fq2 products: two lanes each, one for either coordinate (a0 b0 - a1 b1, a0
+// b1 + a1 b0, each one sum of two products), which takes 0.6 of the time of
+// the whole product on one lane.
+template <int N>
+__device__ __forceinline__ void warp_products(Fq2 (&r)[N], const Fq2 (&a)[N], const Fq2 (&b)[N])
+{
+    const int lane = threadIdx.x & 31, k0 = lane >> 1;
+    Fq2 x = a[0], y = b[0];
+    _Pragma("unroll") for (int k = 1; k < N; k++) {
+        if (k0 == k) { x = a[k]; y = b[k]; }
+    }
+    const Fq n = neg_operand(y.c1);
+    const bool odd = lane & 1;
+    const Fq z = dot52_call<FqP>(x.c0, odd ? y.c1 : y.c0, x.c1, odd ? y.c0 : n);
+    _Pragma("unroll") for (int k = 0; k < N; k++) r[k] = {shfl_elem(z, 2 * k), shfl_elem(z, 2 * k + 1)};
 }
 
 template <class F> __device__ __noinline__ XYZZ<F> xyzz_dbl_warp(const XYZZ<F> p)

@@ -404,6 +404,28 @@ __device__ __forceinline__ Fp<P> sqr52(const Fp<P>& a)
     return final_sub<P>(t);
 }
 
+// a0 b0 + a1 b1 over 2^256 mod p, canonical, for operands <= p: two products
+// into the same columns and one reduction.
+template <class P>
+__device__ __noinline__ Fp<P> dot52_call(const Fp<P> a0, const Fp<P> b0, const Fp<P> a1, const Fp<P> b1)
+{
+    uint64_t c[10], r[5];
+    _Pragma("unroll") for (int k = 0; k < 10; k++) c[k] = 0 - 2 * prod_bias52(k);
+    {
+        double da[5], db[5];
+        to_d52<4>(da, a0.v);
+        to_d52<0>(db, b0.v);
+        prod_cols52(c, da, db);
+        to_d52<4>(da, a1.v);
+        to_d52<0>(db, b1.v);
+        prod_cols52(c, da, db);
+    }
+    redc52<P>(r, c);
+    uint32_t t[8];
+    from_limbs52(t, r);
+    return final_sub<P>(t);
+}
+
 // Out-of-line bodies for the curve formulas (one product, two independent
 // products interleaved, or two squares), as mul_call / mul2_call in
 // field.cuh.

@@ -8,6 +8,10 @@
 
 namespace lzk {
 
+// G2 points over two lanes (curve.cuh)
+template <class F> struct LaneOf { using T = F; };
+template <> struct LaneOf<Fq2> { using T = Fq2P; };
+
 struct G1 { using F = Fq; };
 struct G2 { using F = Fq2; };
 
@@ -28,17 +32,20 @@ constexpr int kInvGroup = 4;           // products an inverting thread takes
 // proof at 2^20 takes 21.0 ms with 2^24, 22.2 with 2^23 (G1) and 2^22 (G2).
 constexpr size_t kAffSlice = size_t(1) << 24;
 // Rounds R for `entries` sorted entries over B buckets: as long as a bucket
-// still holds kAffFill 2^R entries on average, so that the gaps that pad
-// buckets to multiples of 2^R stay below a tenth of the slots.  At 2^20 over a
-// table (240 entries a bucket) R = 1 .. 4 measured 3480, 3279, 3204, 3207 us,
-// against 3641 us without rounds.  Short lists run at the latency of the
-// rounds' launches, which is more than the additions they save.
-constexpr size_t kAffMinEntries = 1u << 16, kAffFill = 8;
-inline uint32_t affine_rounds(size_t entries, size_t B)
+// still holds fill 2^R entries on average.  Gaps that pad buckets to multiples
+// of 2^R then stay below a tenth (fill 8, one bucket set for all windows) or a
+// fifth of the slots (fill 4, a set per window: buckets are shorter there, and
+// a G2 MSM of 250000 plain points takes 4919 instead of 5529 us; a G1 table
+// MSM of 66000 points 632 instead of 595).  At 2^20 over a table (240 entries
+// a bucket) R = 1 .. 4 measured 3480, 3279, 3204, 3207 us, against 3641 us
+// without rounds.  Lists shorter than kAffMinEntries run at the latency of the
+// rounds' launches.
+constexpr size_t kAffMinEntries = 1u << 16, kAffFillTable = 8, kAffFillPlain = 4;
+inline uint32_t affine_rounds(size_t entries, size_t B, size_t fill)
 {
     uint32_t R = 0;
     if (entries < kAffMinEntries) return 0;
-    while (R < kAffMaxRounds && entries >= (B << (R + 1)) * kAffFill) R++;
+    while (R < kAffMaxRounds && entries >= (B << (R + 1)) * fill) R++;
     // slot numbers are 32 bits
     return entries + (B << R) < (1ull << 32) ? R : 0;
 }
@@ -189,7 +196,7 @@ int msm_g1_form(const Fr* scalars, const void* bases, size_t n, Jac<Fq>* out, co
 // n, window width and table level stride as the sort.
 // Rounds: those of a table MSM of n points (or 0), the same for the sort and
 // its consumers, since the sort pads the buckets.
-inline uint32_t table_rounds(size_t n, uint32_t c) { return affine_rounds(n * (size_t)windows_for(c), size_t(1) << (c - 1)); }
+inline uint32_t table_rounds(size_t n, uint32_t c) { return affine_rounds(n * (size_t)windows_for(c), size_t(1) << (c - 1), kAffFillTable); }
 struct SortWords { size_t cnt, off, ent, bsums; };
 SortWords msm_sort_words(size_t n, uint32_t c, size_t stride, uint32_t rounds);
 // scratch of a table MSM over a shared sort
@@ -234,6 +241,48 @@ int affine_sum(const void* bases, const uint32_t* ent, const uint32_t* total, si
         }
     }
     return LZK_OK;
+}
+
+// bits [lo, lo+c) of an integer of NW limbs
+template <int NW>
+__device__ __forceinline__ uint32_t window_bits(const uint32_t* s, uint32_t lo, uint32_t c)
+{
+    const uint32_t w = lo >> 5, sh = lo & 31;
+    if (w >= NW) return 0;
+    const uint64_t v = ((uint64_t)s[w] | ((uint64_t)(w + 1 < NW ? s[w + 1] : 0u) << 32)) >> sh;
+    return (uint32_t)v & ((1u << c) - 1u);
+}
+
+// Signed-digit recoding of a magnitude: raw = bits + carry in [0, 2^c]; raw >
+// 2^(c-1) is used as raw - 2^c with a carry into the next window, so that
+// |digit| <= 2^(c-1).  f(w, |digit|, negative) for every non-zero digit.
+template <int NW, class Fn>
+__device__ __forceinline__ void for_digits(const uint32_t* s, uint32_t c, uint32_t W, bool neg, Fn f)
+{
+    uint32_t carry = 0;
+    const uint32_t half = 1u << (c - 1);
+    for (uint32_t w = 0; w < W; w++) {
+        const uint32_t raw = window_bits<NW>(s, w * c, c) + carry;
+        carry = raw > half ? 1u : 0u;
+        const uint32_t d = carry ? (1u << c) - raw : raw;
+        if (d) f(w, d, neg != (carry != 0));
+    }
+}
+// The digits of a scalar: of itself (h = 0), or (GLV) of its two halves, f(h,
+// w, |digit|, negative).
+template <bool GLV, class Fn>
+__device__ __forceinline__ void scalar_digits(const Fr* sc, uint32_t c, uint32_t W, Fn f)
+{
+    const Fr k = from_mont(ldg_elem(sc));
+    if (GLV) {
+        uint32_t k1[4], k2[4];
+        bool n1, n2;
+        glv_split(k.v, k1, n1, k2, n2);
+        for_digits<4>(k1, c, W, n1, [&](uint32_t w, uint32_t d, bool neg) { f(0u, w, d, neg); });
+        for_digits<4>(k2, c, W, n2, [&](uint32_t w, uint32_t d, bool neg) { f(1u, w, d, neg); });
+    } else {
+        for_digits<8>(k.v, c, W, false, [&](uint32_t w, uint32_t d, bool neg) { f(0u, w, d, neg); });
+    }
 }
 
 // largest b in [lo, B) with off[b] >> shift <= e
@@ -304,6 +353,28 @@ __device__ __forceinline__ Aff<Fq2> load_raw<Fq2, kLayoutPoints>(const void* bas
     return is_marker(a.x) ? Aff<Fq2>{Fq2::zero(), Fq2::zero()} : a;
 }
 
+// the coordinates of a G2 base that this lane holds (MemOf<Fq2P>)
+template <>
+__device__ __forceinline__ Aff<Fq2P> load_raw<Fq2P, LZK_BASES_AFFINE>(const void* bases, uint32_t idx)
+{
+    const Fq* q = reinterpret_cast<const Fq*>(reinterpret_cast<const Aff<Fq2>*>(bases) + idx) + (threadIdx.x & 1);
+    return {{ldg_elem(q)}, {ldg_elem(q + 2)}};
+}
+template <>
+__device__ __forceinline__ Aff<Fq2P> load_raw<Fq2P, kLayoutPoints>(const void* bases, uint32_t idx)
+{
+    Aff<Fq2P> a = load_raw<Fq2P, LZK_BASES_AFFINE>(bases, idx);
+    if (__shfl_sync(Fq2P::mask(), a.x.c.v[7], threadIdx.x & 30) == 0xffffffffu) a = {Fq2P::zero(), Fq2P::zero()};
+    return a;
+}
+template <>
+__device__ __forceinline__ Aff<Fq2P> load_raw<Fq2P, LZK_BASES_REF_G2_LANES>(const void* bases, uint32_t idx)
+{
+    const Jac<Fq> h = ldg_elem(reinterpret_cast<const Jac<Fq>*>(bases) + 2 * (size_t)idx + (threadIdx.x & 1));
+    if (Fq2P{h.Z}.is_zero()) return {Fq2P::zero(), Fq2P::zero()};
+    return {{h.X}, {h.Y}};
+}
+
 template <class F, int LAYOUT>
 __device__ __forceinline__ Aff<F> load_base(const void* bases, uint32_t v)
 {
@@ -319,8 +390,8 @@ template <class F, int LAYOUT>
 __device__ __forceinline__ void accumulate_chunk(uint64_t t, const void* __restrict__ bases,
                                                  const uint32_t* __restrict__ ent, const uint32_t* __restrict__ off,
                                                  uint32_t B, size_t chunks, uint32_t chunk, uint32_t shift,
-                                                 uint64_t nbases, XYZZ<F>* __restrict__ bsum,
-                                                 XYZZ<F>* __restrict__ head, XYZZ<F>* __restrict__ tail)
+                                                 uint64_t nbases, XYZZm<F>* __restrict__ bsum,
+                                                 XYZZm<F>* __restrict__ head, XYZZm<F>* __restrict__ tail)
 {
     (void)nbases;   // the base records behind the entries (debug checks)
     if (t >= chunks) return;
@@ -334,7 +405,7 @@ __device__ __forceinline__ void accumulate_chunk(uint64_t t, const void* __restr
     for (uint32_t e = cs; e < ce; e++) {
         if (e == bend) {
             // bucket b finished inside this chunk
-            if (bbeg < cs) st_elem(head + t, acc); else st_elem(bsum + b, acc);
+            if (bbeg < cs) st_pt<F>(head + t, acc); else st_pt<F>(bsum + b, acc);
             // almost always the next bucket (at the prover's width a bucket
             // holds about 240 entries): one offset load instead of a binary
             // search of 16 dependent loads, which measured 0.9 % (G1) and
@@ -355,9 +426,9 @@ __device__ __forceinline__ void accumulate_chunk(uint64_t t, const void* __restr
         acc = xyzz_madd(acc, load_base<F, LAYOUT>(bases, v));
     }
     bool began_before = bbeg < cs, cont_after = bend > ce;
-    if (began_before) st_elem(head + t, acc);
-    else if (cont_after) st_elem(tail + t, acc);
-    else st_elem(bsum + b, acc);
+    if (began_before) st_pt<F>(head + t, acc);
+    else if (cont_after) st_pt<F>(tail + t, acc);
+    else st_pt<F>(bsum + b, acc);
 }
 // 128-thread blocks; at most 168 registers for G1 (3 blocks = 12 warps per
 // SM) and 255 for G2 (2 blocks).  With the products on the FP64 pipe the
@@ -368,36 +439,36 @@ template <class F, int LAYOUT>
 __global__ void __launch_bounds__(128, sizeof(F) == 32 ? 3 : 2) k_accumulate(const void* __restrict__ bases, const uint32_t* __restrict__ ent,
                                                     const uint32_t* __restrict__ off, uint32_t B, size_t chunks,
                                                     uint32_t chunk, uint32_t shift, uint64_t nbases,
-                                                    XYZZ<F>* __restrict__ bsum, XYZZ<F>* __restrict__ head,
-                                                    XYZZ<F>* __restrict__ tail)
+                                                    XYZZm<F>* __restrict__ bsum, XYZZm<F>* __restrict__ head,
+                                                    XYZZm<F>* __restrict__ tail)
 {
-    accumulate_chunk<F, LAYOUT>(gtid(), bases, ent, off, B, chunks, chunk, shift, nbases, bsum, head, tail);
+    accumulate_chunk<F, LAYOUT>(gtid() / MemOf<F>::lanes, bases, ent, off, B, chunks, chunk, shift, nbases, bsum, head, tail);
 }
 
 template <class F>
 __device__ __forceinline__ void fixup_items(const uint32_t* __restrict__ off, uint32_t B, uint32_t chunk, uint32_t shift,
-                        uint64_t chunks, XYZZ<F>* __restrict__ bsum, const XYZZ<F>* __restrict__ head, const XYZZ<F>* __restrict__ tail,
+                        uint64_t chunks, XYZZm<F>* __restrict__ bsum, const XYZZm<F>* __restrict__ head, const XYZZm<F>* __restrict__ tail,
                         uint32_t* __restrict__ large)
 {
     (void)chunks;
-    for (uint64_t b = gtid(); b < B; b += gstride()) {
+    for (uint64_t b = gtid() / MemOf<F>::lanes; b < B; b += gstride() / MemOf<F>::lanes) {
         uint32_t s = off[b] >> shift, e = off[b + 1] >> shift;
         if (s == e) continue;
         uint32_t c0 = s / chunk, c1 = (e - 1) / chunk;
         if (!LZK_CHECK(c1 < chunks, 4)) continue;
         if (c0 == c1) continue;
         if (c1 - c0 > kFixSmall) {
-            large[1 + atomicAdd(large, 1u)] = (uint32_t)b;
+            if (MemOf<F>::lanes == 1 || !(threadIdx.x & 1)) large[1 + atomicAdd(large, 1u)] = (uint32_t)b;
             continue;
         }
-        XYZZ<F> acc = ld_elem(tail + c0);
-        for (uint32_t c = c0 + 1; c <= c1; c++) acc = xyzz_add_cold(acc, ld_elem(head + c));
-        st_elem(bsum + b, acc);
+        XYZZ<F> acc = ld_pt<F>(tail + c0);
+        for (uint32_t c = c0 + 1; c <= c1; c++) acc = xyzz_add_cold(acc, ld_pt<F>(head + c));
+        st_pt<F>(bsum + b, acc);
     }
 }
 template <class F>
 __global__ void k_fixup(const uint32_t* __restrict__ off, uint32_t B, uint32_t chunk, uint32_t shift, uint64_t chunks,
-                        XYZZ<F>* __restrict__ bsum, const XYZZ<F>* __restrict__ head, const XYZZ<F>* __restrict__ tail,
+                        XYZZm<F>* __restrict__ bsum, const XYZZm<F>* __restrict__ head, const XYZZm<F>* __restrict__ tail,
                         uint32_t* __restrict__ large)
 {
     fixup_items<F>(off, B, chunk, shift, chunks, bsum, head, tail, large);
@@ -405,39 +476,39 @@ __global__ void k_fixup(const uint32_t* __restrict__ off, uint32_t B, uint32_t c
 
 // One block per listed bucket: strided partial sums, then a tree in shared
 // memory.  Partial q of bucket b is tail[c0] (q = 0) or head[c0 + q].
-// (blockDim.x points of shared memory at sm; the persistent batch kernel
+// (a point of shared memory for every point's lanes of the block at sm; the persistent batch kernel
 // runs it too)
 template <class F>
 __device__ __forceinline__ void fixup_large_items(const uint32_t* __restrict__ off, uint32_t chunk, uint32_t shift,
-                                                  XYZZ<F>* __restrict__ bsum, const XYZZ<F>* __restrict__ head,
-                                                  const XYZZ<F>* __restrict__ tail, const uint32_t* __restrict__ large,
-                                                  XYZZ<F>* sm)
+                                                  XYZZm<F>* __restrict__ bsum, const XYZZm<F>* __restrict__ head,
+                                                  const XYZZm<F>* __restrict__ tail, const uint32_t* __restrict__ large,
+                                                  XYZZm<F>* sm)
 {
-    uint32_t nl = large[0];
+    const uint32_t nl = large[0], me = threadIdx.x / MemOf<F>::lanes, all = blockDim.x / MemOf<F>::lanes;
     for (uint32_t idx = blockIdx.x; idx < nl; idx += gridDim.x) {
         uint32_t b = large[1 + idx];
         uint32_t c0 = (off[b] >> shift) / chunk, c1 = ((off[b + 1] >> shift) - 1) / chunk;
         uint32_t np = c1 - c0 + 1;
         XYZZ<F> acc = xyzz_inf<F>();
-        for (uint32_t q = threadIdx.x; q < np; q += blockDim.x)
-            acc = xyzz_add_cold(acc, ld_elem(q ? head + c0 + q : tail + c0));
-        st_elem(sm + threadIdx.x, acc);
+        for (uint32_t q = me; q < np; q += all)
+            acc = xyzz_add_cold(acc, ld_pt<F>(q ? head + c0 + q : tail + c0));
+        st_pt<F>(sm + me, acc);
         __syncthreads();
-        for (uint32_t h = blockDim.x / 2; h > 0; h >>= 1) {
-            if (threadIdx.x < h) st_elem(sm + threadIdx.x, xyzz_add_cold(ld_elem(sm + threadIdx.x), ld_elem(sm + threadIdx.x + h)));
+        for (uint32_t h = all / 2; h > 0; h >>= 1) {
+            if (me < h) st_pt<F>(sm + me, xyzz_add_cold(ld_pt<F>(sm + me), ld_pt<F>(sm + me + h)));
             __syncthreads();
         }
-        if (threadIdx.x == 0) st_elem(bsum + b, ld_elem(sm));
+        if (me == 0) st_pt<F>(bsum + b, ld_pt<F>(sm));
         __syncthreads();
     }
 }
 template <class F>
-__global__ void k_fixup_large(const uint32_t* __restrict__ off, uint32_t chunk, uint32_t shift, XYZZ<F>* __restrict__ bsum,
-                              const XYZZ<F>* __restrict__ head, const XYZZ<F>* __restrict__ tail,
+__global__ void k_fixup_large(const uint32_t* __restrict__ off, uint32_t chunk, uint32_t shift, XYZZm<F>* __restrict__ bsum,
+                              const XYZZm<F>* __restrict__ head, const XYZZm<F>* __restrict__ tail,
                               const uint32_t* __restrict__ large)
 {
     extern __shared__ uint4 fx_raw[];
-    fixup_large_items<F>(off, chunk, shift, bsum, head, tail, large, reinterpret_cast<XYZZ<F>*>(fx_raw));
+    fixup_large_items<F>(off, chunk, shift, bsum, head, tail, large, reinterpret_cast<XYZZm<F>*>(fx_raw));
 }
 
 // Warp shuffles of whole points
@@ -447,7 +518,7 @@ __device__ __forceinline__ XYZZ<F> shfl_down_pt(const XYZZ<F>& x, uint32_t d)
     XYZZ<F> r;
     const uint32_t* s = reinterpret_cast<const uint32_t*>(&x);
     uint32_t* o = reinterpret_cast<uint32_t*>(&r);
-    _Pragma("unroll") for (int i = 0; i < (int)(sizeof(XYZZ<F>) / 4); i++) o[i] = __shfl_down_sync(0xffffffffu, s[i], d);
+    _Pragma("unroll") for (int i = 0; i < (int)(sizeof(XYZZ<F>) / 4); i++) o[i] = __shfl_down_sync(0xffffffffu, s[i], d * MemOf<F>::lanes);
     return r;
 }
 template <class F>
@@ -456,7 +527,7 @@ __device__ __forceinline__ XYZZ<F> shfl_xor_pt(const XYZZ<F>& x, uint32_t m)
     XYZZ<F> r;
     const uint32_t* s = reinterpret_cast<const uint32_t*>(&x);
     uint32_t* o = reinterpret_cast<uint32_t*>(&r);
-    _Pragma("unroll") for (int i = 0; i < (int)(sizeof(XYZZ<F>) / 4); i++) o[i] = __shfl_xor_sync(0xffffffffu, s[i], m);
+    _Pragma("unroll") for (int i = 0; i < (int)(sizeof(XYZZ<F>) / 4); i++) o[i] = __shfl_xor_sync(0xffffffffu, s[i], m * MemOf<F>::lanes);
     return r;
 }
 template <class F>
@@ -467,6 +538,18 @@ __device__ __forceinline__ XYZZ<F> shfl_pt(const XYZZ<F>& x, uint32_t lane)
     uint32_t* o = reinterpret_cast<uint32_t*>(&r);
     _Pragma("unroll") for (int i = 0; i < (int)(sizeof(XYZZ<F>) / 4); i++) o[i] = __shfl_sync(0xffffffffu, s[i], lane);
     return r;
+}
+
+// the warp's first point, whole, in every lane
+template <class F>
+__device__ __forceinline__ XYZZm<F> whole_pt(const XYZZ<F>& x)
+{
+    if constexpr (MemOf<F>::lanes == 2) {
+        return {{shfl_elem(x.X.c, 0), shfl_elem(x.X.c, 1)}, {shfl_elem(x.Y.c, 0), shfl_elem(x.Y.c, 1)},
+                {shfl_elem(x.ZZ.c, 0), shfl_elem(x.ZZ.c, 1)}, {shfl_elem(x.ZZZ.c, 0), shfl_elem(x.ZZZ.c, 1)}};
+    } else {
+        return shfl_pt(x, 0);
+    }
 }
 
 // ---------------------------- bucket reduction ----------------------------
@@ -505,17 +588,21 @@ struct RedShape {
 };
 // run: requested buckets per lane run (a power of two); a set too small
 // for 32 lanes of such runs takes shorter runs, down to single buckets
-inline RedShape red_shape(uint32_t m, uint32_t run = kDefaultRun)
+// lanes: points a warp holds.  16 (two lanes a point) take runs of two at
+// least, so that no set has more tiles than the scratch is sized for.
+inline RedShape red_shape(uint32_t m, uint32_t run, uint32_t lanes)
 {
     RedShape s;
-    s.r = run ? run : 1;
-    while (s.r > 1 && 32 * s.r > m) s.r >>= 1;
-    s.L = m < 32 * s.r ? m : 32 * s.r;
+    const uint32_t least = 32 / lanes;
+    s.r = run > least ? run : least;
+    while (s.r > least && lanes * s.r > m) s.r >>= 1;
+    while (s.r > 1 && s.r > m) s.r >>= 1;
+    s.L = m < lanes * s.r ? m : lanes * s.r;
     s.lgL = 0; while ((1u << s.lgL) < s.L) s.lgL++;
     s.P = m / s.L;
     s.lg = 0; while ((1u << s.lg) < s.P) s.lg++;
-    s.cT = (s.P + 31) / 32;
-    s.cG = (s.P / 2 + 31) / 32;
+    s.cT = (s.P + lanes - 1) / lanes;
+    s.cG = (s.P / 2 + lanes - 1) / lanes;
     s.NP = s.cT + s.lg * s.cG;
     s.NS = 1 + s.lg;
     return s;
@@ -535,9 +622,9 @@ __device__ __forceinline__ uint32_t slice_member(uint32_t v, uint32_t i)
 // end: tiles wb P, slice partials wb NP, sums wb NS, sets wb).
 template <class F>
 struct RedJob {
-    const XYZZ<F>* bsum;
+    const XYZZm<F>* bsum;
     const uint32_t* off;
-    XYZZ<F> *R, *T, *part, *scaled, *win;
+    XYZZm<F> *R, *T, *part, *scaled, *win;
     uint32_t wb, m;
     RedShape sh;
     uint64_t s_tile, s_np, s_ns, s_w;
@@ -561,7 +648,8 @@ __device__ __forceinline__ uint32_t red_job_of(const RedJobs<F>& jobs, uint64_t 
 template <class F>
 __device__ __forceinline__ void red_tile_items(const RedJobs<F>& jobs, uint64_t total)
 {
-    const uint32_t lane = threadIdx.x & 31;
+    constexpr uint32_t LP = MemOf<F>::lanes, NL = 32 / LP;
+    const uint32_t lane = (threadIdx.x & 31) / LP;
     for (uint64_t item = gtid() >> 5; item < total; item += gstride() >> 5) {
         const RedJob<F>& J = jobs.g[red_job_of(jobs, item, &RedJob<F>::s_tile)];
         const uint64_t tile = item - J.s_tile;
@@ -572,7 +660,7 @@ __device__ __forceinline__ void red_tile_items(const RedJobs<F>& jobs, uint64_t 
             const size_t k0 = (size_t)tile * L + (size_t)lane * r;   // = w m + u L + j r
             for (int i = (int)r - 1; i >= 0; i--) {
                 size_t k = k0 + (uint32_t)i;
-                if (J.off[k] != J.off[k + 1]) s = xyzz_add_cold(s, ld_elem(J.bsum + k));
+                if (J.off[k] != J.off[k + 1]) s = xyzz_add_cold(s, ld_pt<F>(J.bsum + k));
                 t = xyzz_add_cold(t, s);
             }
         }
@@ -586,8 +674,8 @@ __device__ __forceinline__ void red_tile_items(const RedJobs<F>& jobs, uint64_t 
         XYZZ<F> V = xyzz_add_cold(t, U);
         for (uint32_t d = nl >> 1; d > 0; d >>= 1) V = xyzz_add_cold(V, shfl_xor_pt(V, d));
         if (lane == 0) {
-            st_elem(J.R + tile, S);
-            st_elem(J.T + tile, V);
+            st_pt<F>(J.R + tile, S);
+            st_pt<F>(J.T + tile, V);
         }
     }
 }
@@ -601,7 +689,8 @@ __global__ void __launch_bounds__(128) k_red_tile(const __grid_constant__ RedJob
 template <class F>
 __device__ __forceinline__ void red_slices_items(const RedJobs<F>& jobs, uint64_t total)
 {
-    const uint32_t lane = threadIdx.x & 31;
+    constexpr uint32_t LP = MemOf<F>::lanes, NL = 32 / LP;
+    const uint32_t lane = (threadIdx.x & 31) / LP;
     for (uint64_t item = gtid() >> 5; item < total; item += gstride() >> 5) {
         const RedJob<F>& J = jobs.g[red_job_of(jobs, item, &RedJob<F>::s_np)];
         const RedShape& sh = J.sh;
@@ -610,14 +699,14 @@ __device__ __forceinline__ void red_slices_items(const RedJobs<F>& jobs, uint64_
         const size_t base = (size_t)w * sh.P;
         XYZZ<F> x = xyzz_inf<F>();
         if (q < sh.cT) {
-            uint32_t v = q * 32 + lane;
-            if (v < sh.P) x = ld_elem(J.T + base + v);
+            uint32_t v = q * NL + lane;
+            if (v < sh.P) x = ld_pt<F>(J.T + base + v);
         } else {
-            uint32_t i = (q - sh.cT) / sh.cG, v = ((q - sh.cT) % sh.cG) * 32 + lane;
-            if (v < sh.P / 2) x = ld_elem(J.R + base + slice_member(v, i));
+            uint32_t i = (q - sh.cT) / sh.cG, v = ((q - sh.cT) % sh.cG) * NL + lane;
+            if (v < sh.P / 2) x = ld_pt<F>(J.R + base + slice_member(v, i));
         }
-        for (uint32_t d = 16; d > 0; d >>= 1) x = xyzz_add_cold(x, shfl_xor_pt(x, d));
-        if (lane == 0) st_elem(J.part + g, x);
+        for (uint32_t d = NL / 2; d > 0; d >>= 1) x = xyzz_add_cold(x, shfl_xor_pt(x, d));
+        if (lane == 0) st_pt<F>(J.part + g, x);
     }
 }
 template <class F>
@@ -629,24 +718,25 @@ __global__ void __launch_bounds__(128) k_red_slices(const __grid_constant__ RedJ
 template <class F>
 __device__ __forceinline__ void red_scale_items(const RedJobs<F>& jobs, uint64_t total)
 {
-    const uint32_t lane = threadIdx.x & 31;
+    constexpr uint32_t LP = MemOf<F>::lanes, NL = 32 / LP;
+    const uint32_t lane = (threadIdx.x & 31) / LP;
     for (uint64_t item = gtid() >> 5; item < total; item += gstride() >> 5) {
         const RedJob<F>& J = jobs.g[red_job_of(jobs, item, &RedJob<F>::s_ns)];
         const RedShape& sh = J.sh;
         const uint64_t g = item - J.s_ns;
         uint32_t w = (uint32_t)(g / sh.NS), s = (uint32_t)(g % sh.NS);
         uint32_t first = s == 0 ? 0 : sh.cT + (s - 1) * sh.cG, cnt = s == 0 ? sh.cT : sh.cG;
-        const XYZZ<F>* src = J.part + (size_t)w * sh.NP + first;
+        const XYZZm<F>* src = J.part + (size_t)w * sh.NP + first;
         XYZZ<F> x = xyzz_inf<F>();
-        for (uint32_t c = lane; c < cnt; c += 32) x = xyzz_add_cold(x, ld_elem(src + c));
-        for (uint32_t d = 16; d > 0; d >>= 1) x = xyzz_add_cold(x, shfl_xor_pt(x, d));
+        for (uint32_t c = lane; c < cnt; c += NL) x = xyzz_add_cold(x, ld_pt<F>(src + c));
+        for (uint32_t d = NL / 2; d > 0; d >>= 1) x = xyzz_add_cold(x, shfl_xor_pt(x, d));
         // lanes may hold different representations of the sum (an addition
         // with swapped operands negates Y and ZZZ); the warp-uniform
         // doublings need one
-        x = shfl_pt(x, 0);
+        XYZZm<F> y = whole_pt(x);
         uint32_t dbls = s == 0 ? 0 : s - 1 + sh.lgL;
-        for (uint32_t d = 0; d < dbls; d++) x = xyzz_dbl_warp(x);
-        if (lane == 0) st_elem(J.scaled + g, x);
+        for (uint32_t d = 0; d < dbls; d++) y = xyzz_dbl_warp(y);
+        if ((threadIdx.x & 31) == 0) st_elem(J.scaled + g, y);
     }
 }
 template <class F>
@@ -658,14 +748,16 @@ __global__ void __launch_bounds__(128) k_red_scale(const __grid_constant__ RedJo
 template <class F>
 __device__ __forceinline__ void red_combine_items(const RedJobs<F>& jobs, uint64_t total)
 {
-    const uint32_t lane = threadIdx.x & 31;
+    constexpr uint32_t LP = MemOf<F>::lanes, NL = 32 / LP;
+    const uint32_t lane = (threadIdx.x & 31) / LP;
     for (uint64_t item = gtid() >> 5; item < total; item += gstride() >> 5) {
         const RedJob<F>& J = jobs.g[red_job_of(jobs, item, &RedJob<F>::s_w)];
         const uint64_t w = item - J.s_w;
         const uint32_t NS = J.sh.NS;
-        XYZZ<F> x = lane < NS ? ld_elem(J.scaled + w * NS + lane) : xyzz_inf<F>();
-        for (uint32_t d = 16; d > 0; d >>= 1) x = xyzz_add_cold(x, shfl_xor_pt(x, d));
-        if (lane == 0) st_elem(J.win + w, x);
+        XYZZ<F> x = xyzz_inf<F>();
+        for (uint32_t c = lane; c < NS; c += NL) x = xyzz_add_cold(x, ld_pt<F>(J.scaled + w * NS + c));
+        for (uint32_t d = NL / 2; d > 0; d >>= 1) x = xyzz_add_cold(x, shfl_xor_pt(x, d));
+        if (lane == 0) st_pt<F>(J.win + w, x);
     }
 }
 template <class F>
@@ -679,13 +771,13 @@ __global__ void __launch_bounds__(128) k_red_combine(const __grid_constant__ Red
 inline size_t red_scratch_points(uint32_t wb, uint32_t m) { return (size_t)wb * (m > kLevelL ? m / kLevelL : 1); }
 
 template <class F>
-RedJob<F> red_job(const XYZZ<F>* bsum, const uint32_t* off, uint32_t wb, uint32_t m, uint32_t run, XYZZ<F>* R,
-                  XYZZ<F>* T, XYZZ<F>* part, XYZZ<F>* scaled, XYZZ<F>* win)
+RedJob<F> red_job(const XYZZm<F>* bsum, const uint32_t* off, uint32_t wb, uint32_t m, uint32_t run, XYZZm<F>* R,
+                  XYZZm<F>* T, XYZZm<F>* part, XYZZm<F>* scaled, XYZZm<F>* win)
 {
     RedJob<F> j{};
     j.bsum = bsum; j.off = off; j.R = R; j.T = T; j.part = part; j.scaled = scaled; j.win = win;
     j.wb = wb; j.m = m;
-    j.sh = red_shape(m, run);
+    j.sh = red_shape(m, run, 32 / MemOf<F>::lanes);
     return j;
 }
 
@@ -720,8 +812,8 @@ int reduce_jobs(RedJob<F>* jv, size_t n, cudaStream_t st)
 // Scratch: R, T, part, scaled of red_scratch_points(wb, m) points each.  win
 // may alias R.
 template <class F>
-int reduce_buckets(const XYZZ<F>* bsum, const uint32_t* off, uint32_t wb, uint32_t m, XYZZ<F>* R, XYZZ<F>* T,
-                   XYZZ<F>* part, XYZZ<F>* scaled, XYZZ<F>* win, cudaStream_t st, uint32_t run = kDefaultRun)
+int reduce_buckets(const XYZZm<F>* bsum, const uint32_t* off, uint32_t wb, uint32_t m, XYZZm<F>* R, XYZZm<F>* T,
+                   XYZZm<F>* part, XYZZm<F>* scaled, XYZZm<F>* win, cudaStream_t st, uint32_t run = kDefaultRun)
 {
     RedJob<F> j = red_job<F>(bsum, off, wb, m, run, R, T, part, scaled, win);
     return reduce_jobs<F>(&j, 1, st);
@@ -759,7 +851,9 @@ inline uint32_t msm_rounds(int group, size_t n, uint32_t c, bool shared, uint32_
 {
     const bool glv = msm_glv(group, n, shared);
     const size_t W = glv ? windows_glv(c) : windows_for(c);
-    return layout == LZK_BASES_AFFINE || glv ? affine_rounds(n * W * (glv ? 2 : 1), (shared ? 1 : W) << (c - 1)) : 0;
+    return layout == LZK_BASES_AFFINE || glv ? affine_rounds(n * W * (glv ? 2 : 1), (shared ? 1 : W) << (c - 1),
+                                                             shared ? kAffFillTable : kAffFillPlain)
+                                           : 0;
 }
 
 // out[i] = base i, out[n + i] = phi(base i)
@@ -787,6 +881,8 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
     using F = typename Gp::F;
     using X = XYZZ<F>;
     using A = Aff<F>;
+    using K = typename LaneOf<F>::T;   // coordinates in the accumulation and after it
+    constexpr uint32_t LP = MemOf<K>::lanes;
     if (!out || (n && (!scalars || !bases))) return LZK_EINVAL;
     if (n >= (1ull << 31)) return LZK_EINVAL;
     uint32_t flags = cfg ? cfg->flags : 0u;
@@ -855,7 +951,7 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
     }
     void* tr = trace_begin(sizeof(F) == 32 ? "msm_g1_accumulate" : "msm_g2_accumulate", st);
     {
-        unsigned g = grid_for(p.chunks, 128);
+        unsigned g = grid_for(p.chunks * LP, 128);
         // base records the entries may name: the whole table, or the n bases
         const uint64_t nbases = shared ? (uint64_t)cfg->precomp_windows * stride : (uint64_t)n * (p.glv ? 2 : 1);
         constexpr int REF = sizeof(F) == 32 ? (int)LZK_BASES_REF_G1_JAC : (int)LZK_BASES_REF_G2_LANES;
@@ -863,20 +959,20 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
             A* fin = reinterpret_cast<A*>(base + p.o_fin);
             LZK_TRY(affine_sum<F>(bases, ent, off + p.B, p.max_slots, p.slice, p.rounds, nbases,
                                   base + p.o_aff, fin, st));
-            k_accumulate<F, kLayoutPoints><<<g, 128, 0, st>>>(fin, ent, off, p.B, p.chunks, p.chunk, p.rounds, p.max_slots >> p.rounds, bsum, head, tail); note_launch();
+            k_accumulate<K, kLayoutPoints><<<g, 128, 0, st>>>(fin, ent, off, p.B, p.chunks, p.chunk, p.rounds, p.max_slots >> p.rounds, bsum, head, tail); note_launch();
         } else if (layout == LZK_BASES_AFFINE) {
-            k_accumulate<F, LZK_BASES_AFFINE><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, 0, nbases, bsum, head, tail); note_launch();
+            k_accumulate<K, LZK_BASES_AFFINE><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, 0, nbases, bsum, head, tail); note_launch();
         } else {
-            k_accumulate<F, REF><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, 0, nbases, bsum, head, tail); note_launch();
+            k_accumulate<K, REF><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, 0, nbases, bsum, head, tail); note_launch();
         }
     }
     trace_end(tr, st);
     void* tr_fix = trace_begin(sizeof(F) == 32 ? "msm_g1_fixup" : "msm_g2_fixup", st);
     LZK_CUDA(cudaMemsetAsync(large, 0, sizeof(uint32_t), st));
-    k_fixup<F><<<grid_for(p.B, 256, sm_count() * 8), 256, 0, st>>>(off, p.B, p.chunk, p.rounds, p.chunks, bsum, head, tail, large); note_launch();
+    k_fixup<K><<<grid_for((size_t)p.B * LP, 256, sm_count() * 8), 256, 0, st>>>(off, p.B, p.chunk, p.rounds, p.chunks, bsum, head, tail, large); note_launch();
     {
-        constexpr unsigned fx_threads = 32768 / sizeof(X);   // 32 KB of shared memory
-        k_fixup_large<F><<<sm_count() * 2, fx_threads, fx_threads * sizeof(X), st>>>(off, p.chunk, p.rounds, bsum, head, tail, large); note_launch();
+        constexpr unsigned fx_points = 32768 / sizeof(X);   // 32 KB of shared memory
+        k_fixup_large<K><<<sm_count() * 2, fx_points * LP, fx_points * sizeof(X), st>>>(off, p.chunk, p.rounds, bsum, head, tail, large); note_launch();
     }
     trace_end(tr_fix, st);
     LZK_TRY(launch_status());
@@ -884,7 +980,7 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
     // weighted sums per bucket set
     void* tr_red = trace_begin(sizeof(F) == 32 ? "msm_g1_reduce" : "msm_g2_reduce", st);
     X* win = lr[0];
-    LZK_TRY(reduce_buckets<F>(bsum, off, p.wb, p.nb, lr[0], la[0], lr[1], la[1], win, st, p.run));
+    LZK_TRY(reduce_buckets<K>(bsum, off, p.wb, p.nb, lr[0], la[0], lr[1], la[1], win, st, p.run));
     void* tr_fin = trace_begin(sizeof(F) == 32 ? "msm_g1_finish" : "msm_g2_finish", st);
     k_finish<F><<<1, 32, 0, st>>>(win, p.wb, c, out); note_launch();
     trace_end(tr_fin, st);

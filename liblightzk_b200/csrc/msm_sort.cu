@@ -31,48 +31,6 @@
 
 namespace lzk {
 
-// bits [lo, lo+c) of an integer of NW limbs
-template <int NW>
-__device__ __forceinline__ uint32_t window_bits(const uint32_t* s, uint32_t lo, uint32_t c)
-{
-    const uint32_t w = lo >> 5, sh = lo & 31;
-    if (w >= NW) return 0;
-    const uint64_t v = ((uint64_t)s[w] | ((uint64_t)(w + 1 < NW ? s[w + 1] : 0u) << 32)) >> sh;
-    return (uint32_t)v & ((1u << c) - 1u);
-}
-
-// Signed-digit recoding of a magnitude: raw = bits + carry in [0, 2^c]; raw >
-// 2^(c-1) is used as raw - 2^c with a carry into the next window, so that
-// |digit| <= 2^(c-1).  f(w, |digit|, negative) for every non-zero digit.
-template <int NW, class Fn>
-__device__ __forceinline__ void for_digits(const uint32_t* s, uint32_t c, uint32_t W, bool neg, Fn f)
-{
-    uint32_t carry = 0;
-    const uint32_t half = 1u << (c - 1);
-    for (uint32_t w = 0; w < W; w++) {
-        const uint32_t raw = window_bits<NW>(s, w * c, c) + carry;
-        carry = raw > half ? 1u : 0u;
-        const uint32_t d = carry ? (1u << c) - raw : raw;
-        if (d) f(w, d, neg != (carry != 0));
-    }
-}
-// The digits of a scalar: of itself (h = 0), or (GLV) of its two halves, f(h,
-// w, |digit|, negative).
-template <bool GLV, class Fn>
-__device__ __forceinline__ void scalar_digits(const Fr* sc, uint32_t c, uint32_t W, Fn f)
-{
-    const Fr k = from_mont(ldg_elem(sc));
-    if (GLV) {
-        uint32_t k1[4], k2[4];
-        bool n1, n2;
-        glv_split(k.v, k1, n1, k2, n2);
-        for_digits<4>(k1, c, W, n1, [&](uint32_t w, uint32_t d, bool neg) { f(0u, w, d, neg); });
-        for_digits<4>(k2, c, W, n2, [&](uint32_t w, uint32_t d, bool neg) { f(1u, w, d, neg); });
-    } else {
-        for_digits<8>(k.v, c, W, false, [&](uint32_t w, uint32_t d, bool neg) { f(0u, w, d, neg); });
-    }
-}
-
 // Scalar i of an MSM whose scalars are the concatenation of two arrays:
 // lo[0..split) then hi[0..n - split) (one array: split = n, hi unused).
 __device__ __forceinline__ const Fr* scalar_at(const Fr* lo, const Fr* hi, size_t split, uint64_t i)

@@ -100,7 +100,7 @@ static __device__ __noinline__ Fq2 inverse(const Fq2& a)
     return {mul(a.c0, t), neg(mul(a.c1, t))};
 }
 
-// Products used by the point formulas: out-of-line Fq products (mul_call),
+// Products used by the point formulas: out-of-line Fq products (mul52_call),
 // Fq2 products built from them.
 __device__ __forceinline__ Fq cmul(const Fq& a, const Fq& b) { return mul52_call(a, b); }
 __device__ __forceinline__ Fq csqr(const Fq& a) { return mul52_call(a, a); }

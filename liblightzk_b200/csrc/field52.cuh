@@ -342,22 +342,6 @@ __device__ __forceinline__ Fp<P> mul52(const Fp<P>& a, const Fp<P>& b)
     return final_sub<P>(t);
 }
 
-// a * b / 2^256 mod p (canonical) with b given already as radix-2^52
-// doubles (to_d52<0>, as a twiddle table stores it), for any 8-limb a with
-// 16 a b < 85 p^2 (a below 2p with b < p qualifies): the drop-in product
-// without b's conversion.
-template <class P>
-__device__ __forceinline__ Fp<P> mul52_pre(const Fp<P>& a, const double db[5])
-{
-    double da[5];
-    to_d52<4>(da, a.v);
-    uint64_t r[5];
-    mont52_core<P>(r, da, db);
-    uint32_t t[8];
-    from_limbs52(t, r);
-    return final_sub<P>(t);
-}
-
 // a + p - b for canonical a, b: in (0, 2p), not reduced (a product operand).
 // Carry chains: 16 instructions, where the 64-bit C form took 40.
 template <class P>
@@ -427,8 +411,13 @@ __device__ __noinline__ Fp<P> dot52_call(const Fp<P> a0, const Fp<P> b0, const F
 }
 
 // Out-of-line bodies for the curve formulas (one product, two independent
-// products interleaved, or two squares), as mul_call / mul2_call in
-// field.cuh.
+// products interleaved, or two squares): one body shared by every call keeps
+// the hot loops inside the instruction cache, where fully inlined mixed
+// additions (ten products each) would not fit.
+template <class P>
+struct FpPair {
+    Fp<P> a, b;
+};
 template <class P> __device__ __noinline__ Fp<P> mul52_call(const Fp<P> a, const Fp<P> b) { return mul52(a, b); }
 template <class P>
 __device__ __noinline__ FpPair<P> mul52x2_call(const Fp<P> a0, const Fp<P> b0, const Fp<P> a1, const Fp<P> b1)

@@ -2,7 +2,7 @@
 // product shared by the SpMV, the witness solver and the prover.
 #pragma once
 #include "common.cuh"
-#include "field.cuh"
+#include "field52.cuh"
 
 namespace lzk {
 
@@ -33,9 +33,9 @@ __device__ __forceinline__ Fr row_dot(const CsrDev& M, uint64_t i, const Fr* __r
     uint64_t e = (i + 1 < M.rows) ? ld_index(M.rowp, i + 1, M.ib) : M.nnz;
     Fr acc = Fr::zero();
     for (uint64_t j = s; j < e; j++) {
-        Fr v = ldg_elem(M.val + j);
         Fr x = ldg_elem(z + ld_index(M.col, j, M.ib));
-        acc = add(acc, is_mont_one(v) ? x : mul(x, v));
+        Fr v = ldg_elem(M.val + j);
+        acc = add(acc, is_mont_one(v) ? x : mul52(x, v));
     }
     return acc;
 }

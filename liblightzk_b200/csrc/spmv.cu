@@ -13,11 +13,26 @@
 
 namespace lzk {
 
-__global__ void __launch_bounds__(256) k_spmv3(CsrDev m0, CsrDev m1, CsrDev m2, const Fr* __restrict__ z,
-                                                Fr* __restrict__ o0, Fr* __restrict__ o1, Fr* __restrict__ o2)
+struct SpmvArgs {
+    CsrDev m[3];
+    Fr* out[3];
+};
+
+// One thread a row; bound by the gathers of z beside the products, so what
+// counts is warps in flight: four blocks an SM (64 registers).  The three
+// descriptors stay in the parameter space and are indexed there: choosing
+// between three parameters by blockIdx.y copied them to the stack, and every
+// entry's loads then went through local memory.  A z, B z, C z of a circuit
+// of 2^20 rows: 184 us before, 174 without the copies, 161 with the products
+// on the FP64 pipe as well; a matrix product's rows of up to 100 entries
+// 120 -> 109.  Slower: the next entry's operands loaded ahead (177), three
+// blocks an SM (171), and, both tried before the copies were found, an entry
+// a thread with the sums through shared memory (244) and one reduction for
+// all products of a row (205).
+__global__ void __launch_bounds__(256, 4) k_spmv3(const __grid_constant__ SpmvArgs args, const Fr* __restrict__ z)
 {
-    const CsrDev& M = blockIdx.y == 0 ? m0 : (blockIdx.y == 1 ? m1 : m2);
-    Fr* out = blockIdx.y == 0 ? o0 : (blockIdx.y == 1 ? o1 : o2);
+    const CsrDev& M = args.m[blockIdx.y];
+    Fr* out = args.out[blockIdx.y];
     if (!out) return;
     for (uint64_t i = gtid(); i < M.rows; i += gstride()) st_elem(out + i, row_dot(M, i, z));
 }
@@ -40,9 +55,11 @@ int lzk_spmv3(const lzk_csr* A, const lzk_csr* B, const lzk_csr* C, const lzk_fr
     uint64_t rows = a.rows > b.rows ? a.rows : b.rows;
     rows = rows > c.rows ? rows : c.rows;
     if (rows == 0) return LZK_OK;
+    const SpmvArgs args{{a, b, c},
+                        {A ? reinterpret_cast<Fr*>(Az) : nullptr, B ? reinterpret_cast<Fr*>(Bz) : nullptr,
+                         C ? reinterpret_cast<Fr*>(Cz) : nullptr}};
     k_spmv3<<<dim3(grid_for(rows, 256, sm_count() * 8), 3), 256, 0, as_stream(stream)>>>(
-        a, b, c, reinterpret_cast<const Fr*>(z), A ? reinterpret_cast<Fr*>(Az) : nullptr,
-        B ? reinterpret_cast<Fr*>(Bz) : nullptr, C ? reinterpret_cast<Fr*>(Cz) : nullptr); note_launch();
+        args, reinterpret_cast<const Fr*>(z)); note_launch();
     return launch_status();
 }
 

@@ -32,6 +32,19 @@ sys.path.insert(0, ROOT)
 METRIC = "Groth16 proofs/s & p50/p99 latency at 2^20 constraints; G1 MSM 2^20 ms"
 IMAD_PER_FP_MUL = 264          # 8x8 lo + 8x8 hi products, 8 x (1 + 8 + 8) reduction
 FP_MUL_PER_G1_MADD = 10        # XYZZ mixed addition: 8M + 2S
+FP_MUL_PER_G1_AFFINE = 6       # batched affine addition: 5M + 1S, the inversions' share left out
+
+
+def g1_products(points, c, windows):
+    """Fq products of a G1 table MSM's bucket accumulation: R rounds of affine
+    additions (the rule of csrc/msm.cuh: they stop while a bucket still holds
+    eight points) merge all but a 2^-R share of the entries, the XYZZ chains
+    add the rest."""
+    entries, rounds = points * windows, 0
+    while entries >= 1 << 16 and rounds < 5 and entries >= 8 << (c - 1 + rounds + 1):
+        rounds += 1
+    rest = entries / (1 << rounds)
+    return (entries - rest) * FP_MUL_PER_G1_AFFINE + rest * FP_MUL_PER_G1_MADD
 
 
 def parse():
@@ -802,13 +815,12 @@ def main():
     # operands kept as limbs), counted in the IMAD-class unit of the
     # algorithmic work (264 per product)
     imad_peak = max(mont_rate, mont_rate_int) * IMAD_PER_FP_MUL
-    W = msm.windows_for(args.window)
     nl = circ.n_vars - circ.n_public - 1
     # G1 accumulation launches per proof: A, B1, and L + H as one MSM
     g1_points_per_proof = 2 * circ.n_vars + nl + (M - 1)
     g1_launches_per_proof = 3
     avg_pts = g1_points_per_proof / g1_launches_per_proof
-    alg_imad = avg_pts * W * FP_MUL_PER_G1_MADD * IMAD_PER_FP_MUL
+    alg_imad = g1_products(avg_pts, args.window, msm.windows_for(args.window)) * IMAD_PER_FP_MUL
     acc_avg_ms = acc_ms / max(acc_n, 1)
     achieved = alg_imad / (acc_avg_ms * 1e-3) if acc_n else None
     traffic = pipe_util = pipe_util_probe = pipe_name = None
@@ -830,7 +842,7 @@ def main():
 
     iso_line = None
     if iso_n:
-        iso_alg = iso_pts * msm.windows_for(g1_window) * FP_MUL_PER_G1_MADD * IMAD_PER_FP_MUL
+        iso_alg = g1_products(iso_pts, g1_window, msm.windows_for(g1_window)) * IMAD_PER_FP_MUL
         iso_avg = iso_ms / iso_n
         iso_line = {"workload": f"G1 MSM 2^{int(np.log2(iso_pts))} alone", "avg_launch_ms": iso_avg,
                     "launches": iso_n, "achieved": iso_alg / (iso_avg * 1e-3) / 1e12,
@@ -874,12 +886,13 @@ def main():
         "e2e": {"value": world * args.steps / (e2e_ms * 1e-3), "unit": "proofs/s",
                 "h2d_bytes_per_step": int(wits[0].numel() * 8), "d2h_bytes_per_step": groth16.PROOF_WORDS * 8},
         "gpu_launches": launches,
-        # the dominant kernel timed alone, on the metric's own G1 MSM 2^20
-        # (CUDA events around each accumulation launch, nothing else on the
-        # GPU); inside a proof the same kernel shares the GPU with three other
+        # the dominant phase timed alone, on the metric's own G1 MSM 2^20
+        # (CUDA events around each MSM's accumulation, nothing else on the
+        # GPU); inside a proof the same kernels share the GPU with three other
         # streams, so its event time there measures the interleaving as much
-        # as the kernel (reported as in_proof)
-        "roofline": {"kernel": "k_accumulate<Fq> (G1 bucket accumulation)", "bound": "int",
+        # as the kernels (reported as in_proof)
+        "roofline": {"kernel": "k_affine_prefix_g1 / k_affine_invert / k_affine_sum_g1 / k_accumulate<Fq> "
+                               "(G1 bucket accumulation)", "bound": "int",
                      "workload": iso_line["workload"] if iso_line else None,
                      "achieved": iso_line["achieved"] if iso_line else None, "peak": imad_peak / 1e12,
                      "unit": "T IMAD/s", "frac": iso_line["frac"] if iso_line else None,
@@ -889,8 +902,9 @@ def main():
                                     "it and the 32-bit-limb integer form) x 264 IMAD-class per product",
                      "mont_products_per_s": mont_rate, "mont_products_per_s_int_form": mont_rate_int,
                      "pipe": pipe_name, "pipe_util": pipe_util, "pipe_util_probe": pipe_util_probe,
-                     "pipe_util_source": "ncu sm__pipe_fp64_cycles_active of one G1 accumulation launch at 2^20 "
-                                         "and of the probe (profiles/k_accumulate_2e20.md)",
+                     "pipe_util_source": "ncu sm__pipe_fp64_cycles_active of the first round's sums at 2^20 "
+                                         "(profiles/k_affine_2e20.md) and of the probe "
+                                         "(profiles/k_accumulate_2e20.md)",
                      "peak_mad_chains_T": mad_chain_rate / 1e12,
                      "algorithmic_imad_per_launch": iso_line["algorithmic_imad_per_launch"] if iso_line else None,
                      "avg_launch_ms": iso_line["avg_launch_ms"] if iso_line else None,

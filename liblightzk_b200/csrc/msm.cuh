@@ -217,7 +217,8 @@ size_t msm_concat_bytes(size_t n, const lzk_msm_cfg* cfg, uint32_t rounds);
 // exclusive scan of cnt[0..B), each rounded up to a multiple of 2^rounds,
 // into off[0..B], off[B] = total; bsums holds (B + 4095) / 4096 + 1 words
 // (msm_sort.cu)
-int scan_offsets(const uint32_t* cnt, uint32_t B, uint32_t* off, uint32_t* bsums, cudaStream_t st, uint32_t rounds = 0);
+int scan_offsets(uint32_t* cnt, uint32_t B, uint32_t* off, uint32_t* bsums, cudaStream_t st, uint32_t rounds = 0,
+                 bool cursors = false);
 // All rounds of a padded list of at most max_slots slots into fin (point i is
 // what slots [i 2^rounds, (i + 1) 2^rounds) sum to), a slice at a time.
 template <class F>

@@ -121,6 +121,11 @@ inline uint32_t acc_chunk(uint32_t chunk, uint32_t rounds)
 inline uint32_t windows_for(uint32_t c) { return (255 + c - 1) / c; }
 // windows of a half scalar: its top digit, with the carry, stays <= 2^(c-1)
 inline uint32_t windows_glv(uint32_t c) { return (kGlvBits + 1 + c - 1) / c; }
+// Sorted entries of n scalars; their numbers, and the offsets of the buckets,
+// are 32 bits.  The endomorphism makes up to two entries a scalar more than
+// the plain digits do (16 against 15 at c = 17), fewer at other widths.
+inline uint64_t msm_entries(uint64_t n, uint32_t c, bool glv) { return n * (glv ? 2 * windows_glv(c) : windows_for(c)); }
+constexpr uint64_t kMaxEntries = (uint64_t(1) << 32) - 1;
 
 // accumulation chunk and reduction run of an MSM of n points in group g:
 // cfg's values, else the tuning table's (plain bases, or tables with
@@ -146,7 +151,7 @@ inline void plan_msm(MsmPlan& p, size_t n, uint32_t c, bool shared, size_t strid
     p.shared = shared; p.stride = stride;
     p.wb = shared ? 1 : p.W;
     p.B = p.wb * p.nb;
-    p.max_entries = n * (size_t)p.W * (glv ? 2 : 1);
+    p.max_entries = msm_entries(n, c, glv);
     p.run = run;
     p.rounds = rounds;
     p.max_slots = p.max_entries + (size_t)p.B * ((1u << rounds) - 1);
@@ -844,15 +849,24 @@ __global__ void k_write_inf(Jac<F>* out)
 }
 
 // Plain G1 bases are doubled by the endomorphism: half the windows, bucket
-// sets and serial doublings for the same additions.  (G2 has none that holds
+// sets and serial doublings for the same additions, where the entries can be
+// numbered and the doubled bases keep their sign bit.  (G2 has none that holds
 // for points outside the prime-order subgroup; a table needs none of these.)
-inline bool msm_glv(int group, size_t n, bool shared) { return group == 1 && !shared && n < (size_t(1) << 30); }
+inline bool msm_glv(int group, size_t n, uint32_t c, bool shared)
+{
+    return group == 1 && !shared && n < (size_t(1) << 30) && msm_entries(n, c, true) <= kMaxEntries;
+}
+// whether an MSM of n points can be sorted at this width, in either form
+inline bool msm_width_fits(int group, size_t n, uint32_t c, bool shared)
+{
+    return msm_glv(group, n, c, shared) || msm_entries(n, c, false) <= kMaxEntries;
+}
 // affine rounds of an MSM over bases in this layout
 inline uint32_t msm_rounds(int group, size_t n, uint32_t c, bool shared, uint32_t layout)
 {
-    const bool glv = msm_glv(group, n, shared);
+    const bool glv = msm_glv(group, n, c, shared);
     const size_t W = glv ? windows_glv(c) : windows_for(c);
-    return layout == LZK_BASES_AFFINE || glv ? affine_rounds(n * W * (glv ? 2 : 1), (shared ? 1 : W) << (c - 1),
+    return layout == LZK_BASES_AFFINE || glv ? affine_rounds(msm_entries(n, c, glv), (shared ? 1 : W) << (c - 1),
                                                              shared ? kAffFillTable : kAffFillPlain)
                                            : 0;
 }
@@ -904,16 +918,17 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
         return launch_status();
     }
     const int group = sizeof(F) == 32 ? 1 : 2;
+    if (!msm_width_fits(group, n, c, shared)) return LZK_EINVAL;
     uint32_t chunk = msm_chunk(cfg, group, n), run = msm_run(cfg, group, n);
     if (!tune_valid(LZK_TUNE_MSM_CHUNK, chunk) || !tune_valid(LZK_TUNE_MSM_REDUCE_RUN, run)) return LZK_EINVAL;
     MsmPlan p;
     plan_msm<Gp>(p, n, c, shared, stride, chunk, run,
                  form != kMsmFull ? 0 : pre_off ? pre_rounds : msm_rounds(group, n, c, shared, layout),
-                 pre_off && !pre_in_ws, form != kMsmLean && msm_glv(group, n, shared));
+                 pre_off && !pre_in_ws, form != kMsmLean && msm_glv(group, n, c, shared));
     void* tr_all = trace_begin(sizeof(F) == 32 ? "msm_g1" : "msm_g2", st);
     Scratch ws;
     int got = ws.acquire(p.bytes, cfg ? cfg->workspace : nullptr, cfg ? cfg->workspace_bytes : 0, st);
-    if (got != LZK_OK && (p.rounds || p.glv) && !pre_off) {
+    if (got != LZK_OK && (p.rounds || p.glv) && !pre_off && msm_entries(n, c, false) <= kMaxEntries) {
         // too little scratch for the affine rounds and the doubled bases: XYZZ
         // additions alone
         plan_msm<Gp>(p, n, c, shared, stride, chunk, run);

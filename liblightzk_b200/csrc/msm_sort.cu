@@ -172,18 +172,19 @@ int msm_sort(const MsmPlan& p, const Fr* scalars, uint32_t* cnt, uint32_t* off, 
 // the reduction (two XYZZ adds per bucket, 12M+2S) plus, for plain bases,
 // the serial Horner doublings, weighted by their latency cost.
 // measured window widths come from the tuning table (tune.cu), by group and
-// ceil(log2 n); an unset entry falls back to the model
+// ceil(log2 n); an unset entry, or one too narrow for this n (kMaxEntries),
+// falls back to the model
 uint32_t msm_autotune(int group, size_t n, bool shared)
 {
     if (n && group >= 1 && group <= 2) {
         uint32_t w = tune_lookup(shared ? LZK_TUNE_MSM_TABLE_WINDOW : LZK_TUNE_MSM_WINDOW, group, n);
-        if (w) return w;
+        if (w && msm_width_fits(group, n, w, shared)) return w;
     }
-    (void)group;
     if (n == 0) return 8;
     double best = 1e300; uint32_t bc = 8;
     for (uint32_t c = 4; c <= 22; c++) {
-        const bool glv = msm_glv(group, n, shared);
+        if (!msm_width_fits(group, n, c, shared)) continue;
+        const bool glv = msm_glv(group, n, c, shared);
         double W = glv ? windows_glv(c) : windows_for(c);
         double sets = shared ? 1.0 : W;
         double cost = (double)n * (glv ? 2.0 : 1.0) * W * 10.0 + sets * (double)(1u << (c - 1)) * 2.0 * 14.0;
@@ -257,13 +258,13 @@ size_t lzk_msm_workspace_bytes(int group, size_t n, const lzk_msm_cfg* cfg)
 {
     bool shared = cfg && (cfg->flags & LZK_MSM_PRECOMPUTED);
     uint32_t c = (cfg && cfg->window_bits) ? cfg->window_bits : msm_autotune(group, n, shared);
-    if (c < 2 || c > 24 || n == 0) return 0;
+    if (c < 2 || c > 24 || n == 0 || !msm_width_fits(group, n, c, shared)) return 0;
     uint32_t chunk = msm_chunk(cfg, group, n), run = msm_run(cfg, group, n);
     if (!tune_valid(LZK_TUNE_MSM_CHUNK, chunk)) return 0;
     MsmPlan p;
     const uint32_t rounds = msm_rounds(group, n, c, shared, cfg ? cfg->base_layout : (uint32_t)LZK_BASES_AFFINE);
     if (group == 2) plan_msm<G2>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run, rounds);
-    else plan_msm<G1>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run, rounds, false, msm_glv(group, n, shared));
+    else plan_msm<G1>(p, n, c, shared, cfg ? cfg->level_stride : 0, chunk, run, rounds, false, msm_glv(group, n, c, shared));
     return p.bytes;
 }
 

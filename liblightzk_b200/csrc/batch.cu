@@ -431,24 +431,58 @@ static uint32_t batch_window(int group, size_t n, bool fixed, bool glv, bool wid
     return best;
 }
 
+// Whether the layout of these widths can be numbered: points and table entries
+// with 31 bits beside the sign, buckets and sorted entries with 32 (and, with
+// few set, a persistent launch takes that many widths).
+static bool widths_fit(const lzk_msm_desc* msms, const std::vector<uint32_t>& cw, const lzk_batch_plan* p, bool few)
+{
+    uint64_t pts = 0, table = 0, buckets = 0, entries = 0;
+    uint32_t used = 0;
+    for (size_t i = 0; i < cw.size(); i++) {
+        const uint32_t c = cw[i], W = p->glv ? windows_glv(c) : windows_for(c);
+        pts += msms[i].n;
+        if (p->fixed) table += msms[i].n * (uint64_t)W;
+        buckets += (uint64_t)(p->fixed ? 1 : W) << (c - 1);
+        entries += msm_entries(msms[i].n, c, p->glv);
+        used |= 1u << c;
+    }
+    return pts < (1ull << 31) && table < (1ull << 31) && buckets < (1ull << 32) - 1 && entries <= kMaxEntries &&
+           !(few && (uint32_t)__builtin_popcount(used) > kMaxRedJobs);
+}
+
+// The MSMs' widths, and whether their scalars are halved: by total work over
+// the endomorphism, or, where that layout has too many entries, table points
+// or widths, without the endomorphism, and at last with the widths of the MSMs
+// alone, which are the widest.
+static int plan_widths(const lzk_msm_desc* msms, size_t n_msm, bool full, lzk_batch_plan* p, std::vector<uint32_t>& cw)
+{
+    size_t all = 0;
+    for (size_t i = 0; i < n_msm; i++) {
+        if (!msms[i].out || (msms[i].n && (!msms[i].scalars || !msms[i].bases))) return LZK_EINVAL;
+        if (msms[i].window_bits == 1 || msms[i].window_bits > 24) return LZK_EINVAL;
+        if (msms[i].n >= (1ull << 31)) return LZK_EINVAL;
+        all += msms[i].n;
+    }
+    for (int form = full ? 0 : 2; form < 3; form++) {
+        p->glv = form == 0 && !p->fixed && p->group == 1 && all < (size_t(1) << 30);
+        for (size_t i = 0; i < n_msm; i++)
+            cw[i] = msms[i].window_bits ? msms[i].window_bits
+                                        : batch_window(p->group, msms[i].n, p->fixed, p->glv, form < 2 && all >= kWidePlan);
+        if (widths_fit(msms, cw, p, p->persistent && form < 2)) return LZK_OK;
+    }
+    return LZK_EINVAL;
+}
+
 template <class F>
 static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_desc* ntts, size_t n_ntt,
                        lzk_batch_plan* p, bool with_rounds)
 {
     using X = XYZZ<F>;
     // MSMs: widths, ordering, global layout
-    std::vector<size_t> order(n_msm);
     std::vector<uint32_t> cw(n_msm);
-    size_t all = 0;
-    for (size_t i = 0; i < n_msm; i++) all += msms[i].n;
-    p->glv = with_rounds && !p->fixed && p->group == 1 && all < (size_t(1) << 30);
-    const bool wide = all >= kWidePlan;
-    for (size_t i = 0; i < n_msm; i++) {
-        if (!msms[i].out || (msms[i].n && (!msms[i].scalars || !msms[i].bases))) return LZK_EINVAL;
-        cw[i] = msms[i].window_bits ? msms[i].window_bits : batch_window(p->group, msms[i].n, p->fixed, p->glv, wide);
-        if (cw[i] < 2 || cw[i] > 24) return LZK_EINVAL;
-        order[i] = i;
-    }
+    LZK_TRY(plan_widths(msms, n_msm, with_rounds, p, cw));
+    std::vector<size_t> order(n_msm);
+    for (size_t i = 0; i < n_msm; i++) order[i] = i;
     std::stable_sort(order.begin(), order.end(), [&](size_t a, size_t b) { return cw[a] < cw[b]; });
     std::vector<uint64_t> ptsoff;
     for (size_t o : order) {
@@ -472,16 +506,13 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
         p->total_pts += m.n;
         p->total_buckets += (uint64_t)d.hw * d.nb;
         p->total_windows += d.hw;
-        p->max_entries += m.n * (uint64_t)d.W * (p->glv ? 2 : 1);
+        p->max_entries += msm_entries(m.n, d.c, p->glv);
         if (p->wgroups.empty() || p->wgroups.back().c != d.c) p->wgroups.push_back({d.c, d.bucket_base, 0, 0, 0, 0});
         p->wgroups.back().windows += d.hw;
         p->wgroups.back().largest = std::max<size_t>(p->wgroups.back().largest, m.n);
         ptsoff.push_back(d.pts_off);
         p->msm.push_back(d);
     }
-    if (p->total_pts >= (1ull << 31) || p->table_pts >= (1ull << 31) || p->total_buckets >= (1ull << 32) - 1 ||
-        p->max_entries >= (1ull << 32))
-        return LZK_EINVAL;
     // the plan's largest MSM picks the accumulation chunk and reduction run
     size_t largest = 0;
     for (size_t i = 0; i < n_msm; i++) largest = std::max(largest, msms[i].n);
@@ -599,7 +630,8 @@ int lzk_batch_plan_create_ex(int group, const lzk_msm_desc* msms, size_t n_msm, 
     *out = nullptr;
     lzk_batch_plan* p = nullptr;
     int rc = LZK_ENOMEM;
-    // a device without room for the affine rounds' scratch still takes the plan
+    // a device without room for the affine rounds' scratch, or for the larger
+    // tables of narrower widths, still takes the plan
     for (bool rounds : {true, false}) {
         p = new (std::nothrow) lzk_batch_plan();
         if (!p) return LZK_ENOMEM;
@@ -610,7 +642,7 @@ int lzk_batch_plan_create_ex(int group, const lzk_msm_desc* msms, size_t n_msm, 
         rc = group == 2 ? create_plan<Fq2>(msms, n_msm, ntts, n_ntt, p, rounds)
                         : create_plan<Fq>(msms, n_msm, ntts, n_ntt, p, rounds);
         if (rc == LZK_OK) break;
-        const bool again = rc == LZK_ENOMEM && (p->rounds || p->glv);
+        const bool again = rc == LZK_ENOMEM && rounds;
         destroy_plan(p);
         if (!again) return rc;
     }

@@ -1,6 +1,6 @@
 """Sorted entries are numbered with 32 bits: an MSM whose two halves a scalar
 (csrc/glv.cuh) would make too many takes the plain digits, one that is too
-large in either form is refused.
+large in either form is refused, and a batch plan falls back the same way.
 
 The sizes are at the limits, so the tests on the CPU stop at the first device
 allocation (any status but LZK_EINVAL means the size was accepted); the GPU
@@ -12,7 +12,7 @@ import pytest
 import torch
 
 EINVAL = -1
-WINDOW = 0
+WINDOW, TABLE_WINDOW = 0, 4
 MAX_ENTRIES = (1 << 32) - 1
 
 
@@ -76,6 +76,46 @@ def test_tuned_width_that_does_not_fit_is_passed_over(n):
         assert msm.workspace_bytes(1, n) > 0
     finally:
         L.lzk_tune_set(WINDOW, 1, 29, saved)
+
+
+def _plan_status(sizes, flags=0, window=0):
+    from liblightzk_b200 import _capi
+    md = (_capi.MsmDesc * len(sizes))()
+    for m, n in zip(md, sizes):
+        m.scalars = m.bases = m.out = 256
+        m.n, m.window_bits = n, window
+    h = ctypes.c_void_p()
+    return _lib().lzk_batch_plan_create_ex(1, md, len(sizes), None, 0, flags, ctypes.byref(h))
+
+
+def test_plan_without_the_endomorphism():
+    _no_gpu()
+    n = MAX_ENTRIES // 16 + 1
+    assert _plan_status([n // 2, n - n // 2], window=17) != EINVAL
+    assert _plan_status([MAX_ENTRIES // 15 + 1], window=17) == EINVAL
+
+
+def test_fixed_plan_with_the_widths_of_its_msms():
+    # by total work these would take narrow windows, whose tables hold more
+    # points than can be numbered
+    _no_gpu()
+    L = _lib()
+    assert L.lzk_tune_set(TABLE_WINDOW, 1, 10, 16) == 0
+    try:
+        assert _plan_status([1000] * 130000, flags=1) != EINVAL
+    finally:
+        L.lzk_tune_set(TABLE_WINDOW, 1, 10, 0)
+
+
+def test_persistent_plan_of_too_many_widths_stays_unsupported():
+    _no_gpu()
+    from liblightzk_b200 import _capi
+    md = (_capi.MsmDesc * 21)()
+    for i, m in enumerate(md):
+        m.scalars = m.bases = m.out = 256
+        m.n, m.window_bits = 10, 2 + i
+    h = ctypes.c_void_p()
+    assert _lib().lzk_batch_plan_create_ex(1, md, 21, None, 0, 2, ctypes.byref(h)) == -5
 
 
 @pytest.mark.gpu

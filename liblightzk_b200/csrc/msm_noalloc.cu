@@ -103,6 +103,10 @@ int lzk_msm_g1_noalloc(const lzk_fr_t* scalars, const lzk_g1_affine_t* bases, si
     // sizes), the endomorphism where its doubled bases fit
     MsmForm form = kMsmNoRounds;
     if (msm_form_bytes(n, &cfg, form) > LZK_MSM_NOALLOC_SCRATCH_BYTES) form = kMsmLean;
+    // longer chunks leave fewer partial sums: a tuned short one does not
+    // refuse a size that fits without it
+    cfg.acc_chunk = msm_chunk(&cfg, 1, n);
+    while (cfg.acc_chunk < kMaxChunk && msm_form_bytes(n, &cfg, form) > LZK_MSM_NOALLOC_SCRATCH_BYTES) cfg.acc_chunk *= 2;
     if (msm_form_bytes(n, &cfg, form) > LZK_MSM_NOALLOC_SCRATCH_BYTES) return LZK_EINVAL;
     void* scratch = nullptr;
     int dev = 0;

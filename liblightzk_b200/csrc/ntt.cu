@@ -559,10 +559,10 @@ int ntt_prepare_launch()
 // Whether a transform of size 2^k is one pass of several steps, whose only
 // block has read every element when it writes the first one: such a DIF
 // transform writes its results in natural order itself.
-static bool ntt_one_pass(uint32_t k) { return k > 2 && (1u << k) <= tune_ntt_block(k); }
+static bool ntt_one_pass(uint32_t k, uint32_t block) { return k > 2 && k < 32 && (1u << k) <= block; }
 
 int ntt_passes(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* tw, bool dit, NttEdge pre,
-               NttEdge post, cudaStream_t st, Fr* const* ptrs, const double* twd, bool natural)
+               NttEdge post, cudaStream_t st, Fr* const* ptrs, const double* twd, uint32_t elems, bool natural)
 {
     if (k == 0 || k > 30 || count == 0 || count > 65535 || (!data && !ptrs) || !tw) return LZK_EINVAL;
     LZK_TRY(ntt_prepare_launch());
@@ -570,8 +570,8 @@ int ntt_passes(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* t
         k_ntt_two<<<count, 32, 0, st>>>(data, pre, post, bstride, ptrs); note_launch();
         return launch_status();
     }
-    // block size from the tuning table: 2^maxm elements, at most maxm stages a pass
-    const uint32_t elems = tune_ntt_block(k);
+    // blocks of 2^maxm elements, at most maxm stages a pass
+    if (!elems) elems = tune_ntt_block(k);
     uint32_t maxm = 0;
     while ((1u << (maxm + 1)) <= elems) maxm++;
     const uint32_t P = (k + maxm - 1) / maxm;
@@ -590,7 +590,7 @@ int ntt_passes(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* t
         if (R == 0) R = 1;
         pp.R = R;
         pp.canon = q == P - 1;
-        pp.natural = natural && ntt_one_pass(k);
+        pp.natural = natural;
         const unsigned threads = G * R / 4 < kNttThreads ? G * R / 4 : kNttThreads;
         size_t blocks = (n >> m) / R;
         size_t smem = (size_t)G * R * sizeof(Fr);
@@ -623,8 +623,12 @@ static int ntt_enqueue(Fr* data, uint32_t k, uint32_t count, size_t bstride, con
         k_ntt_one<<<count, 32, 0, st>>>(data, post.scale, bstride, ptrs); note_launch();
         return launch_status();
     }
-    LZK_TRY(ntt_passes(data, k, count, bstride, tw, false, pre, post, st, ptrs, twd, true));
-    if (k < 2 || ntt_one_pass(k)) return launch_status();
+    // one look at the tuning table, which another thread may be setting: the
+    // passes and the reversal have to agree on it
+    const uint32_t block = tune_ntt_block(k);
+    const bool one = ntt_one_pass(k, block);
+    LZK_TRY(ntt_passes(data, k, count, bstride, tw, false, pre, post, st, ptrs, twd, block, one));
+    if (k < 2 || one) return launch_status();
     if (k < 10) {
         k_ntt_bitrev<<<dim3(grid_for(size_t(1) << k, 256), count), 256, 0, st>>>(data, k, bstride, ptrs); note_launch();
     } else {

@@ -53,9 +53,11 @@ int ntt_run(Fr* data, uint32_t k, int dir, uint32_t count, size_t bstride, const
 // bit-reversed order, DIT bit-reversed order to natural order.  pre applies
 // to the first pass's loads, post to the last pass's stores.  twd, when
 // given, is the same table in radix-2^52 form (NttTables::twd), which the
-// butterflies then read instead of converting tw.  natural: a DIF transform
-// that is one pass writes natural order itself (ntt_run).
+// butterflies then read instead of converting tw.  block: elements a block
+// (0: the tuning table's).  natural: a DIF transform that is one pass writes
+// natural order itself (ntt_run).
 int ntt_passes(Fr* data, uint32_t k, uint32_t count, size_t bstride, const Fr* tw, bool dit, NttEdge pre,
-               NttEdge post, cudaStream_t st, Fr* const* ptrs = nullptr, const double* twd = nullptr, bool natural = false);
+               NttEdge post, cudaStream_t st, Fr* const* ptrs = nullptr, const double* twd = nullptr, uint32_t block = 0,
+               bool natural = false);
 
 }  // namespace lzk

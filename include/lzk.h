@@ -382,7 +382,13 @@ typedef struct lzk_server_stats {
 #define LZK_REQ_WITNESS_PINNED 0x1u
 
 int lzk_server_create(const lzk_server_cfg* cfg, lzk_server** out);
-/* The prover stays owned by the caller and must outlive the server. */
+/* The prover stays owned by the caller and must outlive the server.  LZK_EBUSY:
+ * the budget has no room for it.  A prover that exceeds the budget only with
+ * the scratch of its own proofs (lzk_groth16_prove) gives most of that back,
+ * for good: the call then waits for the device, lzk_prover_device_bytes
+ * shrinks, the prover's own proofs run without the batched affine rounds (at
+ * 2^20 constraints 25 instead of 20 ms), and a CUDA graph that holds one of
+ * them must be captured again. */
 int lzk_server_add_circuit(lzk_server* server, lzk_prover* prover, uint32_t* circuit_id);
 /* z: HOST witness (n_vars Fr); r, s: host values. */
 int lzk_server_submit(lzk_server* server, uint32_t circuit_id, const lzk_fr_t* z, const lzk_fr_t* r,

@@ -226,12 +226,21 @@ static int dalloc(size_t* acct, T** ptr, size_t count)
     return LZK_OK;
 }
 
+// the buffers whose sizes depend on the context's shape
+static void ctx_drop_scratch(ProveCtx* x)
+{
+    for (auto& w : x->ws) { if (w) cudaFree(w); w = nullptr; }
+    uint32_t** sort[] = {&x->zs_cnt, &x->zs_off, &x->zs_ent, &x->zs_bsums};
+    for (auto q : sort) { if (*q) cudaFree(*q); *q = nullptr; }
+    x->bytes -= x->scratch_bytes;
+    x->scratch_bytes = 0;
+}
+
 void ctx_destroy(ProveCtx* x)
 {
     if (!x) return;
-    for (auto w : x->ws) if (w) cudaFree(w);
-    void* misc[] = {x->x, x->g1res, x->g2res, x->sm1, x->sm2, x->z, x->proof,
-                    x->zs_cnt, x->zs_off, x->zs_ent, x->zs_bsums};
+    ctx_drop_scratch(x);
+    void* misc[] = {x->x, x->g1res, x->g2res, x->sm1, x->sm2, x->z, x->proof};
     for (auto m : misc) if (m) cudaFree(m);
     if (x->proof_host) cudaFreeHost(x->proof_host);
     if (x->ev_done) cudaEventDestroy(x->ev_done);
@@ -283,6 +292,28 @@ size_t ctx_bytes(const lzk_prover* p, bool serving, bool lean)
     return serving ? b + p->n_vars * sizeof(Fr) + sizeof(lzk_groth16_proof) : b;
 }
 
+// Scratch of a shape; on failure the context holds none.
+static int ctx_make_scratch(const lzk_prover* p, ProveCtx* x, bool lean)
+{
+    const CtxShape s = ctx_shape(p, lean);
+    x->lean = lean;
+    x->lh_rounds = s.lh_rounds;
+    x->z_rounds = s.z_rounds;
+    int rc = LZK_OK;
+    size_t* acct = &x->scratch_bytes;
+    for (int i = 0; i < 4 && rc == LZK_OK; i++) {
+        x->wsb[i] = s.wsb[i];
+        if (s.wsb[i]) rc = dalloc(acct, reinterpret_cast<char**>(&x->ws[i]), x->wsb[i]);
+    }
+    if (rc == LZK_OK) rc = dalloc(acct, &x->zs_cnt, s.sort.cnt);
+    if (rc == LZK_OK) rc = dalloc(acct, &x->zs_off, s.sort.off);
+    if (rc == LZK_OK) rc = dalloc(acct, &x->zs_ent, s.sort.ent);
+    if (rc == LZK_OK) rc = dalloc(acct, &x->zs_bsums, s.sort.bsums);
+    x->bytes += x->scratch_bytes;
+    if (rc != LZK_OK) { cudaGetLastError(); ctx_drop_scratch(x); }
+    return rc;
+}
+
 // Scratch for one proof of prover p; serving contexts also get their own
 // main stream and witness and proof buffers.
 int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out, bool lean)
@@ -290,10 +321,6 @@ int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out, bool lean)
     *out = nullptr;
     ProveCtx* x = new (std::nothrow) ProveCtx();
     if (!x) return LZK_ENOMEM;
-    x->lean = lean;
-    const CtxShape s = ctx_shape(p, lean);
-    x->lh_rounds = s.lh_rounds;
-    x->z_rounds = s.z_rounds;
     int rc = LZK_OK;
     do {
         if ((rc = dalloc(&x->bytes, &x->x, 3 * p->L))) break;
@@ -301,16 +328,7 @@ int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out, bool lean)
         if ((rc = dalloc(&x->bytes, &x->g2res, 1))) break;
         if ((rc = dalloc(&x->bytes, &x->sm1, 6))) break;
         if ((rc = dalloc(&x->bytes, &x->sm2, 1))) break;
-        for (int i = 0; i < 4 && rc == LZK_OK; i++) {
-            x->wsb[i] = s.wsb[i];
-            if (!s.wsb[i]) continue;
-            rc = dalloc(&x->bytes, reinterpret_cast<char**>(&x->ws[i]), x->wsb[i]);
-        }
-        if (rc) break;
-        if ((rc = dalloc(&x->bytes, &x->zs_cnt, s.sort.cnt))) break;
-        if ((rc = dalloc(&x->bytes, &x->zs_off, s.sort.off))) break;
-        if ((rc = dalloc(&x->bytes, &x->zs_ent, s.sort.ent))) break;
-        if ((rc = dalloc(&x->bytes, &x->zs_bsums, s.sort.bsums))) break;
+        if ((rc = ctx_make_scratch(p, x, lean))) break;
         if (serving) {
             if ((rc = dalloc(&x->bytes, &x->z, p->n_vars))) break;
             if ((rc = dalloc(&x->bytes, &x->proof, 1))) break;
@@ -576,15 +594,26 @@ int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, 
     return launch_status();
 }
 
-int prover_make_lean(lzk_prover* p)
+// the scratch of the prover's own context, where an earlier prover_fit left none
+static int own_scratch(lzk_prover* p) { return p->ctx0->zs_ent ? LZK_OK : ctx_make_scratch(p, p->ctx0, true); }
+
+// The bytes of prover p if they are at most `room`; a prover that exceeds it
+// only with its own context's full scratch gives that back for good and takes
+// the lean scratch.  The larger scratch is freed first, so a nearly full device
+// can still do it; should the smaller one not be had all the same (LZK_ENOMEM),
+// the next proof tries again.
+int prover_fit(lzk_prover* p, size_t room, size_t* bytes)
 {
     std::lock_guard<std::mutex> g(p->mu);
-    if (p->ctx0->lean) return LZK_OK;
-    LZK_CUDA(cudaDeviceSynchronize());   // proofs in flight use the context
-    ProveCtx* x = nullptr;
-    LZK_TRY(ctx_create(p, false, &x, true));
-    ctx_destroy(p->ctx0);
-    p->ctx0 = x;
+    ProveCtx* x = p->ctx0;
+    LZK_TRY(own_scratch(p));
+    if (p->bytes + x->bytes > room) {
+        if (x->lean || p->bytes + ctx_bytes(p, false, true) > room) return LZK_EBUSY;
+        LZK_CUDA(cudaDeviceSynchronize());   // proofs in flight use the context
+        ctx_drop_scratch(x);
+        LZK_TRY(ctx_make_scratch(p, x, true));
+    }
+    *bytes = p->bytes + x->bytes;
     return LZK_OK;
 }
 
@@ -700,7 +729,12 @@ int lzk_prover_destroy(lzk_prover* p)
     return LZK_OK;
 }
 
-size_t lzk_prover_device_bytes(const lzk_prover* p) { return p ? p->bytes + (p->ctx0 ? p->ctx0->bytes : 0) : 0; }
+size_t lzk_prover_device_bytes(const lzk_prover* p)
+{
+    if (!p) return 0;
+    std::lock_guard<std::mutex> g(p->mu);
+    return p->bytes + (p->ctx0 ? p->ctx0->bytes : 0);
+}
 
 int lzk_poly_a_times_b_minus_c(lzk_fr_t* A, const lzk_fr_t* B, const lzk_fr_t* C, size_t n, void* stream)
 {
@@ -716,6 +750,7 @@ int lzk_groth16_prove(lzk_prover* p, const lzk_fr_t* z, const lzk_fr_t* r, const
 {
     if (!p) return LZK_EINVAL;
     std::lock_guard<std::mutex> g(p->mu);
+    LZK_TRY(own_scratch(p));
     return prove_ctx(p, p->ctx0, reinterpret_cast<const Fr*>(z), r, s, proof, as_stream(stream));
 }
 

@@ -37,7 +37,7 @@ struct ProveCtx {
                 ev_sorted = nullptr;
     uint32_t lh_rounds = 0, z_rounds = 0;   // affine rounds of the L + H MSM; of A, B1 and B2
     bool lean = false;                // no affine rounds (affine.cuh): a third of the scratch, slower
-    size_t bytes = 0;
+    size_t bytes = 0, scratch_bytes = 0;   // all; what depends on the shape (ws, zs_*)
 };
 
 }  // namespace lzk
@@ -68,7 +68,7 @@ struct lzk_prover {
     lzk::Aff<lzk::Fq2>* comb2 = nullptr;  // comb table of d2
     lzk::ProveCtx* ctx0 = nullptr;
     size_t bytes = 0;       // resident bytes (tables, constants)
-    std::mutex mu;          // held while ctx0 is used to enqueue or replaced
+    mutable std::mutex mu;  // held while ctx0 is used to enqueue, measured or made lean
 };
 
 namespace lzk {
@@ -77,8 +77,8 @@ namespace lzk {
 // ctx_bytes: what it will hold
 int ctx_create(const lzk_prover* p, bool serving, ProveCtx** out, bool lean = false);
 size_t ctx_bytes(const lzk_prover* p, bool serving, bool lean);
-// replace the prover's own context by a lean one
-int prover_make_lean(lzk_prover* p);
+// the prover's bytes, its own context made lean where only so they are at most room
+int prover_fit(lzk_prover* p, size_t room, size_t* bytes);
 void ctx_destroy(ProveCtx* x);
 // enqueue one proof on stream st using context x (x's side streams join st)
 int prove_ctx(const lzk_prover* p, ProveCtx* x, const Fr* z, const lzk_fr_t* r, const lzk_fr_t* s,

@@ -226,15 +226,9 @@ int lzk_server_add_circuit(lzk_server* s, lzk_prover* prover, uint32_t* circuit_
 {
     if (!s || !prover || !circuit_id) return LZK_EINVAL;
     std::lock_guard<std::mutex> g(s->mu);
-    size_t rb = lzk_prover_device_bytes(prover);
-    if (s->resident_bytes + rb > s->cfg.hbm_budget_bytes) {
-        // a prover too large with its own context's full scratch may fit with
-        // a lean one
-        const size_t lean = rb - prover->ctx0->bytes + lzk::ctx_bytes(prover, false, true);
-        if (s->resident_bytes + lean > s->cfg.hbm_budget_bytes) return LZK_EBUSY;
-        LZK_TRY(lzk::prover_make_lean(prover));
-        rb = lzk_prover_device_bytes(prover);
-    }
+    size_t rb = 0;
+    if (s->resident_bytes > s->cfg.hbm_budget_bytes) return LZK_EBUSY;
+    LZK_TRY(lzk::prover_fit(prover, s->cfg.hbm_budget_bytes - s->resident_bytes, &rb));
     s->resident_bytes += rb;
     Circuit c;
     c.prover = prover;

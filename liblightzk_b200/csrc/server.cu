@@ -7,7 +7,9 @@
 //   * admission: the oldest queued request whose circuit has an idle proof
 //     context, or whose new context fits the budget (idle contexts of other
 //     circuits are released to make room), is started; a request whose
-//     context could never fit is rejected;
+//     context could never fit is rejected.  A new context holds the scratch
+//     of the affine rounds (affine.cuh) where the free budget has room for it
+//     (full_fits), else it is lean, about a third as large;
 //   * each admitted request gets its own streams, so requests that arrive
 //     while others run are admitted as contexts and memory free up and their
 //     kernels overlap on the device;
@@ -49,6 +51,7 @@ struct Circuit {
     lzk_prover* prover = nullptr;
     std::vector<ProveCtx*> idle;
     size_t live = 0;        // contexts allocated (idle + running)
+    size_t full = 0, lean = 0;   // bytes of a context with and without the affine rounds' scratch
 };
 
 }  // namespace
@@ -78,21 +81,44 @@ namespace {
 
 size_t used(const lzk_server* s) { return s->resident_bytes + s->ctx_bytes; }
 
-// release idle contexts of circuits other than `keep` until `need` more
-// bytes fit; true if they do
+// Release idle contexts of circuits other than `keep` until `need` more bytes
+// fit, the full ones first (their circuits take lean ones after that); nothing
+// is released if they would not fit all the same.
 bool make_room(lzk_server* s, uint32_t keep, size_t need)
 {
-    for (uint32_t c = 0; c < s->circuits.size() && used(s) + need > s->cfg.hbm_budget_bytes; c++) {
-        if (c == keep) continue;
-        Circuit& ci = s->circuits[c];
-        while (!ci.idle.empty() && used(s) + need > s->cfg.hbm_budget_bytes) {
-            ProveCtx* x = ci.idle.back();
-            ci.idle.pop_back();
-            s->ctx_bytes -= x->bytes;
-            ci.live--;
-            lzk::ctx_destroy(x);
+    const size_t budget = s->cfg.hbm_budget_bytes;
+    size_t idle = 0;
+    for (uint32_t c = 0; c < s->circuits.size(); c++)
+        if (c != keep) for (const ProveCtx* x : s->circuits[c].idle) idle += x->bytes;
+    if (used(s) - idle + need > budget) return false;
+    for (bool lean : {false, true})
+        for (uint32_t c = 0; c < s->circuits.size(); c++) {
+            Circuit& ci = s->circuits[c];
+            for (size_t i = ci.idle.size(); c != keep && i-- > 0 && used(s) + need > budget;) {
+                ProveCtx* x = ci.idle[i];
+                if (x->lean != lean) continue;
+                ci.idle.erase(ci.idle.begin() + i);
+                s->ctx_bytes -= x->bytes;
+                ci.live--;
+                lzk::ctx_destroy(x);
+            }
         }
+    return true;
+}
+
+// Whether a full context of circuit c fits in the free budget beside lean ones
+// for all that may be wanted besides: one of every circuit that has none, and
+// one of the largest for every further proof in flight.  A full context then
+// never costs residency, or proofs in flight, that lean ones alone would have.
+bool full_fits(const lzk_server* s, uint32_t c)
+{
+    size_t need = s->circuits[c].full, largest = 0;
+    for (uint32_t o = 0; o < s->circuits.size(); o++) {
+        const Circuit& ci = s->circuits[o];
+        if (o != c && !ci.live) need += ci.lean;
+        largest = std::max(largest, ci.lean);
     }
+    need += (s->cfg.max_inflight - 1 - s->running.size()) * largest;
     return used(s) + need <= s->cfg.hbm_budget_bytes;
 }
 
@@ -104,21 +130,23 @@ ProveCtx* get_ctx(lzk_server* s, uint32_t c, bool* never)
     *never = false;
     if (s->running.size() >= s->cfg.max_inflight) return nullptr;
     if (!ci.idle.empty()) {
-        ProveCtx* x = ci.idle.back();
-        ci.idle.pop_back();
+        auto it = std::find_if(ci.idle.begin(), ci.idle.end(), [](const ProveCtx* x) { return !x->lean; });
+        if (it == ci.idle.end()) --it;
+        ProveCtx* x = *it;
+        ci.idle.erase(it);
         return x;
     }
-    // a context with the affine rounds' scratch where it fits, else a lean one
+    if (s->resident_bytes + ci.lean > s->cfg.hbm_budget_bytes) { *never = true; return nullptr; }
     ProveCtx* x = nullptr;
-    for (bool lean : {false, true}) {
-        const size_t need = lzk::ctx_bytes(ci.prover, true, lean);
-        if (lean && s->resident_bytes + need > s->cfg.hbm_budget_bytes) { *never = true; return nullptr; }
-        if (s->resident_bytes + need > s->cfg.hbm_budget_bytes || !make_room(s, c, need)) continue;
-        if (lzk::ctx_create(ci.prover, true, &x, lean) == LZK_OK) break;
-        cudaGetLastError();
-        if (lean && !ci.live && !s->ctx_bytes) *never = true;
+    if (full_fits(s, c) && lzk::ctx_create(ci.prover, true, &x, false) != LZK_OK) cudaGetLastError();
+    if (!x) {
+        if (!make_room(s, c, ci.lean)) return nullptr;
+        if (lzk::ctx_create(ci.prover, true, &x, true) != LZK_OK) {
+            cudaGetLastError();
+            if (!ci.live && !s->ctx_bytes) *never = true;
+            return nullptr;
+        }
     }
-    if (!x) return nullptr;
     s->ctx_bytes += x->bytes;
     ci.live++;
     return x;
@@ -232,6 +260,8 @@ int lzk_server_add_circuit(lzk_server* s, lzk_prover* prover, uint32_t* circuit_
     s->resident_bytes += rb;
     Circuit c;
     c.prover = prover;
+    c.full = lzk::ctx_bytes(prover, true, false);
+    c.lean = lzk::ctx_bytes(prover, true, true);
     s->circuits.push_back(c);
     *circuit_id = (uint32_t)(s->circuits.size() - 1);
     return LZK_OK;

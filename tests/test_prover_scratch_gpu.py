@@ -23,10 +23,9 @@ def _wire(prover, z, r, s):
     return device.to_host(groth16.to_wire(prover.prove(z, r, s)))
 
 
-def _lean_bytes():
-    """of the provers below"""
+def _lean_bytes(log_m, window):
     from liblightzk_b200 import serve
-    _, p = _prover(16, 13)
+    _, p = _prover(log_m, window)
     rb = p.device_bytes()
     srv = serve.Server(rb - 1, max_inflight=1)
     srv.add(p)
@@ -40,8 +39,8 @@ def _lean_bytes():
 def test_shrinks_on_a_full_device(cuda, orc, rng_state):
     import torch
     from liblightzk_b200 import serve
-    lean = _lean_bytes()
-    circ, prover = _prover(16, 13)
+    lean = _lean_bytes(18, 13)
+    circ, prover = _prover(18, 13)
     z, (r, s) = circ.witness(5), orc.rand_field(FR, 2, rng_state)
     want = _wire(prover, z, r, s)
     torch.cuda.synchronize()
@@ -65,8 +64,8 @@ def test_shrinks_on_a_full_device(cuda, orc, rng_state):
 
 def test_no_memory_for_the_lean_scratch(cuda, orc, rng_state):
     from liblightzk_b200 import LzkError, _capi, serve
-    lean = _lean_bytes()
-    circ, prover = _prover(16, 13)
+    lean = _lean_bytes(12, 8)
+    circ, prover = _prover(12, 8)
     z, (r, s) = circ.witness(5), orc.rand_field(FR, 2, rng_state)
     want = _wire(prover, z, r, s)
     srv = serve.Server(prover.device_bytes() - 1, max_inflight=1)

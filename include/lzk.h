@@ -441,14 +441,19 @@ int lzk_batch_plan_create(int group, const lzk_msm_desc* msms, size_t n_msm, con
  * MSM shares one bucket set and no window combination remains; later
  * changes to the bases arrays are not seen (the scalars are still read at
  * every run).  For bases that stay fixed, such as a proving key's queries.
- * Window widths come from LZK_TUNE_MSM_TABLE_WINDOW. */
+ * Widths that the descriptors leave open are at most those of
+ * LZK_TUNE_MSM_TABLE_WINDOW; a plan of 2^15 points or more takes narrower ones
+ * where that is less work in all, and, persistent, widths of its own. */
 #define LZK_BATCH_FIXED_BASES 0x1u
 /* LZK_BATCH_PERSISTENT: the MSM phases after the digit sort (accumulation,
  * fix-up, the bucket reductions of every window width, the window
  * combination) run as one cooperative persistent launch of exactly the
  * blocks the device holds at once, with a grid-wide barrier between phases,
- * instead of nine launches.  Its barrier waits are bounded (about 2 s; then
- * LZK_ETIMEOUT).  Runs are eager and synchronous (use_graph is ignored); at
+ * instead of nine launches.  For a program that has to keep launches few or
+ * the plan's kernels together; it has no batched affine rounds, and the plan
+ * without it, above all captured, is faster (a plan of 24 MSMs up to 2^18
+ * points 6.4 ms over tables, persistent 8.2).  Its barrier waits are bounded
+ * (about 2 s; then LZK_ETIMEOUT).  Runs are eager and synchronous (use_graph is ignored); at
  * most 20 distinct window widths (else LZK_EUNSUPPORTED at creation).  The
  * NTTs still run on a second stream beside it. */
 #define LZK_BATCH_PERSISTENT 0x2u

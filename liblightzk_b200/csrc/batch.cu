@@ -416,10 +416,21 @@ static void destroy_plan(lzk_batch_plan* p)
 // are passed over.  A fixed-bases plan of 24 MSMs up to 2^18 and one of 22 up to
 // 2^13 points: 4716 and 720 us, against 5025 and 946 with the tuned widths.
 constexpr size_t kWidePlan = size_t(1) << 15;
-static uint32_t batch_window(int group, size_t n, bool fixed, bool glv, bool wide)
+// A persistent plan over tables with points enough, which has no rounds and
+// reduces whole G2 points, takes the widths and the chunk measured for that form
+// (the tuning table's are those of the other forms): 24 G1 MSMs up to 2^18
+// points 8221 us, by total work 8526; 12 up to 2^15 1552 and 1685.
+static uint32_t persistent_window(int group, size_t n)
+{
+    const uint32_t lg = log2_ceil(n);
+    return lg <= 10 ? (group == 1 ? 8 : 10) : lg == 11 ? (group == 1 ? 8 : 13) : lg <= 13 ? 13 : lg <= 16 ? 15 : lg <= 18 ? 16 : 17;
+}
+static uint32_t persistent_chunk(size_t largest) { return largest <= (size_t(1) << 19) ? 32 : 64; }
+static uint32_t batch_window(int group, size_t n, bool fixed, bool glv, bool wide, bool persistent)
 {
     const uint32_t tuned = msm_autotune(group, n, fixed), bits = glv ? kGlvBits + 1 : 255;
     if (!wide) return tuned;
+    if (persistent && fixed) return persistent_window(group, n);
     uint32_t best = tuned;
     double least = 1e300;
     for (uint32_t c = 4; c <= tuned; c++) {
@@ -467,7 +478,7 @@ static int plan_widths(const lzk_msm_desc* msms, size_t n_msm, bool full, lzk_ba
         p->glv = form == 0 && !p->fixed && p->group == 1 && all < (size_t(1) << 30);
         for (size_t i = 0; i < n_msm; i++)
             cw[i] = msms[i].window_bits ? msms[i].window_bits
-                                        : batch_window(p->group, msms[i].n, p->fixed, p->glv, form < 2 && all >= kWidePlan);
+                                        : batch_window(p->group, msms[i].n, p->fixed, p->glv, form < 2 && all >= kWidePlan, p->persistent && form < 2);
         if (widths_fit(msms, cw, p, p->persistent && form < 2)) return LZK_OK;
     }
     return LZK_EINVAL;
@@ -516,7 +527,7 @@ static int create_plan(const lzk_msm_desc* msms, size_t n_msm, const lzk_ntt_des
     // the plan's largest MSM picks the accumulation chunk and reduction run
     size_t largest = 0;
     for (size_t i = 0; i < n_msm; i++) largest = std::max(largest, msms[i].n);
-    p->chunk = tune_chunk(p->group, largest, p->fixed);
+    p->chunk = p->persistent && p->fixed && p->total_pts >= kWidePlan ? persistent_chunk(largest) : tune_chunk(p->group, largest, p->fixed);
     p->run = tune_run(p->group, largest, p->fixed);
     // each width group reduces with the run of its own largest MSM's size class
     // (4 buckets a lane at least: shorter runs pay only where lanes are idle)

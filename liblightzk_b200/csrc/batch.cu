@@ -342,9 +342,8 @@ static int run_plan(lzk_batch_plan* p, cudaStream_t st)
                 fin, p->ent, p->off, (uint32_t)p->total_buckets, p->chunks, p->chunk, p->rounds, p->max_slots >> p->rounds,
                 bsum, static_cast<X*>(p->head), static_cast<X*>(p->tail)); note_launch();
         } else {
-            k_accumulate<K, LZK_BASES_AFFINE><<<grid_for(p->chunks * LP, 128), 128, 0, st>>>(
-                pts, p->ent, p->off, (uint32_t)p->total_buckets, p->chunks, p->chunk, 0, npts, bsum,
-                static_cast<X*>(p->head), static_cast<X*>(p->tail)); note_launch();
+            accumulate_plain<F, LZK_BASES_AFFINE>(pts, p->ent, p->off, (uint32_t)p->total_buckets, p->chunks, p->chunk,
+                                                  npts, bsum, static_cast<X*>(p->head), static_cast<X*>(p->tail), st);
         }
         trace_end(tr, st);
         tr = trace_begin("batch_msm_fixup", st);

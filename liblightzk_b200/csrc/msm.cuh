@@ -352,13 +352,6 @@ __device__ __forceinline__ Aff<Fq> load_raw<Fq, kLayoutPoints>(const void* bases
     Aff<Fq> a = ldg_elem(reinterpret_cast<const Aff<Fq>*>(bases) + idx);
     return is_marker(a.x) ? Aff<Fq>{Fq::zero(), Fq::zero()} : a;
 }
-template <>
-__device__ __forceinline__ Aff<Fq2> load_raw<Fq2, kLayoutPoints>(const void* bases, uint32_t idx)
-{
-    Aff<Fq2> a = ldg_elem(reinterpret_cast<const Aff<Fq2>*>(bases) + idx);
-    return is_marker(a.x) ? Aff<Fq2>{Fq2::zero(), Fq2::zero()} : a;
-}
-
 // the coordinates of a G2 base that this lane holds (MemOf<Fq2P>)
 template <>
 __device__ __forceinline__ Aff<Fq2P> load_raw<Fq2P, LZK_BASES_AFFINE>(const void* bases, uint32_t idx)
@@ -436,11 +429,11 @@ __device__ __forceinline__ void accumulate_chunk(uint64_t t, const void* __restr
     else if (cont_after) st_pt<F>(tail + t, acc);
     else st_pt<F>(bsum + b, acc);
 }
-// 128-thread blocks; at most 168 registers for G1 (3 blocks = 12 warps per
-// SM) and 255 for G2 (2 blocks).  With the products on the FP64 pipe the
-// tighter register bounds make the product calls spill: G1 at 3 blocks/SM
-// measured 6 % faster than at 5 (which matched 4 and 6), G2 at 2 blocks 10 %
-// faster than at 3 and 16 % faster than at 4.
+// 128-thread blocks; at most 168 registers for G1 and for G2 over two lanes (3
+// blocks = 12 warps per SM) and 255 for whole G2 points (2 blocks).  With the
+// products on the FP64 pipe the tighter register bounds make the product calls
+// spill: G1 at 3 blocks/SM measured 6 % faster than at 5 (which matched 4 and
+// 6), whole G2 points at 2 blocks 10 % faster than at 3 and 16 % than at 4.
 template <class F, int LAYOUT>
 __global__ void __launch_bounds__(128, sizeof(F) == 32 ? 3 : 2) k_accumulate(const void* __restrict__ bases, const uint32_t* __restrict__ ent,
                                                     const uint32_t* __restrict__ off, uint32_t B, size_t chunks,
@@ -449,6 +442,26 @@ __global__ void __launch_bounds__(128, sizeof(F) == 32 ? 3 : 2) k_accumulate(con
                                                     XYZZm<F>* __restrict__ tail)
 {
     accumulate_chunk<F, LAYOUT>(gtid() / MemOf<F>::lanes, bases, ent, off, B, chunks, chunk, shift, nbases, bsum, head, tail);
+}
+
+// The accumulation of a list without affine rounds.  G2 points over two lanes
+// halve a chunk's chain but issue a quarter more: for lists with fewer chunks
+// than the device has warps to hide the latency of.  Over reference tables of
+// 16-bit windows, chunk 32, whole MSM: 4000 points (2000 chunks) 1035 us with two
+// lanes, 1057 whole; 16000 (8000) 1002 and 996; 32000 1142 and 1030; 262144
+// 3785 and 3106.
+constexpr size_t kWholeG2Chunks = 4096;
+template <class F, int LAYOUT>
+inline void accumulate_plain(const void* bases, const uint32_t* ent, const uint32_t* off, uint32_t B, size_t chunks,
+                             uint32_t chunk, uint64_t nbases, XYZZ<F>* bsum, XYZZ<F>* head, XYZZ<F>* tail, cudaStream_t st)
+{
+    using K = typename LaneOf<F>::T;
+    constexpr uint32_t LP = MemOf<K>::lanes;
+    if (LP == 1 || chunks >= kWholeG2Chunks)
+        k_accumulate<F, LAYOUT><<<grid_for(chunks, 128), 128, 0, st>>>(bases, ent, off, B, chunks, chunk, 0, nbases, bsum, head, tail);
+    else
+        k_accumulate<K, LAYOUT><<<grid_for(chunks * LP, 128), 128, 0, st>>>(bases, ent, off, B, chunks, chunk, 0, nbases, bsum, head, tail);
+    note_launch();
 }
 
 template <class F>
@@ -977,9 +990,9 @@ int run_msm(const Fr* scalars, const void* bases, size_t n, Jac<typename Gp::F>*
                                   base + p.o_aff, fin, st));
             k_accumulate<K, kLayoutPoints><<<g, 128, 0, st>>>(fin, ent, off, p.B, p.chunks, p.chunk, p.rounds, p.max_slots >> p.rounds, bsum, head, tail); note_launch();
         } else if (layout == LZK_BASES_AFFINE) {
-            k_accumulate<K, LZK_BASES_AFFINE><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, 0, nbases, bsum, head, tail); note_launch();
+            accumulate_plain<F, LZK_BASES_AFFINE>(bases, ent, off, p.B, p.chunks, p.chunk, nbases, bsum, head, tail, st);
         } else {
-            k_accumulate<K, REF><<<g, 128, 0, st>>>(bases, ent, off, p.B, p.chunks, p.chunk, 0, nbases, bsum, head, tail); note_launch();
+            accumulate_plain<F, REF>(bases, ent, off, p.B, p.chunks, p.chunk, nbases, bsum, head, tail, st);
         }
     }
     trace_end(tr, st);

@@ -148,10 +148,11 @@ __device__ __forceinline__ bool load_x(const Aff<F>* src, uint32_t v, uint64_t n
     return is_marker(x);
 }
 template <bool FIRST, class F>
-__device__ __forceinline__ F load_y(const Aff<F>* src, uint32_t v)
+__device__ __forceinline__ F load_y(const Aff<F>* src, uint32_t v, uint64_t nbases)
 {
+    (void)nbases;
     if (FIRST) {
-        if (v == kNoEntry) return F::zero();
+        if (v == kNoEntry || !LZK_CHECK((v & 0x7fffffffu) < nbases, 2)) return F::zero();
         F y = ldg_elem(&src[v & 0x7fffffffu].y);
         return v & 0x80000000u ? neg(y) : y;
     }
@@ -194,11 +195,11 @@ __device__ __forceinline__ uint2 pair_at(const AffineRound<F>& a, uint32_t j)
 
 // The denominator of a pair, or one where its sum needs no addition.
 template <bool FIRST>
-__device__ __forceinline__ D5 pair_den(const Aff<Fq>* src, uint2 v, const Fq& x1, const Fq& x2, bool skip)
+__device__ __forceinline__ D5 pair_den(const Aff<Fq>* src, uint64_t nbases, uint2 v, const Fq& x1, const Fq& x2, bool skip)
 {
     Fq d = sub_plus_p(x2, x1);
     if (!skip && x1 == x2) {
-        const Doubling<Fq> e = same_x(x1, load_y<FIRST>(src, v.x), load_y<FIRST>(src, v.y));
+        const Doubling<Fq> e = same_x(x1, load_y<FIRST>(src, v.x, nbases), load_y<FIRST>(src, v.y, nbases));
         d = e.den;
         skip = !e.ok;
     }
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(kAffThreads, kAffBlocksG1) k_affine_prefix_g1(
         bool skip = load_x<FIRST>(a.src, v.x, a.nbases, x1);
         skip |= load_x<FIRST>(a.src, v.y, a.nbases, x2);
         park(a.out + j, acc);
-        const D5 D = pair_den<FIRST>(a.src, v, x1, x2, skip);
+        const D5 D = pair_den<FIRST>(a.src, a.nbases, v, x1, x2, skip);
         mont52_core<FqP>(acc.l, to_d5(acc.l).d, D.d);
     }
     a.acc[t0] = acc;
@@ -253,7 +254,7 @@ __global__ void __launch_bounds__(kAffThreads, kAffBlocksG1) k_affine_sum_g1(con
         const D5 pre = unpark(a.out + j);
         Fq x1, x2;
         const bool inf1 = load_x<FIRST>(a.src, v.x, a.nbases, x1), inf2 = load_x<FIRST>(a.src, v.y, a.nbases, x2);
-        const Fq y1 = load_y<FIRST>(a.src, v.x), y2 = load_y<FIRST>(a.src, v.y);
+        const Fq y1 = load_y<FIRST>(a.src, v.x, a.nbases), y2 = load_y<FIRST>(a.src, v.y, a.nbases);
         Fq d = sub_plus_p(x2, x1), n = sub_plus_p(y2, y1);
         bool skip = inf1 | inf2, none = inf1 & inf2;
         if (!skip && x1 == x2) {
@@ -312,11 +313,11 @@ static __device__ __noinline__ L5 mont_dot_call(const D5 a0, const D5 b0, const 
 // parked beside the prefix.  All products are two out-of-line bodies (a
 // product, a sum of two products), which keeps the kernels' code small.
 template <bool FIRST>
-__device__ __forceinline__ L5 pair_norm(const Aff<Fq2>* src, uint2 v, const Fq2& x1, const Fq2& x2, bool skip)
+__device__ __forceinline__ L5 pair_norm(const Aff<Fq2>* src, uint64_t nbases, uint2 v, const Fq2& x1, const Fq2& x2, bool skip)
 {
     Fq2 d{sub_plus_p(x2.c0, x1.c0), sub_plus_p(x2.c1, x1.c1)};
     if (!skip && x1 == x2) {
-        const Doubling<Fq2> e = same_x(x1, load_y<FIRST>(src, v.x), load_y<FIRST>(src, v.y));
+        const Doubling<Fq2> e = same_x(x1, load_y<FIRST>(src, v.x, nbases), load_y<FIRST>(src, v.y, nbases));
         d = e.den;
         skip = !e.ok;
     }
@@ -338,7 +339,7 @@ __global__ void __launch_bounds__(kAffThreads, kAffBlocksG2) k_affine_prefix_g2(
         skip |= load_x<FIRST>(a.src, v.y, a.nbases, x2);
         char* s = reinterpret_cast<char*>(a.out + j);
         park(s, acc);
-        const L5 N = pair_norm<FIRST>(a.src, v, x1, x2, skip);
+        const L5 N = pair_norm<FIRST>(a.src, a.nbases, v, x1, x2, skip);
         park(s + 32, N);
         acc = mont_call(to_d5(acc.l), to_d5(N.l));
     }
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(kAffThreads, kAffBlocksG2) k_affine_sum_g2(con
         // slope (times 4): (n0 + n1 i)(e0 - e1 i), e = d / norm
         D5 L0, L1;
         {
-            const Fq2 y1 = load_y<FIRST>(a.src, v.x), y2 = load_y<FIRST>(a.src, v.y);
+            const Fq2 y1 = load_y<FIRST>(a.src, v.x, a.nbases), y2 = load_y<FIRST>(a.src, v.y, a.nbases);
             Fq2 d{sub_plus_p(x2.c0, x1.c0), sub_plus_p(x2.c1, x1.c1)};
             Fq2 n{sub_plus_p(y2.c0, y1.c0), sub_plus_p(y2.c1, y1.c1)};
             if (!skip && x1 == x2) {
@@ -397,11 +398,11 @@ __global__ void __launch_bounds__(kAffThreads, kAffBlocksG2) k_affine_sum_g2(con
             neg52<8>(ln.l, l.l);
             y3.c0 = canon52(mont_dot_call(L0, w0, L1, to_d5(ln.l)).l);
             y3.c1 = canon52(mont_dot_call(L0, to_d5(l.l), L1, w0).l);
-            const Fq2 y1 = load_y<FIRST>(a.src, v.x);
+            const Fq2 y1 = load_y<FIRST>(a.src, v.x, a.nbases);
             y3 = sub(y3, y1);
             if (skip) {
                 x3 = none ? marker<Fq2>() : inf1 ? x2 : x1;
-                y3 = inf1 ? load_y<FIRST>(a.src, v.y) : y1;
+                y3 = inf1 ? load_y<FIRST>(a.src, v.y, a.nbases) : y1;
             }
         }
         st_elem(&a.out[j].x, x3);

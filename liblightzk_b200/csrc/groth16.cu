@@ -706,16 +706,16 @@ int lzk_prover_create(const lzk_groth16_circuit* c, const lzk_groth16_pk* pk, in
 {
     if (!out) return LZK_EINVAL;
     *out = nullptr;
-    // a device without room for the affine rounds' scratch still proves
+    // a device without room for the full scratch (the affine rounds', and the
+    // workspace that lets B1 run beside A) still proves
     lzk_prover* p = nullptr;
     for (bool lean : {false, true}) {
         p = new (std::nothrow) lzk_prover();
         if (!p) return LZK_ENOMEM;
         int rc = create(c, pk, mode, window_bits, lean, p);
         if (rc == LZK_OK) break;
-        const bool again = rc == LZK_ENOMEM && !lean && (table_rounds(p->tn[2], p->c) || table_rounds(p->n_vars, p->c));
         destroy(p);
-        if (!again) return rc;
+        if (rc != LZK_ENOMEM || lean) return rc;
     }
     *out = p;
     return LZK_OK;

@@ -62,6 +62,36 @@ def test_shrinks_on_a_full_device(cuda, orc, rng_state):
     srv.close()
 
 
+def test_short_prover_made_on_a_full_device(cuda, orc, rng_state):
+    """too few entries for rounds, but a workspace more that lets B1 run beside
+    A: without room for it the prover is made lean"""
+    import torch
+    from liblightzk_b200 import groth16, synth
+    lean = _lean_bytes(13, 22)
+    circ, prover = _prover(13, 22)
+    full = prover.device_bytes()
+    assert full - lean > 128 << 20
+    z, (r, s) = circ.witness(5), orc.rand_field(FR, 2, rng_state)
+    want = _wire(prover, z, r, s)
+    pk = synth.ProvingKey(circ, seed=4)
+    prover.close()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    hog, chunk = [], 1 << 34
+    try:
+        while chunk >= (4 << 20):
+            if torch.cuda.mem_get_info()[0] <= (full + lean) // 2 + chunk:
+                chunk //= 2
+                continue
+            hog.append(torch.empty(chunk, dtype=torch.uint8, device="cuda"))
+        prover = groth16.Prover(circ, pk, window_bits=22)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert prover.device_bytes() == lean
+    assert (_wire(prover, z, r, s) == want).all()
+
+
 def test_no_memory_for_the_lean_scratch(cuda, orc, rng_state):
     from liblightzk_b200 import LzkError, _capi, serve
     lean = _lean_bytes(12, 8)

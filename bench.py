@@ -499,11 +499,12 @@ def run_tune_case(args):
     benchmark prover's own MSMs, chosen by timing whole proofs"""
     from liblightzk_b200 import autotune, groth16, synth
     t0 = time.time()
-    t1 = autotune.tune_msm(1, log_ns=range(10, 22), spread=2, reps=2)
-    t2 = autotune.tune_msm(2, log_ns=range(10, 21), spread=1, reps=2)
-    tt = autotune.tune_msm_table(1, log_ns=range(10, 21), reps=2)
-    tt2 = autotune.tune_msm_table(2, log_ns=range(10, 21), spread=(4, 1), reps=2)
-    tn = autotune.tune_ntt(range(10, 25), reps=2)
+    t1 = autotune.tune_msm(1, reps=2)
+    t2 = autotune.tune_msm(2, spread=3, reps=2)
+    tt = autotune.tune_msm_table(1, reps=2)
+    tt2 = autotune.tune_msm_table(2, reps=2)
+    tn = autotune.tune_ntt(reps=2)
+    autotune.fill_edges()
     circ = synth.Circuit(args.log_m, seed=1)
     pk = synth.ProvingKey(circ, seed=7)
     tp = autotune.tune_prover(circ, pk, window_bits=args.window)

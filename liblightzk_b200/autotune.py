@@ -5,12 +5,15 @@ seeded random inputs, median of a few runs) and installs the fastest:
 
   window  Pippenger window width of plain-base MSMs (the cost model's
           width and its neighbours)
-  chunk   sorted bucket entries one accumulation thread adds (32, 64, 128)
-  run     buckets per lane run in the bucket-reduction tiles (4, 8, 16)
+  chunk   sorted bucket entries one accumulation thread adds (8 to 128)
+  run     buckets per lane run in the bucket-reduction tiles (1 to 16)
   ntt     elements per block of an NTT pass, i.e. how a transform's stages
           split into passes (256, 512, 1024, 2048)
   table_*  window width, chunk and run of MSMs over shifted-copy tables
           (provers, batch plans with fixed bases)
+
+The sweeps reach from 2^6 to 2^21 points (2^24 elements); `fill_edges` gives
+the size classes beyond them the values of the nearest one measured.
 
 Every autotuned MSM, batch plan and prover made afterwards uses the table
 (a prover or plan reads it when it is created).  `save` / `load` keep a
@@ -30,6 +33,18 @@ DEFAULT_TABLES = {"B200": os.path.join(os.path.dirname(os.path.abspath(__file__)
 WINDOW, CHUNK, RUN, NTT_BLOCK, TABLE_WINDOW, TABLE_CHUNK, TABLE_RUN = range(7)
 KNOBS = {"window": WINDOW, "chunk": CHUNK, "run": RUN, "ntt": NTT_BLOCK, "table_window": TABLE_WINDOW,
          "table_chunk": TABLE_CHUNK, "table_run": TABLE_RUN}
+# candidates of the sweeps: short chunks and runs are for lists that leave the
+# device idle, long ones for lists that fill it several times
+CHUNKS, RUNS, BLOCKS = (8, 16, 32, 64, 128), (1, 2, 4, 8, 16), (256, 512, 1024, 2048)
+# size classes the sweeps of a whole table cover, by group: plain MSMs, table
+# MSMs, and transforms
+PLAIN_CLASSES = {1: range(6, 22), 2: range(8, 21)}
+TABLE_CLASSES = {1: range(8, 21), 2: range(8, 21)}
+NTT_CLASSES = range(10, 25)
+# plain G1 widths hold up to this class: at 2^22 to 2^25 points the width of 2^21
+# is within 1 % of the best; from 2^26 on the cost model's is better (200 instead
+# of 205 ms), and at 2^28 narrow ones make more entries than can be numbered
+PLAIN_WIDTH_TOP = 25
 
 
 def _time(fn, reps):
@@ -72,13 +87,25 @@ def tune(group=1, log_ns=range(10, 21), spread=2, reps=3, seed=11, install=True)
     return table
 
 
-def tune_msm(group=1, log_ns=range(10, 21), spread=2, reps=3, seed=11, chunks=(32, 64, 128), runs=(4, 8, 16)):
-    """per size class: window width and reduction run together (the run
-    sets how much each bucket costs, which moves the best width), then the
-    accumulation chunk at that pair; installs them and returns
+def _best(res):
+    """the fastest (width, run, chunk), the times by width and run (with the
+    best chunk) and by chunk (at the best width and run)"""
+    c, r, v = min(res, key=res.get)
+    pairs = {}
+    for (x, y, _), ms in res.items():
+        pairs[(x, y)] = min(ms, pairs.get((x, y), ms))
+    return c, r, v, pairs, {z: ms for (x, y, z), ms in res.items() if (x, y) == (c, r)}
+
+
+def tune_msm(group=1, log_ns=None, spread=2, reps=3, seed=11, chunks=CHUNKS, runs=RUNS):
+    """per size class: window width, reduction run and accumulation chunk
+    together (the run sets how much each bucket costs and a short chunk fills
+    the device with few entries, which both move the best width); installs
+    them and returns
     {log_n: {"window": best_c, "run": best_run, "chunk": best_chunk,
              "ms": {"c,run": ms}, "chunk_ms": {chunk: ms}}}"""
     out = {}
+    log_ns = PLAIN_CLASSES[group] if log_ns is None else log_ns
     top = max(log_ns)
     sc_all = synth.random_fr(1 << top, seed, 90)
     bases_all = synth.fixed_base(group, synth.random_fr(1 << top, seed, 91))
@@ -92,29 +119,27 @@ def tune_msm(group=1, log_ns=range(10, 21), spread=2, reps=3, seed=11, chunks=(3
         for c in range(max(2, c0 - spread), min(22, c0 + spread) + 1):
             for r in runs:
                 set_value("run", group, lg, r)
-                res[(c, r)] = _time(lambda c=c: msm.msm(group, s, b, window_bits=c), reps)
-        c_best, r_best = min(res, key=res.get)
+                for v in chunks:
+                    set_value("chunk", group, lg, v)
+                    res[(c, r, v)] = _time(lambda c=c: msm.msm(group, s, b, window_bits=c), reps)
+        c_best, r_best, ch_best, res, cres = _best(res)
         set_value("window", group, lg, c_best)
         set_value("run", group, lg, r_best)
-        cres = {}
-        for v in chunks:
-            set_value("chunk", group, lg, v)
-            cres[v] = _time(lambda: msm.msm(group, s, b), reps)
-        ch_best = min(cres, key=cres.get)
         set_value("chunk", group, lg, ch_best)
         out[lg] = {"window": c_best, "run": r_best, "chunk": ch_best,
                    "ms": {f"{c},{r}": v for (c, r), v in res.items()}, "chunk_ms": cres}
     return out
 
 
-def tune_msm_table(group=1, log_ns=range(10, 21), spread=(4, 2), reps=3, seed=11, runs=(4, 8, 16), chunks=(32, 64, 128)):
-    """window width and reduction run (together), then chunk, of an MSM over
-    a shifted-copy table, per size class, timing one MSM of 2^log_n points
+def tune_msm_table(group=1, log_ns=None, spread=(4, 2), reps=3, seed=11, runs=RUNS, chunks=CHUNKS):
+    """window width, reduction run and chunk together, of an MSM over a
+    shifted-copy table, per size class, timing one MSM of 2^log_n points
     (the table of each width built outside the timing; widths from
     spread[0] below the cost model's to spread[1] above); installs the best
     and returns {log_n: {"window", "run", "chunk", "ms": {"c,run": ms},
     "chunk_ms": {chunk: ms}}}"""
     out = {}
+    log_ns = TABLE_CLASSES[group] if log_ns is None else log_ns
     top = max(log_ns)
     sc_all = synth.random_fr(1 << top, seed, 94)
     bases_all = synth.fixed_base(group, synth.random_fr(1 << top, seed, 95))
@@ -124,32 +149,28 @@ def tune_msm_table(group=1, log_ns=range(10, 21), spread=(4, 2), reps=3, seed=11
         for knob in ("table_window", "table_run", "table_chunk"):
             set_value(knob, group, lg, 0)
         c0 = msm.autotune_window(group, n, precomputed=True)
-        res, tabs = {}, {}
+        res = {}
         # the model leans to wide windows (it undercounts the bucket
         # reduction), so the candidates reach further below it than above
         for c in range(max(4, c0 - spread[0]), min(20, c0 + spread[1]) + 1):
             w = msm.windows_for(c)
-            tabs[c] = msm.precompute(group, b, c, w, n)
+            tab = msm.precompute(group, b, c, w, n)
             for r in runs:
                 set_value("table_run", group, lg, r)
-                res[(c, r)] = _time(lambda c=c, w=w: msm.msm_precomputed(group, s, tabs[c], c, w, n), reps)
-        c_best, r_best = min(res, key=res.get)
+                for v in chunks:
+                    set_value("table_chunk", group, lg, v)
+                    res[(c, r, v)] = _time(lambda c=c, w=w: msm.msm_precomputed(group, s, tab, c, w, n), reps)
+            del tab
+        c_best, r_best, ch_best, res, cres = _best(res)
         set_value("table_window", group, lg, c_best)
         set_value("table_run", group, lg, r_best)
-        w = msm.windows_for(c_best)
-        cres = {}
-        for v in chunks:
-            set_value("table_chunk", group, lg, v)
-            cres[v] = _time(lambda: msm.msm_precomputed(group, s, tabs[c_best], c_best, w, n), reps)
-        ch_best = min(cres, key=cres.get)
         set_value("table_chunk", group, lg, ch_best)
-        del tabs
         out[lg] = {"window": c_best, "run": r_best, "chunk": ch_best,
                    "ms": {f"{c},{r}": v for (c, r), v in res.items()}, "chunk_ms": cres}
     return out
 
 
-def tune_ntt(log_ns=range(12, 23), reps=3, seed=12, blocks=(256, 512, 1024, 2048), direction=ntt.COSET_FORWARD):
+def tune_ntt(log_ns=NTT_CLASSES, reps=3, seed=12, blocks=BLOCKS, direction=ntt.COSET_FORWARD):
     """NTT block size per transform size; installs the fastest and returns
     {log_n: (best, {block: ms})}"""
     out = {}
@@ -166,7 +187,7 @@ def tune_ntt(log_ns=range(12, 23), reps=3, seed=12, blocks=(256, 512, 1024, 2048
     return out
 
 
-def tune_prover(circuit, pk, mode=0, window_bits=17, chunks=(32, 64), runs=(4, 8, 16), proofs=8, seed=13):
+def tune_prover(circuit, pk, mode=0, window_bits=0, chunks=CHUNKS[:4], runs=RUNS, proofs=8, seed=13):
     """accumulation chunk and reduction run of a Groth16 prover's own MSMs
     (shifted-table MSMs over the circuit's variables, the L + H concatenation
     and the G2 query), chosen by timing whole proofs; installs the best
@@ -194,6 +215,26 @@ def tune_prover(circuit, pk, mode=0, window_bits=17, chunks=(32, 64), runs=(4, 8
     best = min(res, key=res.get)
     install(*best)
     return res
+
+
+def fill_edges():
+    """give the size classes outside the sweeps the values of the nearest class
+    in them; table widths above stay unset (the cost model), plain G1 ones from
+    2^26 on too (PLAIN_WIDTH_TOP), and so do all of G2 above"""
+    def copy(knob, group, classes, top):
+        for lg in range(33):
+            if lg < classes[0]:
+                set_value(knob, group, lg, get_value(knob, group, classes[0]))
+            elif lg > classes[-1]:
+                set_value(knob, group, lg, get_value(knob, group, classes[-1]) if lg <= top else 0)
+    for g in (1, 2):
+        copy("window", g, PLAIN_CLASSES[g], PLAIN_WIDTH_TOP if g == 1 else 0)
+        for knob in ("chunk", "run"):
+            copy(knob, g, PLAIN_CLASSES[g], 32 if g == 1 else 0)
+        for knob in ("table_window", "table_chunk", "table_run"):
+            for lg in range(TABLE_CLASSES[g][0]):
+                set_value(knob, g, lg, get_value(knob, g, TABLE_CLASSES[g][0]))
+    copy("ntt", 0, NTT_CLASSES, 32)
 
 
 def load_default():

@@ -168,10 +168,11 @@ __device__ __forceinline__ size_t brev_k(size_t j, uint32_t k)
 }
 
 // ---------------- lazily reduced values ----------------
-// Inside a pass a value stays below 2p (DIF) or 4p (DIT) instead of p: the
-// FP64 product takes operands below 4p (times a table value below 2p) and
-// leaves a result below 2p, so a butterfly needs one conditional subtraction
-// instead of three.
+// Inside a pass a value stays below 2p (DIF) or 4p (DIT) instead of p, so a
+// butterfly needs one conditional subtraction instead of three.  The FP64
+// product of x and t is 16 x t / 2^260 + (less than p), with 2^260 = 84.6 p:
+// below 2p for x < 4p and t < 1.3 p (16 4 1.3 = 83.2).  t is a canonical table
+// value, or a product of canonical ones (edge_apply2).
 __host__ __device__ constexpr uint32_t fr_2p(int i) { return (FrP::p(i) << 1) | (i ? FrP::p(i - 1) >> 31 : 0u); }
 
 // a + b, no reduction
@@ -231,7 +232,8 @@ __device__ __forceinline__ Fr sub_2p(const Fr& a, const Fr& b)
     return r;
 }
 
-// A product operand in radix-2^52 form, and x tx, y ty (< 2p) for x, y < 4p.
+// A product operand in radix-2^52 form, and x tx, y ty (< 2p) for x, y < 4p and
+// tx, ty < 1.3 p.
 // Two products to a call: they interleave, and one body of about 700
 // instructions keeps the pass inside the instruction cache.
 struct Tw {
@@ -274,7 +276,9 @@ __device__ __forceinline__ Tw load_tw(const Fr* __restrict__ tw, const double* _
 // Factor a pass applies to each element as it loads it (the first pass) or
 // stores it (the last pass): x * scale * g^e, e = the position j, or, with
 // brev set, the coefficient index brev(j) that a bit-reversed position
-// holds; a null scale or null power tables stand for 1.  x < 4p, result < 2p.
+// holds; a null scale or null power tables stand for 1.  x < 4p, result < 2p:
+// the table values are canonical, so lo hi < (1 + 16 / 84.6) p = 1.19 p, and
+// that times the scale < (1 + 16 1.19 / 84.6) p = 1.23 p.
 __device__ __forceinline__ void edge_apply2(const NttEdge& ed, Fr& x, Fr& y, uint32_t jx, uint32_t jy, uint32_t k)
 {
     if (ed.lo) {

@@ -356,7 +356,8 @@ int lzk_groth16_proof_from_wire(const void* wire, lzk_groth16_proof* proof, uint
  * A worker thread admits queued requests (oldest first) into proof
  * contexts -- an idle context of the request's circuit, or a new one while
  * the device-memory budget allows (idle contexts of other circuits are
- * released to make room) -- and runs each on its own streams, so requests
+ * released to make room; a context is larger, and its proofs faster, where
+ * the budget has room for that beside all others that may be wanted) -- and runs each on its own streams, so requests
  * that arrive while others run start as soon as a context and memory are
  * free and their work overlaps on the device.  Resident provers count
  * against the budget when added.  Latency is submission to completion.
